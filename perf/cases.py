@@ -59,7 +59,7 @@ def listed():
          "nx": 401, "ny": 201, "lo": 2e5, "hi": 6e5, "steps": 5, "layout": 5},
         # the solver as a plugin of the host's own loop: potential and concentration in,
         # potential out, on a grid above those of the configurations
-        {"name": "poisson_801x401", "kind": "poisson", "shape": "mosfet", "nx": 801, "ny": 401,
+        {"name": "poisson_801x401", "kind": "poisson", "shape": "resistor", "nx": 801, "ny": 401,
          "equilibrium": False, "fp32": True, "noalloc": False},
         # the solve that allocates nothing, on the caller's device arrays
         {"name": "noalloc_201x101", "kind": "poisson", "shape": "resistor", "nx": 201, "ny": 101,
@@ -114,8 +114,10 @@ def draw(rng):
     top = 131072 if noalloc else 801 * 401
     nx = round(_log(rng, 41, 801))
     ny = round(_log(rng, 31, min(401, top // nx)))
-    return {"kind": "poisson", "shape": rng.choice(["resistor", "mosfet"]), "nx": nx, "ny": ny,
-            "equilibrium": rng.random() < 0.3,
+    # a step of a running bar, or a MOSFET's equilibrium from its neutral potential
+    shape = rng.choice(["resistor", "resistor", "mosfet"])
+    return {"kind": "poisson", "shape": shape, "nx": nx, "ny": ny,
+            "equilibrium": shape == "mosfet",
             "fp32": noalloc or nx * ny > 80601 or rng.random() < 0.7, "noalloc": noalloc}
 
 
@@ -195,7 +197,7 @@ def _mosfet_layout(case):
 
 def _grids(case, seed):
     """The device, a starting potential and a noisy electron concentration: those of the
-    neutral device, as a step of a running simulation finds them."""
+    neutral device, as a running bar's next step or a MOSFET's first solve finds them."""
     nx, ny = case["nx"], case["ny"]
     dev = _resistor(nx, ny, 0.5e-9, 5e5) if case["shape"] == "resistor" else \
         _mosfet(nx, ny, 0.05)
@@ -208,7 +210,9 @@ def _grids(case, seed):
     conc = rs.poisson(per * n / full) * (full / per)
     if case["shape"] == "resistor":  # the applied voltage falls along the bar
         pot = pot + np.tile(np.linspace(0.5, 0.0, nx) / dev.getThermalVoltage(), ny)
-    pot = pot + 0.02 * rs.standard_normal(pot.size)
+        pot = pot + 0.02 * rs.standard_normal(pot.size)
+    else:
+        pot = pot + 0.02 * rs.standard_normal()
     return dev, pot, (None if case["equilibrium"] else conc)
 
 
