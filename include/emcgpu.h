@@ -309,14 +309,16 @@ int32_t emcg_set_launch(emcg_handle *h, int32_t block_threads,
    launch setting (0: all steps of a call in one launch). */
 int32_t emcg_get_launch(emcg_handle *h, int32_t *block_threads, int32_t *steps_per_launch);
 
-/* Tuning, the step kernel: 0 lockstep (each warp advances its particles
-   step by step and handles their events; the default of the double engine);
+/* Tuning, the step kernel: 0 for a float engine lockstep (each warp advances
+   its particles step by step and handles their events), for a double engine
+   pooled, its default (each warp works on those of its electrons that need the
+   same thing next; the block size and the register cap do not apply);
    1 block-queued (the events of a thread block are processed together by its
    first warps); 2 warp-asynchronous, float only and the float engine's
    default (each lane runs its particle from event to event across step
    boundaries, so a warp's lanes process their events together; per-step
    observables go through a per-warp window).  All follow the same
-   per-particle algorithm; replay always uses the lockstep kernel.  In the
+   per-particle algorithm; replay always uses a lockstep kernel.  In the
    queued kernel a grain event (the grain mechanism's draws and the timer
    redraw) takes its own Philox calls, so its stream differs from the
    lockstep kernel and the oracle in grain events only (without a grain

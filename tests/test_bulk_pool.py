@@ -1,0 +1,95 @@
+"""The double engine's pooled step kernel (mode 0) against the block-queued one
+(mode 1), which runs the plain per-particle step: the same Philox counters, so
+the same trajectories bar last-ulp branch flips.  And its integer forms of the
+uniform draw and the table level, and its log, against the expressions they
+stand for (host, compiled natively)."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from test_host import L_FRAMES
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _native(tmp_path, name):
+    exe = tmp_path / name
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off",
+                    f"-I{ROOT}/viennaemc_gb300/csrc", f"{ROOT}/tests/native/{name}.cpp", "-o",
+                    str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+
+
+def test_log_of_the_draws(tmp_path):
+    """Within 1.01 units in the last place of the extended-precision log (the
+    table sum and the last addition round once each at most half a unit)."""
+    worst, rms, _, specials = _native(tmp_path, "log_check")
+    assert float(worst) <= 1.01 and float(rms) < 0.29 and specials == "1"
+
+
+def test_integer_draw_and_level(tmp_path):
+    assert _native(tmp_path, "draws_check") == ["0"]
+
+
+def _tilted(engine):
+    """Two valleys, the upper one with eight subvalleys whose axes are not the
+    device's."""
+    from viennaemc_gb300 import physics as P
+    mat = P.silicon_material()
+    pt = P.Electron(1000, 2.0)
+    P.add_x_valley(pt, 0.19)
+    v = P.NonParabolicAnisotropValley([0.8, 0.2, 0.2], pt.getMass(), 8, 0.3, 0.15)
+    for s, f in enumerate(L_FRAMES):
+        v.setSubValleyEllipseCoordSystem(s, *f)
+    pt.addValley(v)
+    for k in (0, 1):
+        pt.addScatterMechanism([0], P.AcousticScatterMechanism(k, 9.0, 300.0, mat.rho,
+                                                               mat.velSound))
+    up, down = {s: [0, 3, 5] for s in range(3)}, {s: [s % 3] for s in range(8)}
+    for cls in (P.ZeroOrderInterValleyAbsorptionScatterMechanism,
+                P.ZeroOrderInterValleyEmissionScatterMechanism):
+        pt.addScatterMechanism([0], cls("XL", 0, up, 2e10, 0.03, 300.0, mat.rho, 1))
+        pt.addScatterMechanism([0], cls("LX", 1, down, 2e10, 0.03, 300.0, mat.rho, 0))
+    pt.initScatterTables()
+    return pt
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model", ["silicon", "grain", "tilted"])
+@pytest.mark.parametrize("counts", [(1,), (31, 0, 33), (600, 29300), (60013,), (120001,)])
+def test_pooled_kernel_equals_queued_kernel(engine, model, counts):
+    """Pools of one electron, of a partial warp, of 16 to 32, 33 to 64 and 65 to
+    96 electrons, several ensembles and more than one wave; both step launches
+    of 9 steps, so the window and the sums' tail are passed.  A trajectory may
+    branch on a last-ulp difference, as between the other kernels."""
+    pt = _tilted(engine) if model == "tilted" else \
+        engine.physics.silicon_electron("jacoboni", grain=(0.3, 2e13) if model == "grain" else None)
+    specs = [engine.EnsembleSpec(0, n, 2e6, (1, 2, 3), (2e-7, 3e-7, 1e-6), 1e-15, 21 + e, e)
+             for e, n in enumerate(counts)]
+    runs = []
+    for mode in (0, 1):
+        b = engine.BulkBatch([pt], specs, "fp64")
+        b.set_launch(queued=mode, steps_per_launch=9)
+        for e in range(len(counts)):
+            b.init_particles(e)
+        obs = b.step(22)
+        runs.append(([b.get_state(e) for e in range(len(counts))], obs))
+        b.close()
+    for e, n in enumerate(counts):
+        a, q = runs[0][0][e], runs[1][0][e]
+        # with grains the two kernels draw them from other Philox calls: only the
+        # electrons without a grain event agree (a step has one for 2 in 100)
+        same = np.ones(n, bool) if model != "grain" else np.abs(a.grain_tau - q.grain_tau) < 1e-20
+        bad = (a.valley != q.valley) | (a.sub != q.sub)
+        for f in ("kx", "ky", "kz", "px", "py", "pz", "energy", "tau"):
+            x, y = getattr(a, f), getattr(q, f)
+            bad |= np.abs(x - y) > 1e-12 * np.max(np.abs(y), initial=0.0)
+        assert n == 0 or same.mean() > 0.5 or n < 10
+        assert (bad & same).sum() <= n // 1000, (e, (bad & same).sum())
+        oa, oq = runs[0][1][e], runs[1][1][e]
+        assert np.array_equal(oa[:, :, 2].sum(axis=1), np.full(22, n))
+        if model != "grain" and n:
+            assert np.allclose(oa[:, :, 2], oq[:, :, 2], atol=2)
+            assert np.allclose(oa.sum(axis=1)[:, 0], oq.sum(axis=1)[:, 0], rtol=1e-4)

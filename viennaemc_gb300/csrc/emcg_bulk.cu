@@ -10,6 +10,7 @@
 #include <cstring>
 #include <vector>
 
+#include "emcg_bulk_pool.cuh"
 #include "emcg_common.cuh"
 #include "emcg_host.h"
 #include "emcg_model.h"
@@ -1039,9 +1040,11 @@ struct BulkImpl {
   std::vector<void *> dTables;
   std::vector<RateLayout> rates; // table layout per model (rate-table rebuild)
   RateScratch rateScratch;        // device scratch of rebuilds
+  double *dLogTab = nullptr;      // logTab()'s table (double engine)
   void *dEns = nullptr;
   Tile *dTiles = nullptr;
   int nTiles = 0, tilesCap = 0;
+  int tilePool = 0; // the tiles are pools of at most this many electrons (0: thread blocks)
   bool tilesDirty = true;
   void *dState[9] = {};
   uint32_t *dMeta = nullptr;
@@ -1055,7 +1058,8 @@ struct BulkImpl {
   int blockThreads = 256;
   bool autoBlock = true; // block size chosen per launch (emcg_set_launch, -1)
   int minBlocks = 1; // register cap variant of the step kernel (1, 3 or 4)
-  int queued = 0; // step kernel: 0 lockstep, 1 block-queued, 2 warp-asynchronous (float)
+  int queued = 0; // step kernel: 0 lockstep (float) or pooled (double), 1 block-queued, 2
+                  // warp-asynchronous (float)
   int passActions = kPassActions; // warp-asynchronous kernel: free flights per drift pass
   bool passAuto = true;           // not set by the caller or the autotuner: by launch length
   int stepsPerLaunch = 0;
@@ -1086,7 +1090,7 @@ struct BulkImpl {
   cudaGraphExec_t gexec = nullptr;
   cudaGraphNode_t gKernel = nullptr;
   cudaKernelNodeParams gKp = {};
-  int gNs = -1, gBlock = 0, gMinb = 0, gQueued = -1, gTiles = -1, gPass = -1;
+  int gNs = -1, gBlock = 0, gMinb = 0, gQueued = -1, gTiles = -1, gPass = -1, gPool = 0;
   alignas(16) unsigned char gArgs[256] = {};
   void *gParams[14] = {};
 };
@@ -1104,6 +1108,7 @@ template <class T> struct StepArgs {
   int chunk;
   int nVmax;
   int pass;
+  const double *logT; // the pooled kernel's table of log
   double *obs;
   const uint64_t *words;
   const int64_t *off;
@@ -1178,6 +1183,13 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
   EMCG_CUDA(cudaMalloc(&b->dModels, sizeof(ModelK<T>) * nModels));
   EMCG_CUDA(cudaMemcpy(b->dModels, mk.data(), sizeof(ModelK<T>) * nModels,
                        cudaMemcpyHostToDevice));
+  if constexpr (sizeof(T) == 8) {
+    double tab[kLogTab];
+    for (int i = 0; i < kLogTab; i++)
+      tab[i] = logTabEntry(i);
+    EMCG_CUDA(cudaMalloc(&b->dLogTab, sizeof(tab)));
+    EMCG_CUDA(cudaMemcpy(b->dLogTab, tab, sizeof(tab), cudaMemcpyHostToDevice));
+  }
   std::vector<EnsK<T>> ek(nEns);
   for (int e = 0; e < nEns; e++)
     buildEnsK<T>(ens[e], mk[ens[e].model], models[ens[e].model], b->begin[e], 0, ek[e]);
@@ -1186,17 +1198,22 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
   return EMCG_OK;
 }
 
-static int32_t ensureTiles(BulkImpl *b) {
-  if (!b->tilesDirty)
+// The tiles of the step kernels: thread blocks of b->blockThreads electrons,
+// or (pool > 0) pools of at most pool electrons, those of an ensemble alike in
+// size.
+static int32_t ensureTiles(BulkImpl *b, int pool = 0) {
+  if (!b->tilesDirty && b->tilePool == pool)
     return EMCG_OK;
   std::vector<Tile> t;
   for (int e = 0; e < b->nEns; e++) {
-    for (int64_t o = 0; o < b->count[e]; o += b->blockThreads) {
+    const int64_t n = b->count[e], size = pool ? pool : b->blockThreads;
+    const int64_t m = (n + size - 1) / size;
+    for (int64_t k = 0; k < m; k++) {
       Tile x;
       x.ens = e;
       x.pad_ = 0;
-      x.begin = b->begin[e] + o;
-      x.end = b->begin[e] + std::min<int64_t>(o + b->blockThreads, b->count[e]);
+      x.begin = b->begin[e] + (pool ? n * k / m : k * size);
+      x.end = b->begin[e] + (pool ? n * (k + 1) / m : std::min<int64_t>((k + 1) * size, n));
       t.push_back(x);
     }
   }
@@ -1211,6 +1228,7 @@ static int32_t ensureTiles(BulkImpl *b) {
                               cudaMemcpyHostToDevice, b->stream));
   EMCG_CUDA(cudaStreamSynchronize(b->stream));
   b->nTiles = (int)t.size();
+  b->tilePool = pool;
   b->tilesDirty = false;
   return EMCG_OK;
 }
@@ -1262,9 +1280,38 @@ static int32_t growObs(BulkImpl *b, size_t need) {
   return EMCG_OK;
 }
 
+// Electrons per pool of the double engine's kernel, for n in all.  A pool is one
+// warp, and each of an SM's four schedulers issues one double instruction in 64
+// clocks whatever its lanes do: so enough pools to keep every scheduler busy (6
+// per SM; 16 electrons at least, below which the passes cost the same), and
+// beyond 96 electrons whole waves of the 8 pools that an SM holds at once.
+// Measured (1e9 particle-steps/s; pool size: rate): 10,000 electrons 12: 1.35,
+// 16: 1.46, 18: 1.41; 45,000 37: 3.70, 49: 3.96, 74: 3.51; 75,000 62: 4.52, 83:
+// 4.62; 250,007 69: 4.99, 96: 4.59; 400,000 83: 5.39, 96: 5.22.
+static int poolElectrons(int64_t n, int sms) {
+  const int64_t six = 6LL * sms, wave = 8LL * sms;
+  if (n <= six * 96)
+    return (int)std::max<int64_t>(16, (n + six - 1) / six);
+  const int64_t waves = (n + wave * 96 - 1) / (wave * 96);
+  return (int)((n + wave * waves - 1) / (wave * waves));
+}
+template <bool kOne> static auto poolKernel(int pool) {
+  return pool > 64 ? bulkStepPoolKernel<3, kOne>
+                   : pool > 32 ? bulkStepPoolKernel<2, kOne> : bulkStepPoolKernel<1, kOne>;
+}
+static size_t poolSmemFor(int pool, bool one) {
+  return pool > 64 ? poolSmemBytes<3>(one) : pool > 32 ? poolSmemBytes<2>(one)
+                                                       : poolSmemBytes<1>(one);
+}
+
 // the step kernel of the current launch configuration (Philox streams)
 template <class T> static void *stepKernelFn(const BulkImpl *b, bool *queued) {
   *queued = b->queued != 0;
+  if constexpr (sizeof(T) == 8) {
+    if (b->tilePool)
+      return b->nVmax == 1 ? (void *)poolKernel<true>(b->tilePool)
+                           : (void *)poolKernel<false>(b->tilePool);
+  }
   if constexpr (sizeof(T) == 4) {
     if (b->queued == 2) {
       const bool one = b->nVmax == 1;
@@ -1282,17 +1329,21 @@ template <class T> static void *stepKernelFn(const BulkImpl *b, bool *queued) {
       return (void *)bulkStepQueuedKernel<T, 3>;
     return (void *)bulkStepQueuedKernel<T, 1>;
   }
-  if (b->minBlocks >= 4 && b->blockThreads <= 256)
-    return (void *)bulkStepKernel<T, false, 4>;
-  if (b->minBlocks == 3 && b->blockThreads <= 256)
-    return (void *)bulkStepKernel<T, false, 3>;
-  return (void *)bulkStepKernel<T, false, 1>;
+  if constexpr (sizeof(T) == 4) {
+    if (b->minBlocks >= 4 && b->blockThreads <= 256)
+      return (void *)bulkStepKernel<T, false, 4>;
+    if (b->minBlocks == 3 && b->blockThreads <= 256)
+      return (void *)bulkStepKernel<T, false, 3>;
+    return (void *)bulkStepKernel<T, false, 1>;
+  }
+  return nullptr; // the double engine's mode 0 is the pooled kernel
 }
 
 // (Re)build the graph of one launch of ns steps for the current configuration.
 template <class T> static int32_t graphFor(BulkImpl *b, int ns, size_t smem, size_t qsmem) {
   if (b->gexec && b->gNs == ns && b->gBlock == b->blockThreads && b->gMinb == b->minBlocks &&
-      b->gQueued == b->queued && b->gTiles == b->nTiles && b->gPass == b->passActions)
+      b->gQueued == b->queued && b->gTiles == b->nTiles && b->gPass == b->passActions &&
+      b->gPool == b->tilePool)
     return EMCG_OK;
   dropGraph(b);
   static_assert(sizeof(StepArgs<T>) <= sizeof(b->gArgs), "step arguments exceed the buffer");
@@ -1320,8 +1371,13 @@ template <class T> static int32_t graphFor(BulkImpl *b, int ns, size_t smem, siz
                    &a.err};
   void *asy[13] = {&a.st,   &a.src,   &a.srcEns, &a.mp,   &a.ep,  &a.tiles, &a.ns,
                    &a.step0, &a.chunk, &a.nVmax,  &a.pass, &a.obs, &a.err};
+  a.logT = b->dLogTab;
+  void *pol[10] = {&a.st,    &a.mp,    &a.ep,   &a.tiles, &a.ns,
+                   &a.step0, &a.nVmax, &a.logT, &a.obs,   &a.err};
   static_assert(sizeof(asy) <= sizeof(b->gParams), "kernel parameters exceed the buffer");
-  if (b->queued == 2 && sizeof(T) == 4)
+  if (b->tilePool)
+    std::memcpy(b->gParams, pol, sizeof(pol));
+  else if (b->queued == 2 && sizeof(T) == 4)
     std::memcpy(b->gParams, asy, sizeof(asy));
   else if (queued)
     std::memcpy(b->gParams, que, sizeof(que));
@@ -1343,8 +1399,9 @@ template <class T> static int32_t graphFor(BulkImpl *b, int ns, size_t smem, siz
   kp = {};
   kp.func = fn;
   kp.gridDim = dim3(b->nTiles, 1, 1);
-  kp.blockDim = dim3(b->blockThreads, 1, 1);
-  kp.sharedMemBytes = (unsigned)(b->queued == 2 && sizeof(T) == 4
+  kp.blockDim = dim3(b->tilePool ? 32 : b->blockThreads, 1, 1);
+  kp.sharedMemBytes = (unsigned)(b->tilePool ? poolSmemFor(b->tilePool, b->nVmax == 1)
+                                 : b->queued == 2 && sizeof(T) == 4
                                       ? asyncSmemBytes(b->blockThreads / 32, ns, b->nVmax * 3)
                                       : (queued ? qsmem : smem));
   kp.kernelParams = b->gParams;
@@ -1359,6 +1416,17 @@ template <class T> static int32_t graphFor(BulkImpl *b, int ns, size_t smem, siz
   b->gQueued = b->queued;
   b->gPass = b->passActions;
   b->gTiles = b->nTiles;
+  b->gPool = b->tilePool;
+  return EMCG_OK;
+}
+
+// b->sms, the SMs of the engine's device
+static int32_t smCount(BulkImpl *b) {
+  if (b->sms)
+    return EMCG_OK;
+  int dev = 0;
+  EMCG_CUDA(cudaGetDevice(&dev));
+  EMCG_CUDA(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
   return EMCG_OK;
 }
 
@@ -1383,11 +1451,7 @@ template <class T>
 static int32_t coulombStepTyped(BulkImpl *b, int nSteps, uint32_t step0, double *obsHost) {
   EMCG_TRY(ensureTiles(b));
   const int Q = b->nVmax * 3;
-  if (!b->sms) {
-    int dev = 0;
-    EMCG_CUDA(cudaGetDevice(&dev));
-    EMCG_CUDA(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+  EMCG_TRY(smCount(b));
   int64_t srcNeed = 1, partNeed = 1;
   for (int e = 0; e < b->nEns; e++) {
     const int64_t n = b->count[e], m = n + b->nFixed[e];
@@ -1492,6 +1556,15 @@ static int32_t launchStepTiles(BulkImpl *b, const StateK<T> &st, int ns, uint32_
     else
       bulkStepQueuedKernel<T, 1><<<nT, b->blockThreads, qsmem, b->stream>>>(
           st, mp, ep, tiles, ns, s0, b->chunk, b->nVmax, b->dObs, b->dErr);
+  } else if constexpr (sizeof(T) == 8) {
+    const int pool = b->tilePool;
+    const size_t psmem = poolSmemFor(pool, b->nVmax == 1);
+    if (b->nVmax == 1)
+      poolKernel<true>(pool)<<<nT, 32, psmem, b->stream>>>(
+          st, mp, ep, tiles, ns, s0, b->nVmax, b->dLogTab, b->dObs, b->dErr);
+    else
+      poolKernel<false>(pool)<<<nT, 32, psmem, b->stream>>>(
+          st, mp, ep, tiles, ns, s0, b->nVmax, b->dLogTab, b->dObs, b->dErr);
   } else if (b->minBlocks >= 4 && b->blockThreads <= 256) {
     bulkStepKernel<T, false, 4><<<nT, b->blockThreads, smem, b->stream>>>(
         st, mp, ep, tiles, ns, s0, b->chunk, b->nVmax, b->dObs, nullptr,
@@ -1529,7 +1602,17 @@ static int32_t stepTyped(BulkImpl *b, int nSteps, uint32_t step0, double *obsHos
     const int first = std::min(b->stepsPerLaunch > 0 ? b->stepsPerLaunch : nSteps, nSteps);
     b->passActions = first < kShortLaunchSteps ? kPassActionsShort : kPassActions;
   }
-  EMCG_TRY(ensureTiles(b));
+  // the double engine's mode 0: pools
+  const bool pooled = b->queued == 0 && sizeof(T) == 8 && !b->replay;
+  int pool = 0;
+  if (pooled) {
+    EMCG_TRY(smCount(b));
+    int64_t n = 0;
+    for (int64_t c : b->count)
+      n += c;
+    pool = poolElectrons(n, b->sms);
+  }
+  EMCG_TRY(ensureTiles(b, pool));
   const int Q = b->nVmax * 3;
   int per = b->stepsPerLaunch > 0 ? b->stepsPerLaunch : nSteps;
   if (b->replay)
@@ -1593,6 +1676,7 @@ static void freeBulk(BulkImpl *b) {
   for (void *p : b->dTables)
     cudaFree(p);
   cudaFree(b->dModels);
+  cudaFree(b->dLogTab);
   cudaFree(b->dEns);
   cudaFree(b->dTiles);
   for (void *p : b->dState)
@@ -1681,7 +1765,7 @@ extern "C" int32_t emcg_bulk_create(const emcg_model_desc *models, int32_t n_mod
   b->precision = precision;
   // defaults measured on GB300: the float engine runs the warp-asynchronous
   // kernel with a 4-blocks-per-SM register cap, the double engine the
-  // lockstep kernel without a cap
+  // pooled kernel
   b->queued = precision == EMCG_FP32 ? 2 : 0;
   b->minBlocks = precision == EMCG_FP32 ? 4 : 1;
   b->tsz = precision == EMCG_FP64 ? 8 : 4;

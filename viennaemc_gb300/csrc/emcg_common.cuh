@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "emcg_draws.h"
 #include "emcgpu.h"
 
 namespace emcg {
@@ -33,7 +34,12 @@ template <class T> struct ValleyK {
   T cF[3];                // vogt_i / hbar: dk_ecs = F_ecs cF dt
   int32_t deg;
   int32_t pad_;
+  // rot as a permutation where its entries are 0 and +-1 (kNoPerm: they are
+  // not): for i = 0..2, bits 4 i .. 4 i + 1 the column of row i's entry, bit
+  // 4 i + 2 its sign; bits 16 + 4 i .. the same of the transpose
+  uint32_t perm[EMCG_MAX_DEG];
 };
+constexpr uint32_t kNoPerm = 0xffffffffu;
 
 template <class T> struct MechK {
   int32_t kind, finalValley, nF, pad_;
@@ -355,10 +361,7 @@ __device__ __forceinline__ int energyLevel(const ModelK<T> &M, T E);
 template <>
 __device__ __forceinline__ int energyLevel<double>(const ModelK<double> &M,
                                                    double E) {
-  double f = floor(E / M.dE) - 1;
-  if (!(f >= 0.))
-    return (f == -1.) ? 0 : M.nLevels - 1;
-  return f > (double)(M.nLevels - 1) ? M.nLevels - 1 : (int)f;
+  return levelExact(E, M.dE, M.nLevels);
 }
 template <>
 __device__ __forceinline__ int energyLevel<float>(const ModelK<float> &M,

@@ -111,6 +111,28 @@ inline int32_t validateModel(const emcg_model_desc &m) {
   return EMCG_OK;
 }
 
+// ValleyK::perm of a subvalley frame
+inline uint32_t permOf(const double R[9]) {
+  uint32_t p = 0, cols = 0;
+  for (int i = 0; i < 3; i++) {
+    int at = -1;
+    for (int j = 0; j < 3; j++) {
+      const double r = R[3 * i + j];
+      if (r == 0)
+        continue;
+      if ((r != 1 && r != -1) || at >= 0)
+        return kNoPerm;
+      at = j;
+    }
+    if (at < 0 || (cols >> at & 1))
+      return kNoPerm;
+    cols |= 1u << at;
+    const uint32_t neg = R[3 * i + at] < 0 ? 4u : 0u;
+    p |= ((uint32_t)at | neg) << (4 * i) | ((uint32_t)i | neg) << (16 + 4 * at);
+  }
+  return p;
+}
+
 // Fill the kernel model (without the tables pointer) and the level-major
 // table array of one model.
 template <class T>
@@ -136,9 +158,11 @@ int32_t buildModelK(const emcg_model_desc &m, ModelK<T> &K, std::vector<T> &tabl
     ValleyDerived d = deriveValley(V);
     mcOf[v] = d.mc;
     ValleyK<T> &O = K.v[v];
-    for (int s = 0; s < V.deg; s++)
+    for (int s = 0; s < V.deg; s++) {
       for (int i = 0; i < 9; i++)
         O.rot[s][i] = (T)V.rot[s][i];
+      O.perm[s] = permOf(V.rot[s]);
+    }
     for (int i = 0; i < 3; i++) {
       O.vogt[i] = (T)d.vogt[i];
       O.cF[i] = (T)(d.vogt[i] / kHBAR);
