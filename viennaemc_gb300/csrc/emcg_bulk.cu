@@ -1184,11 +1184,15 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
   EMCG_CUDA(cudaMemcpy(b->dModels, mk.data(), sizeof(ModelK<T>) * nModels,
                        cudaMemcpyHostToDevice));
   if constexpr (sizeof(T) == 8) {
-    double tab[kLogTab];
-    for (int i = 0; i < kLogTab; i++)
-      tab[i] = logTabEntry(i);
-    EMCG_CUDA(cudaMalloc(&b->dLogTab, sizeof(tab)));
-    EMCG_CUDA(cudaMemcpy(b->dLogTab, tab, sizeof(tab), cudaMemcpyHostToDevice));
+    static const std::vector<double> tab = [] { // a constant, formed once
+      std::vector<double> t(kLogTab);
+      for (int i = 0; i < kLogTab; i++)
+        t[i] = logTabEntry(i);
+      return t;
+    }();
+    EMCG_CUDA(cudaMalloc(&b->dLogTab, kLogTab * sizeof(double)));
+    EMCG_CUDA(cudaMemcpy(b->dLogTab, tab.data(), kLogTab * sizeof(double),
+                         cudaMemcpyHostToDevice));
   }
   std::vector<EnsK<T>> ek(nEns);
   for (int e = 0; e < nEns; e++)
@@ -1456,7 +1460,7 @@ static int32_t coulombStepTyped(BulkImpl *b, int nSteps, uint32_t step0, double 
   for (int e = 0; e < b->nEns; e++) {
     const int64_t n = b->count[e], m = n + b->nFixed[e];
     srcNeed = std::max(srcNeed, 4 * m);
-    partNeed = std::max(partNeed, 4 * n * (int64_t)p2pChunks(std::max<int64_t>(n, 1), b->sms));
+    partNeed = std::max(partNeed, 4 * n * (int64_t)p2pPlan<T>(n, m, b->sms).parts);
   }
   EMCG_TRY(growDoubles(b, &b->dSrc, &b->srcCap, srcNeed));
   EMCG_TRY(growDoubles(b, &b->dPart, &b->partCap, partNeed));
@@ -1481,7 +1485,7 @@ static int32_t coulombStepTyped(BulkImpl *b, int nSteps, uint32_t step0, double 
       EMCG_CUDA(cudaGetLastError());
       EMCG_CUDA(p2pLaunch<T>(b->dSrc, b->dSrc + m, b->dSrc + 2 * m, b->dSrc + 3 * m, m, n,
                              b->coulInvCut, b->ens[e].box[0], b->coulImages,
-                             p2pChunks(n, b->sms), b->dPart, b->dCoulF + b->begin[e],
+                             p2pPlan<T>(n, m, b->sms), b->dPart, b->dCoulF + b->begin[e],
                              b->totalCap, b->stream));
     }
     if (b->nTiles > 0) {

@@ -19,15 +19,14 @@ extern "C" int32_t emcg_p2p_coulomb(const double *pos, const double *charge, int
   if (n == 0)
     return EMCG_OK;
   EMCG_CHECK_ARG(pos && charge && force && potential, "NULL array");
-  EMCG_CHECK_ARG(n < (int64_t(1) << 31) * kP2PThreads, "n too large");
-  // enough blocks for every SM: split the sources into chunks when the
-  // targets alone give too few blocks
+  EMCG_CHECK_ARG(n < (int64_t(1) << 39), "n too large");
   int dev = 0, sms = 0;
   EMCG_CUDA(cudaGetDevice(&dev));
   EMCG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int chunks = p2pChunks(n, sms);
+  const P2PPlan plan =
+      precision == EMCG_FP64 ? p2pPlan<double>(n, n, sms) : p2pPlan<float>(n, n, sms);
   double *d = nullptr;
-  EMCG_CUDA(cudaMalloc(&d, (size_t)n * (4 + 4 + 4 * (size_t)chunks) * sizeof(double)));
+  EMCG_CUDA(cudaMalloc(&d, (size_t)n * (4 + 4 + 4 * (size_t)plan.parts) * sizeof(double)));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   auto done = [&](int32_t s) {
     if (e0)
@@ -47,9 +46,9 @@ extern "C" int32_t emcg_p2p_coulomb(const double *pos, const double *charge, int
   cudaEventRecord(e0);
   cudaError_t lerr =
       precision == EMCG_FP64
-          ? p2pLaunch<double>(dx, dx + n, dx + 2 * n, dq, n, n, inv_cutoff, box, images, chunks,
+          ? p2pLaunch<double>(dx, dx + n, dx + 2 * n, dq, n, n, inv_cutoff, box, images, plan,
                               dpart, dout, n, 0)
-          : p2pLaunch<float>(dx, dx + n, dx + 2 * n, dq, n, n, inv_cutoff, box, images, chunks,
+          : p2pLaunch<float>(dx, dx + n, dx + 2 * n, dq, n, n, inv_cutoff, box, images, plan,
                              dpart, dout, n, 0);
   if (lerr != cudaSuccess) {
     setError("p2p launch: %s", cudaGetErrorString(lerr));
