@@ -92,6 +92,10 @@ struct PoissonMG {
   size_t clusterSmem = 0;
   bool clusterEven = true; // the layout's bands have even rows (see clusterDesc)
   bool useCluster = true;
+  // grids without a cluster solve: the first level whose V-cycle runs in one
+  // cluster launch (0: none, every phase is a launch), and that cluster
+  int tailLevel = 0, tailSize = 0;
+  bool tailEven = true;
   // upper bound on clusterSize set by the caller (0: none)
   int clusterCap = 0;
   // the plan for batchFor solves side by side (emcg_device_step_many) under
