@@ -47,11 +47,16 @@ __device__ __forceinline__ double blockMax(double v) {
   return v; // valid in thread 0
 }
 
-// Gauss-Seidel update s / (diagonal): the float smoother divides with the
-// fast approximate division (its error is far below the float multigrid's own
-// 1e-7), the double one exactly
-__device__ __forceinline__ float mgDiv(float s, float den) { return __fdividef(s, den); }
-__device__ __forceinline__ double mgDiv(double s, double den) { return s / den; }
+// Gauss-Seidel update s / (diagonal) as s times the diagonal's reciprocal,
+// which the cluster solve's sweeps form once: the float smoother's by the
+// hardware's approximation (its error is far below the float multigrid's own
+// 1e-7)
+__device__ __forceinline__ float mgRcp(float den) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+  return r;
+}
+__device__ __forceinline__ double mgRcp(double den) { return 1.0 / den; }
 
 __global__ void resetBCKernel(double *pot, const uint8_t *mask, const double *val, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -200,18 +205,34 @@ template <class MT> struct LevelK {
   MT *d, *r, *rho;
 };
 
+// (the sums of the multigrid are written as fused multiply-adds in both solve
+// paths, so that they round alike whatever the compiler would contract)
 template <class MT>
 __device__ __forceinline__ MT applyRow(const LevelK<MT> &L, int i, int x, int y, MT di) {
-  MT s = (L.diag0[i] + L.area[i] * L.rho[i]) * di;
+  MT s = fma(L.area[i], L.rho[i], L.diag0[i]) * di;
   if (x > 0)
-    s -= L.cw[i] * L.d[i - 1];
+    s = fma(-L.cw[i], L.d[i - 1], s);
   if (x < L.nx - 1)
-    s -= L.ce[i] * L.d[i + 1];
+    s = fma(-L.ce[i], L.d[i + 1], s);
   if (y > 0)
-    s -= L.cs[i] * L.d[i - L.nx];
+    s = fma(-L.cs[i], L.d[i - L.nx], s);
   if (y < L.ny - 1)
-    s -= L.cn[i] * L.d[i + L.nx];
+    s = fma(-L.cn[i], L.d[i + L.nx], s);
   return s;
+}
+// the Gauss-Seidel value of node i
+template <class MT>
+__device__ __forceinline__ MT sweepValue(const LevelK<MT> &L, int i, int x, int y) {
+  MT s = L.r[i];
+  if (x > 0)
+    s = fma(L.cw[i], L.d[i - 1], s);
+  if (x < L.nx - 1)
+    s = fma(L.ce[i], L.d[i + 1], s);
+  if (y > 0)
+    s = fma(L.cs[i], L.d[i - L.nx], s);
+  if (y < L.ny - 1)
+    s = fma(L.cn[i], L.d[i + L.nx], s);
+  return s * mgRcp(fma(L.area[i], L.rho[i], L.diag0[i]));
 }
 
 template <class MT> __global__ void smoothKernel(LevelK<MT> L, int color) {
@@ -227,16 +248,7 @@ template <class MT> __global__ void smoothKernel(LevelK<MT> L, int color) {
   int i = y * L.nx + x;
   if (L.fixed[i])
     return;
-  MT s = L.r[i];
-  if (x > 0)
-    s += L.cw[i] * L.d[i - 1];
-  if (x < L.nx - 1)
-    s += L.ce[i] * L.d[i + 1];
-  if (y > 0)
-    s += L.cs[i] * L.d[i - L.nx];
-  if (y < L.ny - 1)
-    s += L.cn[i] * L.d[i + L.nx];
-  L.d[i] = mgDiv(s, L.diag0[i] + L.area[i] * L.rho[i]);
+  L.d[i] = sweepValue(L, i, x, y);
 }
 
 // coarse rhs = P^T (fine residual); coarse reaction by injection; coarse d = 0
@@ -268,7 +280,7 @@ __global__ void restrictKernel(LevelK<MT> F, LevelK<MT> Cc, const int *rxIdx, co
       int i = y * F.nx + x;
       if (F.fixed[i])
         continue;
-      acc += wx * wy * (F.r[i] - applyRow(F, i, x, y, F.d[i]));
+      acc = fma(wx * wy, F.r[i] - applyRow(F, i, x, y, F.d[i]), acc);
     }
   }
   Cc.r[I] = acc;
@@ -285,13 +297,13 @@ __global__ void prolongKernel(LevelK<MT> F, LevelK<MT> Cc, const int *pxIdx, con
   MT wx = (MT)pxW[x], wy = (MT)pyW[y];
   MT v = wx * wy * Cc.d[Y0 * Cc.nx + X0];
   if (wx < MT(1))
-    v += (MT(1) - wx) * wy * Cc.d[Y0 * Cc.nx + X0 + 1];
+    v = fma((MT(1) - wx) * wy, Cc.d[Y0 * Cc.nx + X0 + 1], v);
   if (wy < MT(1)) {
-    v += wx * (MT(1) - wy) * Cc.d[(Y0 + 1) * Cc.nx + X0];
+    v = fma(wx * (MT(1) - wy), Cc.d[(Y0 + 1) * Cc.nx + X0], v);
     if (wx < MT(1))
-      v += (MT(1) - wx) * (MT(1) - wy) * Cc.d[(Y0 + 1) * Cc.nx + X0 + 1];
+      v = fma((MT(1) - wx) * (MT(1) - wy), Cc.d[(Y0 + 1) * Cc.nx + X0 + 1], v);
   }
-  F.d[i] += v;
+  F.d[i] = F.d[i] + v;
 }
 
 // coarsest level: red-black sweeps inside one block
@@ -303,16 +315,7 @@ template <class MT> __global__ void coarseSolveKernel(LevelK<MT> L, int sweeps) 
         int x = i % L.nx, y = i / L.nx;
         if (((x + y) & 1) != color || L.fixed[i])
           continue;
-        MT s = L.r[i];
-        if (x > 0)
-          s += L.cw[i] * L.d[i - 1];
-        if (x < L.nx - 1)
-          s += L.ce[i] * L.d[i + 1];
-        if (y > 0)
-          s += L.cs[i] * L.d[i - L.nx];
-        if (y < L.ny - 1)
-          s += L.cn[i] * L.d[i + L.nx];
-        L.d[i] = mgDiv(s, L.diag0[i] + L.area[i] * L.rho[i]);
+        L.d[i] = sweepValue(L, i, x, y);
       }
       __syncthreads();
     }
@@ -503,157 +506,289 @@ __device__ __forceinline__ T *cRowNearT(const CCtx &c, const CLevel<MT> &L, unsi
   return cRowNear<T>(c, L, off, ly);
 }
 
-template <bool kS, class MT>
-__device__ __forceinline__ void cSmoothT(const CCtx &c, const CLevel<MT> &L, int color) {
-  int r0, r1;
-  cOwnRows(c, L, r0, r1);
-  const int half = (L.nx + 1) / 2, cnt = half * (r1 - r0), stride = cStride(L);
-  for (int t = threadIdx.x; t < cnt; t += stride) {
-    const int ly = L.byHalf.div(t), y = r0 + ly;
-    const int x = 2 * (t - ly * half) + ((y + color) & 1);
-    if (x >= L.nx)
-      continue;
-    // row ly is this CTA's own; its neighbours are too, but at a band edge
-    const Coef<MT> K = cCoef(c, L, cRowNearT<true, uint8_t>(c, L, L.offCls, ly)[x]);
-    if (K.fixed != MT(0))
-      continue;
-    MT *d = cRowNearT<true, MT>(c, L, L.offD, ly);
-    MT s = cRowNearT<true, MT>(c, L, L.offR, ly)[x];
-    if (x > 0)
-      s += K.cw * d[x - 1];
-    if (x < L.nx - 1)
-      s += K.ce * d[x + 1];
-    if (y > 0)
-      s += K.cs * (kS || ly > 0 ? cRowNearT<true, MT>(c, L, L.offD, ly - 1)[x]
-                                : cRowNearT<false, MT>(c, L, L.offD, ly - 1)[x]);
-    if (y < L.ny - 1)
-      s += K.cn * (kS || ly + 1 < L.rowsPer ? cRowNearT<true, MT>(c, L, L.offD, ly + 1)[x]
-                                            : cRowNearT<false, MT>(c, L, L.offD, ly + 1)[x]);
-    d[x] = mgDiv(s, K.diag0 + K.area * cRowNearT<true, MT>(c, L, L.offRho, ly)[x]);
-  }
-}
-template <class MT> __device__ void cSmooth(const CCtx &c, const CLevel<MT> &Lr, int color) {
-  const CLevel<MT> L = Lr; // a private copy: stores to shared memory cannot alias it
-  if (cIdle(L))
-    return;
-  if (L.small)
-    cSmoothT<true>(c, L, color);
-  else
-    cSmoothT<false>(c, L, color);
-  cSync(L);
-}
-
 // Several red-black sweeps over level L with each thread's nodes held in
-// registers: a thread keeps the same nodes over the sweeps, so their position,
-// class, right-hand side and diagonal are read once, and a half sweep reads
-// only the neighbours' corrections.  The arithmetic is cSmoothT's.
+// registers: a thread keeps the same nodes of each colour over the three sweeps,
+// so their position, class, right-hand side and the diagonal's reciprocal are
+// formed once, and a half sweep reads only the coefficients and the neighbours'
+// corrections.  The arithmetic is cSmoothT's.
 //
-// kSweepNodes: nodes of one colour per thread.  Six, for the 2,814-node bands
-// of a 401 x 201 grid, spilled registers: 0.5 % faster there, 1.4 % slower on
-// 201 x 101.
+// A phase costs its longest chain of dependent instructions and what the four
+// warps of a scheduler issue in it, not its work: so a thread's nodes go through
+// each stage side by side, without branches -- all their loads, then the sums,
+// then the stores (see heldNeighbours) --, a warp without nodes keeps the barriers
+// only, and only a neighbour in another CTA's rows goes through distributed shared
+// memory.  Measured on the 201 x 101 resistor's solves (two Newton steps): 0.399 ms
+// with a branch per node and neighbour, 0.402 without branches but with every
+// warp taking part, 0.323 with the idle warps out of the way, 0.301 with two
+// nodes per thread where two are enough and the neighbours' addresses held.  On
+// 401 x 201 0.735 -> 0.613 ms.
+//
+// kSweepNodes: nodes of one colour per thread.
 constexpr int kSweepNodes = 3;
-template <bool kS, int K, class MT>
-__device__ __forceinline__ void cHalfSweep(const CCtx &c, const CLevel<MT> &L, int r0,
-                                           const int (&pos)[2][kSweepNodes],
-                                           const int (&cl)[2][kSweepNodes],
-                                           const MT (&rr)[2][kSweepNodes],
-                                           const MT (&den)[2][kSweepNodes]) {
-#pragma unroll
-  for (int j = 0; j < kSweepNodes; j++) {
-    if (pos[K][j] < 0)
-      continue;
-    const int ly = pos[K][j] >> 16, x = pos[K][j] & 0xffff, y = r0 + ly;
-    const Coef<MT> C = cCoef(c, L, cl[K][j]);
-    MT *d = cRowNearT<true, MT>(c, L, L.offD, ly);
-    MT s = rr[K][j];
-    if (x > 0)
-      s += C.cw * d[x - 1];
-    if (x < L.nx - 1)
-      s += C.ce * d[x + 1];
-    if (y > 0)
-      s += C.cs * (kS || ly > 0 ? cRowNearT<true, MT>(c, L, L.offD, ly - 1)[x]
-                                : cRowNearT<false, MT>(c, L, L.offD, ly - 1)[x]);
-    if (y < L.ny - 1)
-      s += C.cn * (kS || ly + 1 < L.rowsPer ? cRowNearT<true, MT>(c, L, L.offD, ly + 1)[x]
-                                            : cRowNearT<false, MT>(c, L, L.offD, ly + 1)[x]);
-    d[x] = mgDiv(s, den[K][j]);
-  }
-  cSync(L);
+template <class MT> struct Held {
+  unsigned a;    // shared address of the node's correction; 0: no node
+  unsigned s, n; // of the neighbours below and above; bit 0: in another CTA
+  unsigned k;    // shared address of its coefficients
+  MT r, inv;     // right-hand side, 1 / diagonal
+};
+
+__device__ __forceinline__ float ldsAt(unsigned a, float) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double ldsAt(unsigned a, double) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void stsIf(unsigned a, bool on, float v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p st.shared.f32 [%0], %2;\n\t}" ::"r"(a),
+               "r"((unsigned)on), "f"(v)
+               : "memory");
+}
+__device__ __forceinline__ void stsIf(unsigned a, bool on, double v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p st.shared.f64 [%0], %2;\n\t}" ::"r"(a),
+               "r"((unsigned)on), "d"(v)
+               : "memory");
+}
+// on: the value at shared address a, else 0
+__device__ __forceinline__ float ldsIf(unsigned a, bool on, float) {
+  float v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+               "@p ld.shared.f32 %0, [%1];\n\t}"
+               : "=f"(v)
+               : "r"(a), "r"((unsigned)on)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ double ldsIf(unsigned a, bool on, double) {
+  double v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.f64 %0, "
+               "0d0000000000000000;\n\t@p ld.shared.f64 %0, [%1];\n\t}"
+               : "=d"(v)
+               : "r"(a), "r"((unsigned)on)
+               : "memory");
+  return v;
+}
+// the same where the address may be another CTA's (far: a shared::cluster address)
+__device__ __forceinline__ float ldsFar(unsigned a, bool on, bool far, float) {
+  float v;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+               "mov.f32 %0, 0f00000000;\n\t@p ld.shared.f32 %0, [%1];\n\t"
+               "@q ld.shared::cluster.f32 %0, [%1];\n\t}"
+               : "=f"(v)
+               : "r"(a), "r"((unsigned)(on && !far)), "r"((unsigned)(on && far))
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ double ldsFar(unsigned a, bool on, bool far, double) {
+  double v;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+               "mov.f64 %0, 0d0000000000000000;\n\t@p ld.shared.f64 %0, [%1];\n\t"
+               "@q ld.shared::cluster.f64 %0, [%1];\n\t}"
+               : "=d"(v)
+               : "r"(a), "r"((unsigned)(on && !far)), "r"((unsigned)(on && far))
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned mapShared(unsigned a, int rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
 }
 
-// residual r - A d at the held nodes of colour K (cResidualT's arithmetic;
-// the Dirichlet nodes' zeros are written once, at the start of the launch)
-template <bool kS, int K, class MT>
-__device__ __forceinline__ void cResidualHeld(const CCtx &c, const CLevel<MT> &L, int r0,
-                                              const int (&pos)[2][kSweepNodes],
-                                              const int (&cl)[2][kSweepNodes],
-                                              const MT (&rr)[2][kSweepNodes],
-                                              const MT (&den)[2][kSweepNodes]) {
-#pragma unroll
-  for (int j = 0; j < kSweepNodes; j++) {
-    if (pos[K][j] < 0)
-      continue;
-    const int ly = pos[K][j] >> 16, x = pos[K][j] & 0xffff, y = r0 + ly;
-    const Coef<MT> C = cCoef(c, L, cl[K][j]);
-    const MT *d = cRowNearT<true, MT>(c, L, L.offD, ly);
-    MT a = den[K][j] * d[x];
-    if (x > 0)
-      a -= C.cw * d[x - 1];
-    if (x < L.nx - 1)
-      a -= C.ce * d[x + 1];
-    if (y > 0)
-      a -= C.cs * (kS || ly > 0 ? cRowNearT<true, MT>(c, L, L.offD, ly - 1)[x]
-                                : cRowNearT<false, MT>(c, L, L.offD, ly - 1)[x]);
-    if (y < L.ny - 1)
-      a -= C.cn * (kS || ly + 1 < L.rowsPer ? cRowNearT<true, MT>(c, L, L.offD, ly + 1)[x]
-                                            : cRowNearT<false, MT>(c, L, L.offD, ly + 1)[x]);
-    cRowNearT<true, MT>(c, L, L.offRes, ly)[x] = rr[K][j] - a;
-  }
-}
-
+// A level's array in this CTA's rows and the row above and below them: shared
+// addresses, the neighbours' rows mapped.
+struct NearRows {
+  unsigned base, below, above; // own rows; row r0 - 1; row r0 + rowsPer
+};
 template <bool kS, class MT>
-__device__ __forceinline__ void cSweepsHeld(const CCtx &c, const CLevel<MT> &L, int r0, int r1,
-                                            int sweeps, int first, bool residual) {
-  const int half = (L.nx + 1) / 2, cnt = half * (r1 - r0), stride = cStride(L);
-  int pos[2][kSweepNodes], cl[2][kSweepNodes];
-  MT rr[2][kSweepNodes], den[2][kSweepNodes];
+__device__ __forceinline__ NearRows nearRows(const CCtx &c, const CLevel<MT> &L, unsigned off) {
+  NearRows n;
+  n.base = (unsigned)__cvta_generic_to_shared(c.smem) + off;
+  n.below = n.above = n.base;
+  if (!kS) {
+    if (c.rank > 0)
+      n.below = mapShared(n.base + (unsigned)((L.rowsPer - 1) * L.nx * sizeof(MT)), c.rank - 1);
+    if (c.rank + 1 < (int)cg::this_cluster().num_blocks())
+      n.above = mapShared(n.base, c.rank + 1);
+  }
+  return n;
+}
+// element x of local row ly, where on
+template <bool kS, class MT>
+__device__ __forceinline__ MT nearLoad(const CLevel<MT> &L, const NearRows &n, int ly, int x,
+                                       bool on) {
+  if (kS)
+    return ldsIf(n.base + (unsigned)((ly * L.nx + x) * (int)sizeof(MT)), on, MT());
+  const bool lo = ly < 0, hi = ly >= L.rowsPer;
+  const unsigned row = lo ? n.below : hi ? n.above : n.base + (unsigned)(ly * L.nx * (int)sizeof(MT));
+  return ldsFar(row + (unsigned)(x * (int)sizeof(MT)), on, lo || hi, MT());
+}
+
+// the corrections beside a thread's nodes: past a row's end the next row's or the
+// padding, past the domain's edge the node's own, all with a zero coefficient
+template <bool kS, int N, class MT>
+__device__ __forceinline__ void heldNeighbours(const Held<MT> (&h)[N], MT (&d)[N][4]) {
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-#pragma unroll
-    for (int j = 0; j < kSweepNodes; j++) {
-      pos[k][j] = -1;
-      cl[k][j] = 0;
-      rr[k][j] = MT(0);
-      den[k][j] = MT(1);
-      const int t = threadIdx.x + j * stride;
-      if (t >= cnt)
-        continue;
-      const int ly = L.byHalf.div(t), y = r0 + ly;
-      const int x = 2 * (t - ly * half) + ((y + k) & 1);
-      if (x >= L.nx)
-        continue;
-      const int q = cRowNearT<true, uint8_t>(c, L, L.offCls, ly)[x];
-      const Coef<MT> K = cCoef(c, L, q);
-      if (K.fixed != MT(0))
-        continue;
-      pos[k][j] = (ly << 16) | x;
-      cl[k][j] = q;
-      rr[k][j] = cRowNearT<true, MT>(c, L, L.offR, ly)[x];
-      den[k][j] = K.diag0 + K.area * cRowNearT<true, MT>(c, L, L.offRho, ly)[x];
+  for (int j = 0; j < N; j++) {
+    d[j][0] = ldsAt(h[j].a - (unsigned)sizeof(MT), MT());
+    d[j][1] = ldsAt(h[j].a + (unsigned)sizeof(MT), MT());
+    if (kS) {
+      d[j][2] = ldsAt(h[j].s, MT());
+      d[j][3] = ldsAt(h[j].n, MT());
+    } else {
+      d[j][2] = ldsFar(h[j].s & ~1u, true, h[j].s & 1u, MT());
+      d[j][3] = ldsFar(h[j].n & ~1u, true, h[j].n & 1u, MT());
     }
   }
+}
+__device__ __forceinline__ void coefAt(unsigned a, float (&c)[4]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void coefAt(unsigned a, double (&c)[4]) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(c[0]), "=d"(c[1]) : "r"(a) : "memory");
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
+               : "=d"(c[2]), "=d"(c[3])
+               : "r"(a + 16u)
+               : "memory");
+}
+
+// the nodes threadIdx.x + (j0 + j) * stride of a colour of this CTA's rows; an
+// absent or Dirichlet node reads the level's first and stores nothing
+template <bool kS, int N, class MT>
+__device__ __forceinline__ void loadHeld(const CCtx &c, const CLevel<MT> &L, const NearRows &nd,
+                                         int r0, int cnt, int j0, int colour, Held<MT> (&h)[N]) {
+  const int half = (L.nx + 1) / 2, stride = cStride(L);
+  const unsigned base = nd.base - L.offD, row = (unsigned)(L.nx * (int)sizeof(MT));
+  int q[N];
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    const int t = threadIdx.x + (j0 + j) * stride, u = t < cnt ? t : 0;
+    const int ly = L.byHalf.div(u), y = r0 + ly, x = 2 * (u - ly * half) + ((y + colour) & 1);
+    const bool on = t < cnt && x < L.nx;
+    const int i = on ? ly * L.nx + x : 0;
+    h[j].a = nd.base + (unsigned)(i * (int)sizeof(MT));
+    q[j] = *reinterpret_cast<const uint8_t *>(c.smem + L.offCls + i);
+    h[j].s = on && y > 0 ? h[j].a - row : h[j].a;
+    h[j].n = on && y < L.ny - 1 ? h[j].a + row : h[j].a;
+    if (!kS) {
+      if (on && y > 0 && ly == 0)
+        h[j].s = (nd.below + (unsigned)(x * (int)sizeof(MT))) | 1u;
+      if (on && y < L.ny - 1 && ly + 1 == L.rowsPer)
+        h[j].n = (nd.above + (unsigned)(x * (int)sizeof(MT))) | 1u;
+    }
+    h[j].k = on ? 1u : 0u;
+  }
+  MT e[N][4];
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    const unsigned k = base + L.offTab + (unsigned)(8 * q[j] * (int)sizeof(MT));
+    h[j].r = ldsAt(h[j].a + (L.offR - L.offD), MT());
+    h[j].inv = ldsAt(h[j].a + (L.offRho - L.offD), MT());
+    coefAt(k + 4u * (unsigned)sizeof(MT), e[j]); // area, diagonal, fixed
+    q[j] = (int)h[j].k;
+    h[j].k = k;
+  }
+#pragma unroll
+  for (int j = 0; j < N; j++)
+    h[j].inv = q[j] && e[j][2] == MT(0) ? mgRcp(fma(e[j][0], h[j].inv, e[j][1])) : MT(0);
+}
+
+// a half sweep over nodes of a colour
+template <bool kS, int N, class MT>
+__device__ __forceinline__ void cHalfSweep(const CCtx &c, const CLevel<MT> &L, const NearRows &nd,
+                                           int r0, const Held<MT> (&h)[N]) {
+  MT f[N][4], d[N][4];
+#pragma unroll
+  for (int j = 0; j < N; j++)
+    coefAt(h[j].k, f[j]);
+  heldNeighbours<kS>(h, d);
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    MT s = h[j].r;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      s = fma(f[j][q], d[j][q], s);
+    stsIf(h[j].a, h[j].inv != MT(0), s * h[j].inv);
+  }
+}
+
+// residual r - A d of the correction equation at nodes of a colour, as
+// restrictKernel evaluates it (the Dirichlet nodes' zeros are written once, at
+// the start of the launch)
+template <bool kS, int N, class MT>
+__device__ __forceinline__ void cResidualHeld(const CCtx &c, const CLevel<MT> &L,
+                                              const NearRows &nd, int r0,
+                                              const Held<MT> (&h)[N]) {
+  MT f[N][4], e[N][4], d[N][4], rho[N], o[N];
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    coefAt(h[j].k, f[j]);
+    coefAt(h[j].k + 4u * (unsigned)sizeof(MT), e[j]); // area, diagonal, fixed
+    rho[j] = ldsAt(h[j].a + (L.offRho - L.offD), MT());
+    o[j] = ldsAt(h[j].a, MT());
+  }
+  heldNeighbours<kS>(h, d);
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    MT s = fma(e[j][0], rho[j], e[j][1]) * o[j];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      s = fma(-f[j][q], d[j][q], s);
+    stsIf(h[j].a + (L.offRes - L.offD), h[j].inv != MT(0), h[j].r - s);
+  }
+}
+
+template <bool kS, int N, class MT>
+__device__ __forceinline__ void cSweepsHeld(const CCtx &c, const CLevel<MT> &L, int r0, int cnt,
+                                            int sweeps, int first, bool residual) {
+  const NearRows nd = nearRows<kS>(c, L, L.offD);
+  Held<MT> h[2][N];
+  loadHeld<kS>(c, L, nd, r0, cnt, 0, 0, h[0]);
+  loadHeld<kS>(c, L, nd, r0, cnt, 0, 1, h[1]);
   for (int s = 0; s < sweeps; s++) {
     if (first == 0) {
-      cHalfSweep<kS, 0>(c, L, r0, pos, cl, rr, den);
-      cHalfSweep<kS, 1>(c, L, r0, pos, cl, rr, den);
+      cHalfSweep<kS>(c, L, nd, r0, h[0]);
+      cSync(L);
+      cHalfSweep<kS>(c, L, nd, r0, h[1]);
+      cSync(L);
     } else {
-      cHalfSweep<kS, 1>(c, L, r0, pos, cl, rr, den);
-      cHalfSweep<kS, 0>(c, L, r0, pos, cl, rr, den);
+      cHalfSweep<kS>(c, L, nd, r0, h[1]);
+      cSync(L);
+      cHalfSweep<kS>(c, L, nd, r0, h[0]);
+      cSync(L);
     }
   }
   if (residual) {
-    cResidualHeld<kS, 0>(c, L, r0, pos, cl, rr, den);
-    cResidualHeld<kS, 1>(c, L, r0, pos, cl, rr, den);
+    cResidualHeld<kS>(c, L, nd, r0, h[0]);
+    cResidualHeld<kS>(c, L, nd, r0, h[1]);
+    cSync(L);
+  }
+}
+
+// the same for bands of more nodes than a thread holds, kBatchNodes at a time
+constexpr int kBatchNodes = 4;
+template <bool kS, class MT>
+__device__ __forceinline__ void cSweepsBatch(const CCtx &c, const CLevel<MT> &L, int r0, int cnt,
+                                             int sweeps, int first, bool residual) {
+  const NearRows nd = nearRows<kS>(c, L, L.offD);
+  const int per = (cnt + cStride(L) - 1) / cStride(L);
+  for (int s = 0; s < 2 * sweeps + (residual ? 1 : 0); s++) {
+    const bool res = s == 2 * sweeps;
+    for (int k = 0; k < (res ? 2 : 1); k++)
+      for (int j0 = 0; j0 < per; j0 += kBatchNodes) {
+        Held<MT> h[kBatchNodes];
+        loadHeld<kS>(c, L, nd, r0, cnt, j0, res ? k : (first + s) & 1, h);
+        if (res)
+          cResidualHeld<kS>(c, L, nd, r0, h);
+        else
+          cHalfSweep<kS>(c, L, nd, r0, h);
+      }
     cSync(L);
   }
 }
@@ -669,60 +804,32 @@ __device__ void cSmoothSweeps(const CCtx &c, const CLevel<MT> &Lr, int sweeps, i
     return;
   int r0, r1;
   cOwnRows(c, L, r0, r1);
-  const int cnt = (L.nx + 1) / 2 * (r1 - r0);
-  if (cnt <= kSweepNodes * cStride(L) && L.nx <= 0xffff && r1 - r0 <= 0x7fff) {
-    if (L.small)
-      cSweepsHeld<true>(c, L, r0, r1, sweeps, first, residual);
+  const int cnt = (L.nx + 1) / 2 * (r1 - r0), stride = cStride(L);
+  // nodes of a colour of this warp's first thread: a warp without any only keeps
+  // the barriers (four warps share a scheduler, so what they issue in vain
+  // delays the others)
+  const int mine = (cnt - (int)(threadIdx.x & ~31u) + stride - 1) / stride;
+  if (mine <= 0) {
+    for (int s = 0; s < 2 * sweeps + (residual ? 1 : 0); s++)
+      cSync(L);
+  } else if (cnt <= kSweepNodes * stride) {
+    if (L.small && mine == 1)
+      cSweepsHeld<true, 1>(c, L, r0, cnt, sweeps, first, residual);
+    else if (L.small && mine == 2)
+      cSweepsHeld<true, 2>(c, L, r0, cnt, sweeps, first, residual);
+    else if (L.small)
+      cSweepsHeld<true, kSweepNodes>(c, L, r0, cnt, sweeps, first, residual);
+    else if (mine == 1)
+      cSweepsHeld<false, 1>(c, L, r0, cnt, sweeps, first, residual);
+    else if (mine == 2)
+      cSweepsHeld<false, 2>(c, L, r0, cnt, sweeps, first, residual);
     else
-      cSweepsHeld<false>(c, L, r0, r1, sweeps, first, residual);
-    return;
+      cSweepsHeld<false, kSweepNodes>(c, L, r0, cnt, sweeps, first, residual);
+  } else if (L.small) {
+    cSweepsBatch<true>(c, L, r0, cnt, sweeps, first, residual);
+  } else {
+    cSweepsBatch<false>(c, L, r0, cnt, sweeps, first, residual);
   }
-  for (int s = 0; s < sweeps; s++) {
-    cSmooth(c, L, first);
-    cSmooth(c, L, 1 - first);
-  }
-  if (residual)
-    cResidual(c, L);
-}
-
-// residual r - A d of the correction equation at this CTA's nodes of level F
-// (0 at Dirichlet nodes), as restrictKernel evaluates it
-template <bool kS, class MT>
-__device__ __forceinline__ void cResidualT(const CCtx &c, const CLevel<MT> &F) {
-  int r0, r1;
-  cOwnRows(c, F, r0, r1);
-  const int cnt = F.nx * (r1 - r0), stride = cStride(F);
-  for (int t = threadIdx.x; t < cnt; t += stride) {
-    const int ly = F.byNx.div(t), y = r0 + ly, x = t - ly * F.nx;
-    const Coef<MT> K = cCoef(c, F, cRowNearT<true, uint8_t>(c, F, F.offCls, ly)[x]);
-    MT res = MT(0);
-    if (K.fixed == MT(0)) {
-      const MT *d = cRowNearT<true, MT>(c, F, F.offD, ly);
-      MT a = (K.diag0 + K.area * cRowNearT<true, MT>(c, F, F.offRho, ly)[x]) * d[x];
-      if (x > 0)
-        a -= K.cw * d[x - 1];
-      if (x < F.nx - 1)
-        a -= K.ce * d[x + 1];
-      if (y > 0)
-        a -= K.cs * (kS || ly > 0 ? cRowNearT<true, MT>(c, F, F.offD, ly - 1)[x]
-                                  : cRowNearT<false, MT>(c, F, F.offD, ly - 1)[x]);
-      if (y < F.ny - 1)
-        a -= K.cn * (kS || ly + 1 < F.rowsPer ? cRowNearT<true, MT>(c, F, F.offD, ly + 1)[x]
-                                              : cRowNearT<false, MT>(c, F, F.offD, ly + 1)[x]);
-      res = cRowNearT<true, MT>(c, F, F.offR, ly)[x] - a;
-    }
-    cRowNearT<true, MT>(c, F, F.offRes, ly)[x] = res;
-  }
-}
-template <class MT> __device__ void cResidual(const CCtx &c, const CLevel<MT> &Fr) {
-  const CLevel<MT> F = Fr;
-  if (cIdle(F))
-    return;
-  if (F.small)
-    cResidualT<true>(c, F);
-  else
-    cResidualT<false>(c, F);
-  cSync(F);
 }
 
 // coarse rows whose injection row mapY[Y] this CTA holds: [Y0, Y1)
@@ -744,43 +851,79 @@ __device__ __forceinline__ void cRestrictRows(const CCtx &c, const CLevel<MT> &F
   Y1 = r1 == F.ny ? Cc.ny : min(Cc.ny, (r1 + 1) / 2);
 }
 
-// coarse right-hand side P^T (fine residual), reaction by injection, d = 0
+// row Y of an array of the coarse level, wherever it lives
 template <bool kS, class MT>
+__device__ __forceinline__ char *cCoarseRow(const CCtx &c, const CLevel<MT> &Cc, int Y) {
+  // (without the array's offset: one owner for the row's arrays)
+  if (kS)
+    return c.smem + (size_t)Y * Cc.nx * sizeof(MT);
+  if (Cc.small)
+    return (c.rank == 0 ? c.smem : c.base[0]) + (size_t)Y * Cc.nx * sizeof(MT);
+  const int owner = Cc.byRows.div(Y);
+  return (owner == c.rank ? c.smem : c.base[owner]) +
+         (size_t)(Y - owner * Cc.rowsPer) * Cc.nx * sizeof(MT);
+}
+
+// coarse right-hand side P^T (fine residual), reaction by injection, d = 0; a
+// coarse node is a Dirichlet node where the fine node under it is
+// (U: coarse nodes of a thread side by side)
+template <bool kS, int U, class MT>
 __device__ __forceinline__ void cRestrictT(const CCtx &c, const CLevel<MT> &F,
-                                        const CLevel<MT> &Cc) {
-  int Y0, Y1;
+                                           const CLevel<MT> &Cc) {
+  int Y0, Y1, r0, r1;
   cRestrictRows(c, F, Cc, Y0, Y1);
+  cOwnRows(c, F, r0, r1);
   const int cnt = Cc.nx * (Y1 - Y0), stride = cStride(F);
-  for (int t = threadIdx.x; t < cnt; t += stride) {
-    const int q = Cc.byNx.div(t), Y = Y0 + q, X = t - q * Cc.nx;
-    cRowT<kS, MT>(c, Cc, Cc.offD, Y)[X] = MT(0);
-    cRowT<kS, MT>(c, Cc, Cc.offRho, Y)[X] =
-        cRowT<kS, MT>(c, F, F.offRho, cTab<int>(c, F.offMapY)[Y])[cTab<int>(c, F.offMapX)[X]];
-    const Coef<MT> KC = cCoef(c, Cc, cRowT<kS, uint8_t>(c, Cc, Cc.offCls, Y)[X]);
-    MT acc = MT(0);
-    if (KC.fixed == MT(0)) {
-      MT wxs[3];
-      int xs[3];
+  const NearRows nr = nearRows<kS>(c, F, F.offRes);
+  for (int t0 = threadIdx.x; t0 < cnt; t0 += U * stride) {
+    int X[U], Y[U], xm[U], lym[U], xs[U][3], lys[U][3];
+    MT wx[U][3], wy[U][3], rho[U], fixed[U], v[U][3][3];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = t0 + u * stride < cnt ? t0 + u * stride : t0;
+      const int q = Cc.byNx.div(t);
+      Y[u] = Y0 + q;
+      X[u] = t - q * Cc.nx;
+      xm[u] = cTab<int>(c, F.offMapX)[X[u]];
+      lym[u] = cTab<int>(c, F.offMapY)[Y[u]] - r0;
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        wxs[k] = (MT)cTab<float>(c, F.offRxW)[3 * X + k];
-        xs[k] = cTab<int>(c, F.offRxI)[3 * X + k];
-      }
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        const MT wy = (MT)cTab<float>(c, F.offRyW)[3 * Y + b];
-        if (wy == MT(0))
-          continue;
-        const MT *res = cRowT<kS, MT>(c, F, F.offRes, cTab<int>(c, F.offRyI)[3 * Y + b]);
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-          if (wxs[a] == MT(0))
-            continue;
-          acc += wxs[a] * wy * res[xs[a]];
-        }
+        wx[u][k] = (MT)cTab<float>(c, F.offRxW)[3 * X[u] + k];
+        wy[u][k] = (MT)cTab<float>(c, F.offRyW)[3 * Y[u] + k];
+        xs[u][k] = cTab<int>(c, F.offRxI)[3 * X[u] + k];
+        lys[u][k] = cTab<int>(c, F.offRyI)[3 * Y[u] + k] - r0;
       }
     }
-    cRowT<kS, MT>(c, Cc, Cc.offR, Y)[X] = acc;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = lym[u] * F.nx + xm[u];
+      const int q = *reinterpret_cast<const uint8_t *>(c.smem + F.offCls + i);
+      rho[u] = reinterpret_cast<const MT *>(c.smem + F.offRho)[i];
+      fixed[u] = reinterpret_cast<const MT *>(c.smem + F.offTab)[8 * q + 6];
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) // a zero weight reads nothing (its row may be far)
+          v[u][b][a] = nearLoad<kS>(F, nr, lys[u][b], xs[u][a],
+                                    wx[u][a] != MT(0) && wy[u][b] != MT(0));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      MT acc = MT(0);
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+          acc = fma(wx[u][a] * wy[u][b], v[u][b][a], acc);
+      if (fixed[u] != MT(0))
+        acc = MT(0);
+      if (t0 + u * stride < cnt) {
+        char *row = cCoarseRow<kS>(c, Cc, Y[u]) + X[u] * sizeof(MT);
+        *reinterpret_cast<MT *>(row + Cc.offD) = MT(0);
+        *reinterpret_cast<MT *>(row + Cc.offRho) = rho[u];
+        *reinterpret_cast<MT *>(row + Cc.offR) = acc;
+      }
+    }
   }
 }
 template <class MT>
@@ -789,35 +932,60 @@ __device__ void cRestrict(const CCtx &c, const CLevel<MT> &Fr, const CLevel<MT> 
   if (cIdle(F))
     return;
   if (F.small)
-    cRestrictT<true>(c, F, Cc);
+    cRestrictT<true, 1>(c, F, Cc);
   else
-    cRestrictT<false>(c, F, Cc);
+    cRestrictT<false, 1>(c, F, Cc);
   cSync(F);
 }
 
-template <bool kS, class MT>
+// The coarse correction added to the fine nodes of colour 0: those of colour 1,
+// with which the sweeps that follow begin, are formed anew from their neighbours.
+// (U: fine nodes of a thread side by side)
+template <bool kS, int U, class MT>
 __device__ __forceinline__ void cProlongT(const CCtx &c, const CLevel<MT> &F,
-                                        const CLevel<MT> &Cc) {
+                                          const CLevel<MT> &Cc) {
   int r0, r1;
   cOwnRows(c, F, r0, r1);
-  const int cnt = F.nx * (r1 - r0), stride = cStride(F);
-  for (int t = threadIdx.x; t < cnt; t += stride) {
-    const int ly = F.byNx.div(t), y = r0 + ly, x = t - ly * F.nx;
-    if (cCoef(c, F, cRowNearT<true, uint8_t>(c, F, F.offCls, ly)[x]).fixed != MT(0))
-      continue;
-    const int X0 = cTab<int>(c, F.offPxI)[x], Y0 = cTab<int>(c, F.offPyI)[y];
-    const MT wx = (MT)cTab<float>(c, F.offPxW)[x], wy = (MT)cTab<float>(c, F.offPyW)[y];
-    const MT *c0 = cRowT<kS, MT>(c, Cc, Cc.offD, Y0);
-    MT v = wx * wy * c0[X0];
-    if (wx < MT(1))
-      v += (MT(1) - wx) * wy * c0[X0 + 1];
-    if (wy < MT(1)) {
-      const MT *c1 = cRowT<kS, MT>(c, Cc, Cc.offD, Y0 + 1);
-      v += wx * (MT(1) - wy) * c1[X0];
-      if (wx < MT(1))
-        v += (MT(1) - wx) * (MT(1) - wy) * c1[X0 + 1];
+  const int half = (F.nx + 1) / 2, cnt = half * (r1 - r0), stride = cStride(F);
+  for (int t0 = threadIdx.x; t0 < cnt; t0 += U * stride) {
+    int i[U], X0[U], Y0[U];
+    bool on[U];
+    MT wx[U], wy[U], v[U][4], d[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = t0 + u * stride < cnt ? t0 + u * stride : t0;
+      const int ly = F.byHalf.div(t), x = 2 * (t - ly * half) + ((r0 + ly) & 1);
+      on[u] = t0 + u * stride < cnt && x < F.nx;
+      const int xx = x < F.nx ? x : 0;
+      i[u] = ly * F.nx + xx;
+      X0[u] = cTab<int>(c, F.offPxI)[xx];
+      Y0[u] = cTab<int>(c, F.offPyI)[r0 + ly];
+      wx[u] = (MT)cTab<float>(c, F.offPxW)[xx];
+      wy[u] = (MT)cTab<float>(c, F.offPyW)[r0 + ly];
     }
-    cRowNearT<true, MT>(c, F, F.offD, ly)[x] += v;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int q = *reinterpret_cast<const uint8_t *>(c.smem + F.offCls + i[u]);
+      const bool bx = wx[u] < MT(1), by = wy[u] < MT(1);
+      const MT *c0 = reinterpret_cast<const MT *>(cCoarseRow<kS>(c, Cc, Y0[u]) + Cc.offD) + X0[u];
+      const MT *c1 =
+          reinterpret_cast<const MT *>(cCoarseRow<kS>(c, Cc, Y0[u] + (by ? 1 : 0)) + Cc.offD) + X0[u];
+      v[u][0] = c0[0];
+      v[u][1] = bx ? c0[1] : MT(0);
+      v[u][2] = by ? c1[0] : MT(0);
+      v[u][3] = bx && by ? c1[1] : MT(0);
+      d[u] = reinterpret_cast<const MT *>(c.smem + F.offD)[i[u]];
+      on[u] = on[u] && reinterpret_cast<const MT *>(c.smem + F.offTab)[8 * q + 6] == MT(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      MT s = wx[u] * wy[u] * v[u][0];
+      s = fma((MT(1) - wx[u]) * wy[u], v[u][1], s);
+      s = fma(wx[u] * (MT(1) - wy[u]), v[u][2], s);
+      s = fma((MT(1) - wx[u]) * (MT(1) - wy[u]), v[u][3], s);
+      if (on[u])
+        reinterpret_cast<MT *>(c.smem + F.offD)[i[u]] = d[u] + s;
+    }
   }
 }
 template <class MT>
@@ -826,9 +994,9 @@ __device__ void cProlong(const CCtx &c, const CLevel<MT> &Fr, const CLevel<MT> &
   if (cIdle(F))
     return;
   if (F.small)
-    cProlongT<true>(c, F, Cc);
+    cProlongT<true, 1>(c, F, Cc);
   else
-    cProlongT<false>(c, F, Cc);
+    cProlongT<false, 2>(c, F, Cc);
   cSync(F);
 }
 
@@ -846,28 +1014,19 @@ template <class MT> __device__ void cCoarse(const CCtx &c, const CLevel<MT> &L, 
       const Coef<MT> K = cCoef(c, L, live ? cRowT<true, uint8_t>(c, L, L.offCls, y)[x] : 0);
       MT *dp = live ? cRowT<true, MT>(c, L, L.offD, y) + x : nullptr;
       const MT r = live ? cRowT<true, MT>(c, L, L.offR, y)[x] : MT(0);
-      const MT den = live ? K.diag0 + K.area * cRowT<true, MT>(c, L, L.offRho, y)[x] : MT(1);
+      const MT den = live ? fma(K.area, cRowT<true, MT>(c, L, L.offRho, y)[x], K.diag0) : MT(1);
+      const MT inv = mgRcp(den);
       const bool upd = live && K.fixed == MT(0);
       MT d = live ? *dp : MT(0);
-      for (int it = 0; it < sweeps; it++) {
-        for (int color = 0; color < 2; color++) {
-          const MT dw = __shfl_sync(0xffffffffu, d, (i + 31) & 31);
-          const MT de = __shfl_sync(0xffffffffu, d, (i + 1) & 31);
-          const MT ds = __shfl_sync(0xffffffffu, d, (i - L.nx + 32) & 31);
-          const MT dn = __shfl_sync(0xffffffffu, d, (i + L.nx) & 31);
-          if (upd && ((x + y) & 1) == color) {
-            MT s = r;
-            if (x > 0)
-              s += K.cw * dw;
-            if (x < L.nx - 1)
-              s += K.ce * de;
-            if (y > 0)
-              s += K.cs * ds;
-            if (y < L.ny - 1)
-              s += K.cn * dn;
-            d = mgDiv(s, den);
-          }
-        }
+      // (beyond the domain's edge the coefficient is zero)
+      const int lw = (i + 31) & 31, le = (i + 1) & 31, ls = (i - L.nx + 32) & 31,
+                ln = (i + L.nx) & 31;
+      const bool upd0 = upd && ((x + y) & 1) == 0, upd1 = upd && ((x + y) & 1) == 1;
+      for (int it = 0; it < 2 * sweeps; it++) {
+        const MT dw = __shfl_sync(0xffffffffu, d, lw), de = __shfl_sync(0xffffffffu, d, le);
+        const MT ds = __shfl_sync(0xffffffffu, d, ls), dn = __shfl_sync(0xffffffffu, d, ln);
+        const MT s = fma(K.cn, dn, fma(K.cs, ds, fma(K.ce, de, fma(K.cw, dw, r))));
+        d = (it & 1 ? upd1 : upd0) ? s * inv : d;
       }
       if (live)
         *dp = d;
@@ -886,14 +1045,14 @@ template <class MT> __device__ void cCoarse(const CCtx &c, const CLevel<MT> &L, 
         MT *d = cRowT<true, MT>(c, L, L.offD, y);
         MT s = cRowT<true, MT>(c, L, L.offR, y)[x];
         if (x > 0)
-          s += K.cw * d[x - 1];
+          s = fma(K.cw, d[x - 1], s);
         if (x < L.nx - 1)
-          s += K.ce * d[x + 1];
+          s = fma(K.ce, d[x + 1], s);
         if (y > 0)
-          s += K.cs * cRowT<true, MT>(c, L, L.offD, y - 1)[x];
+          s = fma(K.cs, cRowT<true, MT>(c, L, L.offD, y - 1)[x], s);
         if (y < L.ny - 1)
-          s += K.cn * cRowT<true, MT>(c, L, L.offD, y + 1)[x];
-        d[x] = mgDiv(s, K.diag0 + K.area * cRowT<true, MT>(c, L, L.offRho, y)[x]);
+          s = fma(K.cn, cRowT<true, MT>(c, L, L.offD, y + 1)[x], s);
+        d[x] = s * mgRcp(fma(K.area, cRowT<true, MT>(c, L, L.offRho, y)[x], K.diag0));
       }
       cSync(L);
     }
@@ -1119,6 +1278,17 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   // cluster barrier makes them visible
   auto stageRest = [&]() {
     copyCls(1, M.nLev);
+    for (int l = 0; l < M.nLev; l++) { // the padding around d, and rows past the grid's
+      const CLevel<MT> &L = M.L[l];
+      int r0, r1;
+      cOwnRows(c, L, r0, r1);
+      const int q = (int)(16 / sizeof(MT));
+      MT *d = reinterpret_cast<MT *>(smem + L.offD);
+      if ((int)threadIdx.x < q)
+        d[(int)threadIdx.x - q] = MT(0);
+      for (int k = L.nx * (r1 - r0) + threadIdx.x; k < L.nx * L.rowsPer + q; k += blockDim.x)
+        d[k] = MT(0);
+    }
     for (int l = 0; l + 1 < M.nLev; l++) {
       const CLevel<MT> &L = M.L[l];
       int r0, r1;
@@ -1302,7 +1472,10 @@ CMG<MT> clusterDesc(const MGSet &P, int CL, size_t *bytes, bool evenRows = true)
     c.byHalf.set((c.nx + 1) / 2);
     c.byRows.set(c.rowsPer);
     const size_t cells = (size_t)c.rowsPer * c.nx;
-    c.offD = take(cells * sizeof(MT));
+    // zeroed padding before and after d: the sweeps read past the ends of its first
+    // and last rows
+    take(16);
+    c.offD = take(cells * sizeof(MT) + 16);
     c.offR = take(cells * sizeof(MT));
     c.offRho = take(cells * sizeof(MT));
     c.offRes = l + 1 < M.nLev ? take(cells * sizeof(MT)) : 0;
