@@ -2072,9 +2072,13 @@ extern "C" int32_t emcg_get_state_f32(emcg_handle *h, int32_t e, emcg_state_f32 
   EMCG_CUDA(cudaStreamSynchronize(b->stream));
   float *dst[9] = {s->kx, s->ky, s->kz, s->px, s->py, s->pz, s->energy, s->tau, s->grain_tau};
   for (int f = 0; f < 9; f++)
-    if (dst[f] && n)
+    if (dst[f] && n) {
+      touchPages(dst[f], n * sizeof(float));
       EMCG_CUDA(cudaMemcpyAsync(dst[f], static_cast<float *>(b->dState[f]) + base,
                                 n * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
+    }
+  if (s->meta && n)
+    touchPages(s->meta, n * sizeof(uint32_t));
   if (s->meta && n)
     EMCG_CUDA(cudaMemcpyAsync(s->meta, b->dMeta + base, n * sizeof(uint32_t),
                               cudaMemcpyDeviceToHost, b->stream));
@@ -2387,8 +2391,8 @@ extern "C" int32_t emcg_bulk_get_coulomb(emcg_handle *h, int32_t e, double *forc
   for (int v = 0; v < 4; v++) {
     double *dst = v < 3 ? (force ? force + (size_t)v * n : nullptr) : potential;
     if (dst && n)
-      EMCG_CUDA(cudaMemcpy(dst, b->dCoulF + (size_t)v * b->totalCap + b->begin[e],
-                           (size_t)n * sizeof(double), cudaMemcpyDeviceToHost));
+      EMCG_CUDA(copyToCaller(dst, b->dCoulF + (size_t)v * b->totalCap + b->begin[e],
+                             (size_t)n * sizeof(double)));
   }
   return EMCG_OK;
 }

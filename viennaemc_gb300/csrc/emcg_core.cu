@@ -53,6 +53,28 @@ const void *mappedHostRange(const void *p, size_t bytes) {
   return it->second.dev + off;
 }
 
+void touchPages(void *dst, size_t bytes) {
+  // below some pages the copy's own faults cost less than asking what dst is
+  if (!dst || bytes < 16384)
+    return;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered)
+    return;
+  volatile char *p = static_cast<volatile char *>(dst);
+  for (size_t o = 0; o < bytes; o += 4096)
+    p[o] = 0;
+  p[bytes - 1] = 0;
+}
+
+cudaError_t copyToCaller(void *dst, const void *src, size_t bytes) {
+  touchPages(dst, bytes);
+  return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+}
+
 } // namespace emcg
 
 extern "C" const char *emcg_last_error(void) {

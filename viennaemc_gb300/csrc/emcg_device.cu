@@ -1512,7 +1512,7 @@ extern "C" int32_t emcg_device_get_grid(emcg_handle *h, int32_t which, double *v
   if (which == EMCG_GRID_EX || which == EMCG_GRID_EY) {
     void *e = which == EMCG_GRID_EX ? d->dEx : d->dEy;
     if (d->precision == EMCG_FP64) {
-      EMCG_CUDA(cudaMemcpy(v, e, n * sizeof(double), cudaMemcpyDeviceToHost));
+      EMCG_CUDA(copyToCaller(v, e, n * sizeof(double)));
     } else {
       std::vector<float> f(n);
       EMCG_CUDA(cudaMemcpy(f.data(), e, n * sizeof(float), cudaMemcpyDeviceToHost));
@@ -1526,7 +1526,7 @@ extern "C" int32_t emcg_device_get_grid(emcg_handle *h, int32_t which, double *v
                 : which == EMCG_GRID_CONC    ? d->dConc
                                              : nullptr;
   EMCG_CHECK_ARG(src, "unknown grid %d", which);
-  EMCG_CUDA(cudaMemcpy(v, src, n * sizeof(double), cudaMemcpyDeviceToHost));
+  EMCG_CUDA(copyToCaller(v, src, n * sizeof(double)));
   return EMCG_OK;
 }
 

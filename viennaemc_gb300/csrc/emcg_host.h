@@ -46,6 +46,16 @@ const char *statusName(int32_t s);
 // space), else nullptr: only such ranges are read by kernels over the host link.
 const void *mappedHostRange(const void *p, size_t bytes);
 
+// Copy from the device to the caller's array, whose pages are touched first: a
+// copy into ordinary memory that no one has written yet (a freshly zeroed
+// array) takes its page faults from the GPU's side, one after another.  Measured
+// on 64 KB pages, 643 KB: 550 to 2600 us into untouched memory, 18 us into
+// touched, 11 us to touch it.  On the null stream, complete on return.
+cudaError_t copyToCaller(void *dst, const void *src, size_t bytes);
+// The touch alone, for asynchronous copies (a no-op for page-locked and device
+// memory).
+void touchPages(void *dst, size_t bytes);
+
 struct BulkImpl;
 struct DeviceImpl;
 

@@ -55,6 +55,8 @@ extern "C" int32_t emcg_p2p_coulomb(const double *pos, const double *charge, int
     return done(EMCG_ERR_CUDA);
   }
   cudaEventRecord(e1);
+  touchPages(force, (size_t)n * 3 * sizeof(double)); // while the sums run
+  touchPages(potential, (size_t)n * sizeof(double));
   cudaError_t err = cudaGetLastError();
   if (err == cudaSuccess)
     err = cudaEventSynchronize(e1);
