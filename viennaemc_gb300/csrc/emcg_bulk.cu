@@ -59,7 +59,7 @@ __device__ __forceinline__ int bulkParticleStep(const ModelK<T> &M, const EnsK<T
       err = e;
       break;
     }
-    T nt = -m_log(rng.ulog()) * tauOf(M, valley, region);
+    T nt = -drawLog(M, rng.ulog()) * tauOf(M, valley, region);
     tau += nt;
     driftBulk(M.v[valley], sub, EK.fv[valley][sub], nt < tRem ? nt : tRem, k, E, pos, kN,
               EK.box);
@@ -72,7 +72,7 @@ __device__ __forceinline__ int bulkParticleStep(const ModelK<T> &M, const EnsK<T
       grainScatter(M, k, rng);
       toEcs(M.v[valley].rot[sub], k[0], k[1], k[2], kN);
     }
-    gtau = -m_log(rng.ulog()) * M.grainTau;
+    gtau = -drawLog(M, rng.ulog()) * M.grainTau;
   }
   return err;
 }
@@ -110,7 +110,7 @@ __device__ __forceinline__ int bulkParticleStepF(const ModelK<T> &M, const EnsK<
       err = e;
       break;
     }
-    T nt = -m_log(rng.ulog()) * tauOf(M, valley, region);
+    T nt = -drawLog(M, rng.ulog()) * tauOf(M, valley, region);
     tau += nt;
     fvOf(fv);
     driftBulk(M.v[valley], sub, fv, nt < tRem ? nt : tRem, k, E, pos, kN, EK.box);
@@ -123,7 +123,7 @@ __device__ __forceinline__ int bulkParticleStepF(const ModelK<T> &M, const EnsK<
       grainScatter(M, k, rng);
       toEcs(M.v[valley].rot[sub], k[0], k[1], k[2], kN);
     }
-    gtau = -m_log(rng.ulog()) * M.grainTau;
+    gtau = -drawLog(M, rng.ulog()) * M.grainTau;
   }
   return err;
 }
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(256, MINB)
         e = scatterParticle(M, k, E, valley, sub, region, rng);
         if (e)
           break;
-        T nt = -m_log(rng.ulog()) * tauOf(M, valley, region);
+        T nt = -drawLog(M, rng.ulog()) * tauOf(M, valley, region);
         tau += nt;
         driftBulk(M.v[valley], sub, EK.fv[valley][sub], nt < tRem ? nt : tRem, k, E, pos, kN,
                   EK.box);
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(256, MINB)
           B.n1[me] = kN[1];
           B.n2[me] = kN[2];
         }
-        gtau = -m_log(rng.ulog()) * M.grainTau;
+        gtau = -drawLog(M, rng.ulog()) * M.grainTau;
       }
       B.gtau[me] = gtau;
       const ValleyK<T> &V = M.v[valley];
@@ -615,7 +615,7 @@ __global__ void bulkInitKernel(StateK<T> st, const ModelK<T> *__restrict__ model
   int valley = (int)m_floor((T)M.nV * rng.ulog());
   const ValleyK<T> &V = M.v[valley];
   int sub = (int)m_floor((T)V.deg * rng.ulog());
-  T E = T(-1.5) * (T)Vt * m_log(rng.ulog());
+  T E = T(-1.5) * (T)Vt * drawLog(M, rng.ulog());
   T k[3];
   randomDirection(V.cK * m_sqrt(gammaOf(V, E)), rng, k);
   if (coords) {
@@ -624,8 +624,8 @@ __global__ void bulkInitKernel(StateK<T> st, const ModelK<T> *__restrict__ model
       if ((c[d] == 0 && k[d] < T(0)) || (c[d] == ext[d] - 1 && k[d] > T(0)))
         k[d] *= T(-1);
   }
-  T tau = -m_log(rng.ulog()) * tauOf(M, valley, 0);
-  T gtau = -m_log(rng.ulog()) * M.grainTau;
+  T tau = -drawLog(M, rng.ulog()) * tauOf(M, valley, 0);
+  T gtau = -drawLog(M, rng.ulog()) * M.grainTau;
   int64_t g = begin + i;
   st.kx[g] = k[0];
   st.ky[g] = k[1];
@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(256, MINB)
           live = false;
           s = nSteps;
         } else {
-          tau = -m_log(rng.ulog()) * tauOf(M, valley, region);
+          tau = -drawLog(M, rng.ulog()) * tauOf(M, valley, region);
         }
         toEcs(M.v[valley].rot[sub], k[0], k[1], k[2], kE);
       }
@@ -930,7 +930,7 @@ __global__ void __launch_bounds__(256, MINB)
                 grainScatter(M, k, rng);
                 toEcs(R, k[0], k[1], k[2], kE);
               }
-              gtau = -m_log(rng.ulog()) * M.grainTau;
+              gtau = -drawLog(M, rng.ulog()) * M.grainTau;
             }
             const int slot = ws * 32 + lane;
             winE[slot] = E;
@@ -1108,7 +1108,6 @@ template <class T> struct StepArgs {
   int chunk;
   int nVmax;
   int pass;
-  const double *logT; // the pooled kernel's table of log
   double *obs;
   const uint64_t *words;
   const int64_t *off;
@@ -1169,6 +1168,8 @@ template <class T>
 static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nModels,
                            const emcg_ensemble_desc *ens, int nEns) {
   std::vector<ModelK<T>> mk(nModels);
+  if (sizeof(T) == 8)
+    EMCG_TRY(uploadLogTable(&b->dLogTab));
   b->dTables.assign(nModels, nullptr);
   b->rates.resize(nModels);
   for (int i = 0; i < nModels; i++) {
@@ -1179,21 +1180,11 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
     EMCG_CUDA(cudaMemcpy(b->dTables[i], tab.data(), tab.size() * sizeof(T),
                          cudaMemcpyHostToDevice));
     mk[i].tables = (const T *)b->dTables[i];
+    mk[i].logT = b->dLogTab;
   }
   EMCG_CUDA(cudaMalloc(&b->dModels, sizeof(ModelK<T>) * nModels));
   EMCG_CUDA(cudaMemcpy(b->dModels, mk.data(), sizeof(ModelK<T>) * nModels,
                        cudaMemcpyHostToDevice));
-  if constexpr (sizeof(T) == 8) {
-    static const std::vector<double> tab = [] { // a constant, formed once
-      std::vector<double> t(kLogTab);
-      for (int i = 0; i < kLogTab; i++)
-        t[i] = logTabEntry(i);
-      return t;
-    }();
-    EMCG_CUDA(cudaMalloc(&b->dLogTab, kLogTab * sizeof(double)));
-    EMCG_CUDA(cudaMemcpy(b->dLogTab, tab.data(), kLogTab * sizeof(double),
-                         cudaMemcpyHostToDevice));
-  }
   std::vector<EnsK<T>> ek(nEns);
   for (int e = 0; e < nEns; e++)
     buildEnsK<T>(ens[e], mk[ens[e].model], models[ens[e].model], b->begin[e], 0, ek[e]);
@@ -1375,9 +1366,7 @@ template <class T> static int32_t graphFor(BulkImpl *b, int ns, size_t smem, siz
                    &a.err};
   void *asy[13] = {&a.st,   &a.src,   &a.srcEns, &a.mp,   &a.ep,  &a.tiles, &a.ns,
                    &a.step0, &a.chunk, &a.nVmax,  &a.pass, &a.obs, &a.err};
-  a.logT = b->dLogTab;
-  void *pol[10] = {&a.st,    &a.mp,    &a.ep,   &a.tiles, &a.ns,
-                   &a.step0, &a.nVmax, &a.logT, &a.obs,   &a.err};
+  void *pol[9] = {&a.st, &a.mp, &a.ep, &a.tiles, &a.ns, &a.step0, &a.nVmax, &a.obs, &a.err};
   static_assert(sizeof(asy) <= sizeof(b->gParams), "kernel parameters exceed the buffer");
   if (b->tilePool)
     std::memcpy(b->gParams, pol, sizeof(pol));
@@ -1565,10 +1554,10 @@ static int32_t launchStepTiles(BulkImpl *b, const StateK<T> &st, int ns, uint32_
     const size_t psmem = poolSmemFor(pool, b->nVmax == 1);
     if (b->nVmax == 1)
       poolKernel<true>(pool)<<<nT, 32, psmem, b->stream>>>(
-          st, mp, ep, tiles, ns, s0, b->nVmax, b->dLogTab, b->dObs, b->dErr);
+          st, mp, ep, tiles, ns, s0, b->nVmax, b->dObs, b->dErr);
     else
       poolKernel<false>(pool)<<<nT, 32, psmem, b->stream>>>(
-          st, mp, ep, tiles, ns, s0, b->nVmax, b->dLogTab, b->dObs, b->dErr);
+          st, mp, ep, tiles, ns, s0, b->nVmax, b->dObs, b->dErr);
   } else if (b->minBlocks >= 4 && b->blockThreads <= 256) {
     bulkStepKernel<T, false, 4><<<nT, b->blockThreads, smem, b->stream>>>(
         st, mp, ep, tiles, ns, s0, b->chunk, b->nVmax, b->dObs, nullptr,

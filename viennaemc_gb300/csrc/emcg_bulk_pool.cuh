@@ -32,7 +32,6 @@
 #pragma once
 
 #include "emcg_common.cuh"
-#include "emcg_draws.h"
 #include "emcg_log.h"
 
 namespace emcg {
@@ -55,43 +54,6 @@ template <int G> __host__ __device__ constexpr size_t poolSmemBytes(bool one) {
   constexpr size_t P = PoolShape<G>::P, PW = PoolShape<G>::PW;
   return sizeof(double) * 2 * kPoolWindow * PW + (one ? 0 : kPoolWindow * P) +
          (G > 1 ? sizeof(double) * kPoolFields * P + 4 * 4 * P + 32 : 0);
-}
-
-// 1 / sqrt(t) for normal t > 0: the hardware's approximation (about 20 bits)
-// and one step of Householder's method of third order (Householder 1970):
-// with e = 1 - t y^2, y (1 + e / 2 + 3 e^2 / 8)
-__device__ __forceinline__ double poolRsqrt(double t) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
-  const double e = fma(-t * y, y, 1.0);
-  return fma(fma(0.375, e, 0.5), y * e, y);
-}
-
-// 1 / d for normal d > 0: the hardware's approximation (about 20 bits) and
-// y (1 + r + r^2), r = 1 - d y (the geometric series to third order)
-__device__ __forceinline__ double poolRcp(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double r = fma(-d, y, 1.0);
-  return fma(y, fma(r, r, r), y);
-}
-
-// sqrt(x): x / sqrt(x) corrected once; 0, subnormals, infinities, negative
-// values and NaN go to the library's
-__device__ __forceinline__ double poolSqrt(double x) {
-  const uint32_t h = (uint32_t)__double2hiint(x);
-  if (h - 0x00100000u >= 0x7fe00000u)
-    return sqrt(x);
-  const double y = poolRsqrt(x), s = x * y;
-  return fma(fma(-s, s, x), 0.5 * y, s);
-}
-
-// a < b for a double a and b >= 0 without a double-precision instruction: the
-// bit patterns of non-negative doubles order like the values, those of
-// negative ones are negative integers; a NaN is not below
-__device__ __forceinline__ bool poolBelow(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return x < y && (unsigned long long)x <= 0xfff0000000000000ull;
 }
 
 // One Philox block and the draws' log out of line: the code of a pass is run a
@@ -160,28 +122,6 @@ struct PoolEl {
   uint32_t words, meta, kind; // draws consumed in the step; PoolKind | mechanism << 8
 };
 
-// a rotated into the subvalley's frame (toEcs) or back (toDev): where the
-// frame's axes are the device's, a permutation with signs, which gives the same
-// values without double-precision instructions
-template <bool kBack>
-__device__ __forceinline__ void poolRotate(const ValleyK<double> &V, int sub, const double a[3],
-                                           double o[3]) {
-  const uint32_t p = V.perm[sub];
-  if (p == kNoPerm) {
-    if (kBack)
-      toDev(V.rot[sub], a[0], a[1], a[2], o);
-    else
-      toEcs(V.rot[sub], a[0], a[1], a[2], o);
-    return;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const uint32_t q = p >> ((kBack ? 16 : 0) + 4 * i);
-    const double x = (q & 3) == 0 ? a[0] : (q & 3) == 1 ? a[1] : a[2];
-    o[i] = __hiloint2double(__double2hiint(x) ^ (int)((q & 4) << 29), __double2loint(x));
-  }
-}
-
 // The summed ellipse-frame displacement into the device frame and the periodic
 // box, as flushPos of the float engine.
 __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, const double box[3],
@@ -192,11 +132,11 @@ __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, con
     d[i] = p.d[i] * V.vogt[i];
     p.d[i] = 0.0;
   }
-  poolRotate<true>(V, sub, d, dd);
+  rotate<true>(V, sub, d, dd);
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     double c = p.x[i] + dd[i];
-    if (poolBelow(c, 0.0) || poolBelow(box[i], c))
+    if (belowD(c, 0.0) || belowD(box[i], c))
       c -= box[i] * floor(c / box[i]);
     p.x[i] = c;
   }
@@ -204,8 +144,7 @@ __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, con
 
 // the grain timer ran out (basicBulkParticleHandler.hpp:215-219)
 __device__ __forceinline__ void poolGrain(const ModelK<double> &M, const EnsK<double> &EK,
-                                       uint32_t pid, uint32_t step, const double *logT,
-                                       PoolEl &p) {
+                                       uint32_t pid, uint32_t step, PoolEl &p) {
   PoolDraws rng(EK, pid, step, p.words);
   if (M.grain) {
     const double *R = M.v[p.meta & 0xff].rot[(p.meta >> 8) & 0xff];
@@ -214,7 +153,7 @@ __device__ __forceinline__ void poolGrain(const ModelK<double> &M, const EnsK<do
     grainScatter(M, k, rng);
     toEcs(R, k[0], k[1], k[2], p.k);
   }
-  p.gtau = -poolLog(rng.ulog(), logT) * M.grainTau;
+  p.gtau = -poolLog(rng.ulog(), M.logT) * M.grainTau;
 }
 
 struct PoolValley { // a valley's constants of the free flight
@@ -226,11 +165,10 @@ struct PoolValley { // a valley's constants of the free flight
 // vd then the velocity along the field.
 __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<double> &EK,
                                            const ModelK<double> &M, int valley, int sub,
-                                           uint32_t pid, uint32_t step0, const double *logT,
-                                           PoolEl &p, double &vd) {
+                                           uint32_t pid, uint32_t step0, PoolEl &p, double &vd) {
   const double *fv = EK.fv[valley][sub];
   const double rem = EK.dt - p.in;
-  const bool ev = poolBelow(p.tau, rem);
+  const bool ev = belowD(p.tau, rem);
   const double t = ev ? p.tau : rem;
   double kO[3];
 #pragma unroll
@@ -238,19 +176,9 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
     kO[i] = p.k[i];
     p.k[i] = fma(fv[i], t, kO[i]);
   }
-  // E = g / (1 + s), s = sqrt(1 + 2 alpha g) = 1 + 2 alpha E; both quotients
-  // corrected once, so E is as close as with the library's square root and
-  // division
-  const double g = V.cE * fma(p.k[2], p.k[2], fma(p.k[1], p.k[1], p.k[0] * p.k[0]));
-  const double u = fma(V.alpha2, g, 1.0);
-  const double rs = poolRsqrt(u), hs = 0.5 * rs;
-  double s = u * rs;
-  s = fma(fma(-s, s, u), hs, s);
-  const double den = 1.0 + s;
-  const double inv = poolRcp(den);
-  p.E = g * inv;
-  p.E = fma(fma(-den, p.E, g), inv, p.E);
-  const double vh = V.cX * hs; // hbar / (2 mc (1 + 2 alpha E))
+  double rs;
+  p.E = energyRoot(V.cE, V.alpha2, fma(p.k[2], p.k[2], fma(p.k[1], p.k[1], p.k[0] * p.k[0])), rs);
+  const double vh = V.cX * (0.5 * rs); // hbar / (2 mc (1 + 2 alpha E))
   const double c = vh * t;
 #pragma unroll
   for (int i = 0; i < 3; i++)
@@ -263,8 +191,8 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
   p.tau -= t;
   p.in = 0.0;
   p.gtau -= EK.dt;
-  if (poolBelow(p.gtau, 0.0) || __double_as_longlong(p.gtau) == 0)
-    poolGrain(M, EK, pid, step0 + (uint32_t)p.step, logT, p);
+  if (belowD(p.gtau, 0.0) || __double_as_longlong(p.gtau) == 0)
+    poolGrain(M, EK, pid, step0 + (uint32_t)p.step, p);
   const double *gd = EK.g[valley][sub];
   const double gk = fma(gd[2], p.k[2], fma(gd[1], p.k[1], gd[0] * p.k[0]));
   vd = vh * (gk + gk);
@@ -278,8 +206,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
 // state: a mechanism's draws are counted here and taken in poolScatter.
 template <bool kOne>
 __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<double> &M,
-                                          uint32_t pid, uint32_t step0, const double *logT,
-                                          PoolEl &p) {
+                                          uint32_t pid, uint32_t step0, PoolEl &p) {
   PoolDraws rng(EK, pid, step0 + (uint32_t)p.step, p.words);
   int valley = kOne ? 0 : (int)(p.meta & 0xff);
   const int region = p.meta >> 16;
@@ -310,7 +237,7 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
       }
     }
   }
-  p.tau = -poolLog(rng.ulog(), logT) * tauOf(M, valley, region);
+  p.tau = -poolLog(rng.ulog(), M.logT) * tauOf(M, valley, region);
   if (p.kind == kFlight)
     p.words = rng.i;
   return 0;
@@ -342,16 +269,16 @@ __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK
       const double cK = M.v[valley].cK;
       n2 = cK * cK * gammaOf(M.v[valley], p.E);
     }
-    const double nk = poolSqrt(n2);
+    const double nk = sqrtD(n2);
     const double ct = 1.0 - 2.0 * rng.u01(), r1 = rng.u01();
     double sn, cs;
     sincospi(2.0 * r1, &sn, &cs);
-    const double ns = nk * poolSqrt(1.0 - ct * ct);
+    const double ns = nk * sqrtD(1.0 - ct * ct);
     kd[0] = ns * cs;
     kd[1] = ns * sn;
     kd[2] = nk * ct;
   }
-  poolRotate<false>(M.v[valley], sub, kd, p.k);
+  rotate<false>(M.v[valley], sub, kd, p.k);
   p.words = rng.i + 1; // the free flight's draw is taken
   p.kind = kFlight;
 }
@@ -363,8 +290,8 @@ template <int G, bool kOne>
 __global__ void __launch_bounds__(32)
     bulkStepPoolKernel(StateK<double> st, const ModelK<double> *__restrict__ models,
                        const EnsK<double> *__restrict__ ens, const Tile *__restrict__ tiles,
-                       int nSteps, uint32_t step0, int nVmax, const double *__restrict__ logT,
-                       double *__restrict__ obs, int *__restrict__ err) {
+                       int nSteps, uint32_t step0, int nVmax, double *__restrict__ obs,
+                       int *__restrict__ err) {
   constexpr int P = PoolShape<G>::P, PW = PoolShape<G>::PW, W = kPoolWindow;
   constexpr bool kReg = G == 1;
   extern __shared__ __align__(16) double poolSmem[];
@@ -410,7 +337,7 @@ __global__ void __launch_bounds__(32)
       const int64_t gi = tl.begin + j;
       p.meta = st.meta[gi];
       const double kd[3] = {st.kx[gi], st.ky[gi], st.kz[gi]};
-      poolRotate<false>(M.v[p.meta & 0xff], (p.meta >> 8) & 0xff, kd, p.k);
+      rotate<false>(M.v[p.meta & 0xff], (p.meta >> 8) & 0xff, kd, p.k);
       p.x[0] = st.px[gi];
       p.x[1] = st.py[gi];
       p.x[2] = st.pz[gi];
@@ -537,7 +464,7 @@ __global__ void __launch_bounds__(32)
       const PoolValley V = kOne ? one : PoolValley{VK.cE, 2.0 * VK.alpha, VK.cX};
       const int slot = p.step & (W - 1);
       double vd;
-      if (poolFlight(V, EK, M, valley, sub, pid, step0, logT, p, vd)) {
+      if (poolFlight(V, EK, M, valley, sub, pid, step0, p, vd)) {
         wE[slot * PW + j] = p.E;
         wD[slot * PW + j] = vd;
         if (!kOne)
@@ -550,7 +477,7 @@ __global__ void __launch_bounds__(32)
     } else if (pick == kSelect) {
       if (!kReg)
         p.E = f[6 * P + j];
-      const int e = poolSelect<kOne>(EK, M, pid, step0, logT, p);
+      const int e = poolSelect<kOne>(EK, M, pid, step0, p);
       if (e) {
         myErr = e;
         p.kind = kDone;
@@ -590,7 +517,7 @@ __global__ void __launch_bounds__(32)
     const int sub = (p.meta >> 8) & 0xff;
     poolFlush(V, sub, EK.box, p);
     double k[3];
-    poolRotate<true>(V, sub, p.k, k);
+    rotate<true>(V, sub, p.k, k);
     st.kx[gi] = k[0];
     st.ky[gi] = k[1];
     st.kz[gi] = k[2];

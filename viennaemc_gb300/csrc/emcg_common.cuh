@@ -10,6 +10,8 @@
 #include <stdint.h>
 
 #include "emcg_draws.h"
+#include "emcg_fp64.cuh"
+#include "emcg_log.h"
 #include "emcgpu.h"
 
 namespace emcg {
@@ -59,6 +61,7 @@ template <class T> struct ModelK {
   T tauMax[EMCG_MAX_TABLESETS];
   uint8_t tsMech[EMCG_MAX_TABLESETS][EMCG_MAX_MECH];
   const T *tables; // level-major per set: tables[tsOff + L * nT + t]
+  const double *logT; // logTab()'s table (double engines)
   int32_t surfKind[4]; // EMCG_SURFACE_* per device boundary (XMIN, XMAX, YMIN, YMAX)
   T surfParam[4];      // its specularity or roughness height [m]
 };
@@ -95,13 +98,13 @@ __host__ __device__ inline uint32_t packMeta(int v, int s, int r) {
 // precision-dispatched math.  Float uses the SFU approximations: the float
 // engine is a statistical engine checked against the double one.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double m_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double m_sqrt(double x) { return sqrtD(x); }
 __device__ __forceinline__ float m_sqrt(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ double m_div(double a, double b) { return a / b; }
+__device__ __forceinline__ double m_div(double a, double b) { return divD(a, b); }
 __device__ __forceinline__ float m_div(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double m_log(double x) { return log(x); }
 __device__ __forceinline__ float m_log(float x) { return __logf(x); }
@@ -112,9 +115,7 @@ __device__ __forceinline__ float m_exp(float x) { return expf(x); }
 __device__ __forceinline__ void m_sincos(double x, double *s, double *c) { sincos(x, s, c); }
 __device__ __forceinline__ void m_sincos(float x, float *s, float *c) { sincosf(x, s, c); }
 __device__ __forceinline__ void m_sincos2pi(double u, double *s, double *c) {
-  double phi = 2 * kPI * u; // 2 * emcPi<T>() * rand (include/emcUtil.hpp:132)
-  *s = sin(phi);
-  *c = cos(phi);
+  sincospi(2.0 * u, s, c); // of 2 * emcPi<T>() * rand (include/emcUtil.hpp:132)
 }
 __device__ __forceinline__ void m_sincos2pi(float u, float *s, float *c) {
   // the angle 2 pi u - pi in [-pi, pi) keeps the SFU in its accurate range;
@@ -153,13 +154,6 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1,
   o[1] = c1;
   o[2] = c2;
   o[3] = c3;
-}
-
-// libstdc++ generate_canonical<double,53>(mt19937_64): (double)w / 2^64,
-// clamped below 1; then uniform_real_distribution: u * (b - a) + a.
-__device__ __forceinline__ double canonical53(uint64_t w) {
-  double r = __dmul_rn(__ull2double_rn(w), 0x1p-64);
-  return r >= 1.0 ? 0x1.fffffffffffffp-1 : r;
 }
 
 // Counter-based source: counter = (particle, step, call, stream), key = seed.
@@ -214,15 +208,18 @@ template <> struct PhiloxSrc<double> {
     return w;
   }
   __device__ __forceinline__ uint32_t pick(uint32_t n) {
-    return f32 ? __umulhi(word32(), n) : (uint32_t)(word() % (uint64_t)n);
+    if (f32)
+      return __umulhi(word32(), n);
+    const uint64_t w = word();
+    return (n & (n - 1)) == 0 ? (uint32_t)w & (n - 1) : (uint32_t)(w % (uint64_t)n);
   }
   __device__ __forceinline__ double u01() {
-    return f32 ? (double)((float)(word32() >> 8) * 0x1p-24f) : canonical53(word());
+    return f32 ? (double)((float)(word32() >> 8) * 0x1p-24f) : canonicalBits(word());
   }
   __device__ __forceinline__ double ulog() {
     if (f32)
       return (double)fmaf((float)(word32() >> 8) * 0x1p-24f, 1.f - 1e-6f, 1e-6f);
-    return __dadd_rn(__dmul_rn(canonical53(word()), 1. - 1e-6), 1e-6);
+    return __dadd_rn(__dmul_rn(canonicalBits(word()), 1. - 1e-6), 1e-6);
   }
   __device__ __forceinline__ bool failed() const { return false; }
 };
@@ -290,9 +287,9 @@ struct ReplaySrc {
   __device__ __forceinline__ uint32_t pick(uint32_t n) {
     return (uint32_t)(word() % (uint64_t)n);
   }
-  __device__ __forceinline__ double u01() { return canonical53(word()); }
+  __device__ __forceinline__ double u01() { return canonicalBits(word()); }
   __device__ __forceinline__ double ulog() {
-    return __dadd_rn(__dmul_rn(canonical53(word()), 1. - 1e-6), 1e-6);
+    return __dadd_rn(__dmul_rn(canonicalBits(word()), 1. - 1e-6), 1e-6);
   }
   __device__ __forceinline__ bool failed() const { return bad != 0; }
 };
@@ -313,6 +310,42 @@ __device__ __forceinline__ void toDev(const T *R, T a0, T a1, T a2, T o[3]) {
   o[2] = a0 * R[2] + a1 * R[5] + a2 * R[8];
 }
 
+// a in the subvalley's frame (toEcs), or back (kBack, toDev).  Double: where the
+// frame's axes are the device's, a permutation with signs, which gives the same
+// values without double-precision instructions.
+template <bool kBack, class T>
+__device__ __forceinline__ void rotate(const ValleyK<T> &V, int sub, const T a[3], T o[3]) {
+  if constexpr (sizeof(T) == 8) {
+    const uint32_t p = V.perm[sub];
+    if (p != kNoPerm) {
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const uint32_t q = p >> ((kBack ? 16 : 0) + 4 * i);
+        const double x = (q & 3) == 0 ? a[0] : (q & 3) == 1 ? a[1] : a[2];
+        o[i] = __hiloint2double(__double2hiint(x) ^ (int)((q & 4) << 29), __double2loint(x));
+      }
+      return;
+    }
+  }
+  if (kBack)
+    toDev(V.rot[sub], a[0], a[1], a[2], o);
+  else
+    toEcs(V.rot[sub], a[0], a[1], a[2], o);
+}
+
+// A free flight's energy and reciprocal root, double: with g = hbar^2 k^2 / (mc q)
+// and s = sqrt(1 + 2 alpha g) = 1 + 2 alpha E, E = g / (1 + s) and 1 / s.  Both
+// quotients corrected once, so E is as close as with the library's square root
+// and division.
+__device__ __forceinline__ double energyRoot(double cE, double alpha2, double k2, double &rs) {
+  const double g = cE * k2, u = fma(alpha2, g, 1.0);
+  rs = rsqrtD(u);
+  double s = u * rs;
+  s = fma(fma(-s, s, u), 0.5 * rs, s);
+  const double den = 1.0 + s, inv = rcpD(den), E = g * inv;
+  return fma(fma(-den, E, g), inv, E);
+}
+
 // E(k) = gamma / (1 + sqrt(1 + 2 alpha gamma)), gamma = hbar^2 k^2/(mc q)  (:109-113)
 template <class T>
 __device__ __forceinline__ T energyOf(const ValleyK<T> &V, T sq) {
@@ -331,6 +364,24 @@ template <class T, int DIM>
 __device__ __forceinline__ void drift(const ValleyK<T> &V, int sub,
                                       const T fv[3], T dt, T k[3], T &E,
                                       T *pos, T kN[3]) {
+  if constexpr (sizeof(T) == 8) {
+    double kO[3], d[3], dd[3], rs;
+    rotate<false>(V, sub, k, kO);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      kN[i] = fma(fv[i], dt, kO[i]);
+    rotate<true>(V, sub, kN, k);
+    E = energyRoot(V.cE, 2.0 * V.alpha, fma(kN[2], kN[2], fma(kN[1], kN[1], kN[0] * kN[0])), rs);
+    const double c = (V.cX * (0.5 * rs)) * dt; // hbar dt / (2 mc (1 + 2 E alpha))
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      d[i] = V.vogt[i] * (kN[i] + kO[i]) * c;
+    rotate<true>(V, sub, d, dd);
+#pragma unroll
+    for (int i = 0; i < DIM; i++)
+      pos[i] += dd[i];
+    return;
+  }
   const T *R = V.rot[sub];
   T kO[3];
   toEcs(R, k[0], k[1], k[2], kO);
@@ -361,7 +412,7 @@ __device__ __forceinline__ int energyLevel(const ModelK<T> &M, T E);
 template <>
 __device__ __forceinline__ int energyLevel<double>(const ModelK<double> &M,
                                                    double E) {
-  return levelExact(E, M.dE, M.nLevels);
+  return levelFast(E, M.dE, M.invdE, M.nLevels);
 }
 template <>
 __device__ __forceinline__ int energyLevel<float>(const ModelK<float> &M,
@@ -461,6 +512,13 @@ __device__ __forceinline__ void applyMechanism(const ModelK<T> &M,
   }
 }
 
+// a <= b for table entries and draws (non-negative doubles order like their
+// bit patterns)
+__device__ __forceinline__ bool notAbove(float a, float b) { return a <= b; }
+__device__ __forceinline__ bool notAbove(double a, double b) {
+  return __double_as_longlong(a) <= __double_as_longlong(b);
+}
+
 // emcScatterHandler::scatterParticle (include/emcScatterHandler.hpp:148-170).
 // Returns EMCG_ERR_OUT_OF_TABLE if the (valley, region) pair has no tables.
 template <class T, class R>
@@ -476,7 +534,7 @@ __device__ __forceinline__ int scatterParticle(const ModelK<T> &M, T k[3],
   int L = energyLevel(M, E);
   T rnd = rng.u01();
   const T *row = M.tables + M.tsOff[ts] + (int64_t)L * nT;
-  if (rnd > ldg(row + nT - 1))
+  if (!notAbove(rnd, ldg(row + nT - 1)))
     return 0; // self-scattering
   // the first t with row[t-1] <= rnd < row[t] (row[-1] = 0): the row is
   // cumulative, so nondecreasing, and t is the number of entries <= rnd.  The
@@ -484,10 +542,16 @@ __device__ __forceinline__ int scatterParticle(const ModelK<T> &M, T k[3],
   int t = 0;
 #pragma unroll 4
   for (int q = 0; q < nT; q++)
-    t += ldg(row + q) <= rnd ? 1 : 0;
+    t += notAbove(ldg(row + q), rnd) ? 1 : 0;
   if (t < nT) // t = nT: rnd equals the last entry, no mechanism (as the loop above)
     applyMechanism(M, M.m[M.tsMech[ts][t]], k, E, valley, sub, region, rng);
   return 0;
+}
+
+// log of a draw in (0, 1]
+__device__ __forceinline__ float drawLog(const ModelK<float> &, float u) { return m_log(u); }
+__device__ __forceinline__ double drawLog(const ModelK<double> &M, double u) {
+  return logTab(u, M.logT);
 }
 
 // free-flight constant of (valley, region); 2e-15 s without tables

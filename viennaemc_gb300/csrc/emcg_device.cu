@@ -37,7 +37,16 @@ struct DevK {
 };
 
 template <class T> __device__ __forceinline__ int roundIdx(T v, double h, double invh);
-template <> __device__ __forceinline__ int roundIdx<double>(double v, double h, double) {
+// double: the nearest whole number of v (1 / h) in fixed point; within 2^-20 of
+// halfway, where v / h may round to the other side, by the division
+template <> __device__ __forceinline__ int roundIdx<double>(double v, double h, double invh) {
+  uint64_t f;
+  if (fixedOf(v * invh, f)) {
+    f += 1u << 19;
+    const uint32_t frac = (uint32_t)f & 0xfffffu;
+    if (frac - 1u < 0xffffeu)
+      return (int)(f >> 20);
+  }
   return (int)round(v / h);
 }
 template <> __device__ __forceinline__ int roundIdx<float>(float v, double, double invh) {
@@ -46,8 +55,26 @@ template <> __device__ __forceinline__ int roundIdx<float>(float v, double, doub
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 template <class T> __device__ __forceinline__ T floorDiv(T v, double h, double invh, int &m);
-template <> __device__ __forceinline__ double floorDiv<double>(double v, double h, double, int &m) {
-  double q = v / h;
+// double: the quotient corrected once; within 2^-20 of a whole number, where its
+// neighbour's floor may differ, the division
+template <>
+__device__ __forceinline__ double floorDiv<double>(double v, double h, double invh, int &m) {
+  double q = v * invh;
+  q = fma(fma(-q, h, v), invh, q);
+  uint64_t x;
+  if (fixedOf(q, x)) {
+    const uint32_t frac = (uint32_t)x & 0xfffffu;
+    if (frac - 1u < 0xffffeu) {
+      m = (int)(x >> 20);
+      const int e = (int)((uint32_t)__double2hiint(q) >> 20) - 1023;
+      // q without its fraction's bits
+      const double f = e < 0 ? 0.0
+                             : __longlong_as_double(__double_as_longlong(q) &
+                                                    (long long)(~0ull << (52 - e)));
+      return q - f;
+    }
+  }
+  q = v / h;
   double f = floor(q);
   m = (int)f;
   return q - f;
@@ -178,6 +205,13 @@ __device__ __forceinline__ int boundaryOf(const DevK &G, int x, int y) {
   return x == 0 ? 0 : x == G.nx - 1 ? 1 : y == 0 ? 2 : 3;
 }
 
+// v < 0 or v > mx (double: without double-precision instructions)
+__device__ __forceinline__ bool outside(float v, float mx) { return v < 0.f || v > mx; }
+__device__ __forceinline__ bool outside(double v, double mx) {
+  const long long b = __double_as_longlong(v);
+  return belowD(v, 0.0) || (b > __double_as_longlong(mx) && b <= 0x7ff0000000000000ll);
+}
+
 // free flight under force F, then the boundary treatment of
 // include/emcParticleDrift.hpp:41-66 (removal at ohmic contacts, a surface
 // mechanism or specular reflection elsewhere) and the region update of
@@ -189,13 +223,14 @@ __device__ __forceinline__ bool devDrift(const ModelK<T> &M, const DevK &G, int 
                                          const T F[2], T dt, T k[3], T &E, T pos[2],
                                          int &region, Src &rng) {
   const ValleyK<T> &V = M.v[valley];
+  const T FF[3] = {F[0], F[1], T(0)};
   T fE[3];
-  toEcs(V.rot[sub], F[0], F[1], T(0), fE);
+  rotate<false>(V, sub, FF, fE);
   T fv[3] = {fE[0] * V.cF[0], fE[1] * V.cF[1], fE[2] * V.cF[2]};
   T kN[3];
   drift<T, 2>(V, sub, fv, dt, k, E, pos, kN);
   const T mx[2] = {(T)G.maxX, (T)G.maxY};
-  if (pos[0] < T(0) || pos[0] > mx[0] || pos[1] < T(0) || pos[1] > mx[1]) {
+  if (outside(pos[0], mx[0]) || outside(pos[1], mx[1])) {
     T pb[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) {
@@ -237,47 +272,159 @@ __device__ __forceinline__ void recordErr(int *err, int code) {
 }
 
 // driftScatterParticles for one particle
-// (include/ParticleHandler/emcBasicParticleHandler.hpp:93-139)
+// (include/ParticleHandler/emcBasicParticleHandler.hpp:93-139), in three parts:
+// the free flight to the event or the step's end, the events inside the step, the
+// timers at its end.
+template <class T, int SCHEME, bool kSurf, class Src>
+__device__ __forceinline__ bool devFirstFlight(const ModelK<T> &M, const DevK &G, const T *Ex,
+                                               const T *Ey, T charge, T dt, T k[3], T pos[2], T &E,
+                                               T tau, int valley, int sub, int &region, Src &rng) {
+  T F[2];
+  interpForce<T, SCHEME>(G, Ex, Ey, pos[0], pos[1], charge, F);
+  return devDrift<T, kSurf>(M, G, valley, sub, F, tau >= dt ? dt : tau, k, E, pos, region, rng);
+}
+
+template <class T, int SCHEME, bool kSurf, class Src>
+__device__ __forceinline__ int devEvents(const ModelK<T> &M, const DevK &G, const T *Ex,
+                                         const T *Ey, T charge, T dt, T k[3], T pos[2], T &E,
+                                         T &tau, int &valley, int &sub, int &region, Src &rng,
+                                         bool &removed) {
+  T F[2];
+  T tRem = dt - tau;
+  int guard = 0;
+  while (tRem > T(0) && !removed) {
+    if (++guard > kMaxScatterPerStepDev)
+      return EMCG_ERR_TIMEOUT;
+    int e = scatterParticle(M, k, E, valley, sub, region, rng);
+    if (e)
+      return e;
+    T nt = -drawLog(M, rng.ulog()) * tauOf(M, valley, region);
+    tau += nt;
+    interpForce<T, SCHEME>(G, Ex, Ey, pos[0], pos[1], charge, F);
+    removed = devDrift<T, kSurf>(M, G, valley, sub, F, nt < tRem ? nt : tRem, k, E, pos, region,
+                                 rng);
+    tRem -= nt;
+  }
+  return 0;
+}
+
+template <class T, class Src>
+__device__ __forceinline__ void devStepEnd(const ModelK<T> &M, T dt, T k[3], T &tau, T &gtau,
+                                           Src &rng, bool removed) {
+  tau -= dt;
+  gtau -= dt;
+  if (gtau <= T(0) && !removed) { // emcBasicParticleHandler.hpp:131-138
+    if (M.grain)
+      grainScatter(M, k, rng);
+    gtau = -drawLog(M, rng.ulog()) * M.grainTau;
+  }
+}
+
 template <class T, int SCHEME, bool kSurf, class Src>
 __device__ __forceinline__ int devParticleStep(const ModelK<T> &M, const DevK &G, const T *Ex,
                                                const T *Ey, T charge, T dt, T k[3], T pos[2],
                                                T &E, T &tau, T &gtau, int &valley, int &sub,
                                                int &region, Src &rng, bool &removed) {
   int err = 0;
-  T F[2];
-  interpForce<T, SCHEME>(G, Ex, Ey, pos[0], pos[1], charge, F);
-  if (tau >= dt) {
-    removed = devDrift<T, kSurf>(M, G, valley, sub, F, dt, k, E, pos, region, rng);
-  } else {
-    removed = devDrift<T, kSurf>(M, G, valley, sub, F, tau, k, E, pos, region, rng);
-    T tRem = dt - tau;
-    int guard = 0;
-    while (tRem > T(0) && !removed) {
-      if (++guard > kMaxScatterPerStepDev) {
-        err = EMCG_ERR_TIMEOUT;
-        break;
-      }
-      int e = scatterParticle(M, k, E, valley, sub, region, rng);
-      if (e) {
-        err = e;
-        break;
-      }
-      T nt = -m_log(rng.ulog()) * tauOf(M, valley, region);
-      tau += nt;
-      interpForce<T, SCHEME>(G, Ex, Ey, pos[0], pos[1], charge, F);
-      removed = devDrift<T, kSurf>(M, G, valley, sub, F, nt < tRem ? nt : tRem, k, E, pos,
-                                       region, rng);
-      tRem -= nt;
+  removed = devFirstFlight<T, SCHEME, kSurf>(M, G, Ex, Ey, charge, dt, k, pos, E, tau, valley, sub,
+                                             region, rng);
+  if (!(tau >= dt))
+    err = devEvents<T, SCHEME, kSurf>(M, G, Ex, Ey, charge, dt, k, pos, E, tau, valley, sub,
+                                      region, rng, removed);
+  devStepEnd(M, dt, k, tau, gtau, rng, removed);
+  return err;
+}
+
+// the particle's state after its step, and its removal through a contact
+template <class T>
+__device__ __forceinline__ void devStore(const StateK<T> &st, const DevK &G, int64_t i,
+                                         const T k[3], const T pos[2], T E, T tau, T gtau,
+                                         int valley, int sub, int region, bool removed,
+                                         uint8_t *drop, int32_t *netto) {
+  st.kx[i] = k[0];
+  st.ky[i] = k[1];
+  st.kz[i] = k[2];
+  st.px[i] = pos[0];
+  st.py[i] = pos[1];
+  st.E[i] = E;
+  st.tau[i] = tau;
+  st.gtau[i] = gtau;
+  st.meta[i] = packMeta(valley, sub, region);
+  drop[i] = removed ? 1 : 0;
+  if (removed) {
+    int cx = clampi(roundIdx<T>(pos[0], G.hx, G.invhx), 0, G.nx - 1);
+    int cy = clampi(roundIdx<T>(pos[1], G.hy, G.invhy), 0, G.ny - 1);
+    int c = G.nodeContact[cy * G.nx + cx];
+    if (c >= 0)
+      atomicAdd(&netto[c], 1);
+  }
+}
+
+// The double engine's move.  A double instruction of a warp takes its scheduler 64
+// clocks whatever its lanes do, and in a step of 0.1 fs every thirtieth electron
+// has an event: two warps in three would run the event path for a lane or two.
+// So the events of a block are queued and one warp -- another one from block to
+// block, as warps of the same number share a scheduler -- works on 32 of them at
+// a time.  Measured with the building blocks of emcg_fp64.cuh on 5e4 electrons
+// (nearest-node scheme, under ncu): 105 us before.
+template <int SCHEME>
+__global__ void __launch_bounds__(256)
+    devMoveQueuedKernel(StateK<double> st, const ModelK<double> *__restrict__ models, DevK G,
+                        const double *__restrict__ Ex, const double *__restrict__ Ey,
+                        double charge, double dt, const int64_t *__restrict__ nPtr, uint32_t step,
+                        uint32_t key0, uint32_t key1, uint32_t stream, uint8_t *__restrict__ drop,
+                        int32_t *__restrict__ netto, int *__restrict__ err) {
+  __shared__ double q[8][256]; // k, pos, E, tau, gtau of the queued electrons
+  __shared__ uint32_t qMeta[256];
+  __shared__ uint16_t qIdx[256];
+  __shared__ int qCount;
+  if (threadIdx.x == 0)
+    qCount = 0;
+  __syncthreads();
+  const int64_t n = *nPtr, i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + threadIdx.x;
+  const ModelK<double> &M = models[0];
+  if (i < n) {
+    double k[3] = {st.kx[i], st.ky[i], st.kz[i]}, pos[2] = {st.px[i], st.py[i]};
+    double E = st.E[i], tau = st.tau[i], gtau = st.gtau[i];
+    const uint32_t mt = st.meta[i];
+    const int valley = mt & 0xff, sub = (mt >> 8) & 0xff;
+    int region = mt >> 16;
+    PhiloxSrc<double> rng;
+    rng.init((uint32_t)i, step, stream, key0, key1);
+    bool removed = devFirstFlight<double, SCHEME, false>(M, G, Ex, Ey, charge, dt, k, pos, E, tau,
+                                                         valley, sub, region, rng);
+    if (!(tau >= dt) && !removed) {
+      const int s = atomicAdd(&qCount, 1);
+      const double v[8] = {k[0], k[1], k[2], pos[0], pos[1], E, tau, gtau};
+#pragma unroll
+      for (int f = 0; f < 8; f++)
+        q[f][s] = v[f];
+      qMeta[s] = packMeta(valley, sub, region);
+      qIdx[s] = (uint16_t)threadIdx.x;
+    } else {
+      devStepEnd(M, dt, k, tau, gtau, rng, removed);
+      devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
     }
   }
-  tau -= dt;
-  gtau -= dt;
-  if (gtau <= T(0) && !removed) { // emcBasicParticleHandler.hpp:131-138
-    if (M.grain)
-      grainScatter(M, k, rng);
-    gtau = -m_log(rng.ulog()) * M.grainTau;
-  }
-  return err;
+  __syncthreads();
+  const int nq = qCount, nWarps = blockDim.x >> 5;
+  // warp (blockIdx mod nWarps) takes the first 32, the next warp the next ...
+  const int w = ((threadIdx.x >> 5) + nWarps - (int)(blockIdx.x % nWarps)) % nWarps;
+  const int s = 32 * w + (threadIdx.x & 31);
+  if (s >= nq)
+    return;
+  double k[3] = {q[0][s], q[1][s], q[2][s]}, pos[2] = {q[3][s], q[4][s]};
+  double E = q[5][s], tau = q[6][s], gtau = q[7][s];
+  const uint32_t mt = qMeta[s];
+  int valley = mt & 0xff, sub = (mt >> 8) & 0xff, region = mt >> 16;
+  const int64_t j = i0 + qIdx[s];
+  PhiloxSrc<double> rng;
+  rng.init((uint32_t)j, step, stream, key0, key1);
+  bool removed = false;
+  recordErr(err, devEvents<double, SCHEME, false>(M, G, Ex, Ey, charge, dt, k, pos, E, tau, valley,
+                                                  sub, region, rng, removed));
+  devStepEnd(M, dt, k, tau, gtau, rng, removed);
+  devStore(st, G, j, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
 }
 
 // the float instance is capped at 64 registers, 4 blocks of 256 per SM (72
@@ -315,23 +462,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
                                           sub, region, src, removed);
   }
   recordErr(err, e);
-  st.kx[i] = k[0];
-  st.ky[i] = k[1];
-  st.kz[i] = k[2];
-  st.px[i] = pos[0];
-  st.py[i] = pos[1];
-  st.E[i] = E;
-  st.tau[i] = tau;
-  st.gtau[i] = gtau;
-  st.meta[i] = packMeta(valley, sub, region);
-  drop[i] = removed ? 1 : 0;
-  if (removed) {
-    int cx = clampi(roundIdx<T>(pos[0], G.hx, G.invhx), 0, G.nx - 1);
-    int cy = clampi(roundIdx<T>(pos[1], G.hy, G.invhy), 0, G.ny - 1);
-    int c = G.nodeContact[cy * G.nx + cx];
-    if (c >= 0)
-      atomicAdd(&netto[c], 1);
-  }
+  devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
 }
 
 // ---- stable compaction ------------------------------------------------------
@@ -583,14 +714,14 @@ __device__ __forceinline__ void initParticle2D(const ModelK<T> &M, const DevK &G
   valley = (int)m_floor((T)M.nV * rng.ulog());
   const ValleyK<T> &V = M.v[valley];
   sub = (int)m_floor((T)V.deg * rng.ulog());
-  E = T(-1.5) * (T)G.Vt * m_log(rng.ulog());
+  E = T(-1.5) * (T)G.Vt * drawLog(M, rng.ulog());
   randomDirection(V.cK * m_sqrt(gammaOf(V, E)), rng, k);
 #pragma unroll
   for (int d = 0; d < 2; d++)
     if ((c[d] == 0 && k[d] < T(0)) || (c[d] == ext[d] - 1 && k[d] > T(0)))
       k[d] *= T(-1);
-  tau = -m_log(rng.ulog()) * tauOf(M, valley, tauRegionIsValley ? valley : region);
-  gtau = -m_log(rng.ulog()) * M.grainTau;
+  tau = -drawLog(M, rng.ulog()) * tauOf(M, valley, tauRegionIsValley ? valley : region);
+  gtau = -drawLog(M, rng.ulog()) * M.grainTau;
 }
 
 template <class T, bool REPLAY>
@@ -882,6 +1013,7 @@ struct DeviceImpl {
   std::vector<double> expNrH;
   // device
   void *dModel = nullptr, *dTables = nullptr;
+  double *dLogTab = nullptr; // logTab()'s table (double engine)
   RateLayout rates;            // table layout (rate-table rebuild)
   RateScratch rateScratch;     // device scratch of rebuilds
   int32_t *dRegion = nullptr, *dNodeContact = nullptr, *dNodeRes = nullptr, *dBnd[4] = {};
@@ -997,7 +1129,7 @@ int32_t destroyDevice(emcg_handle *h) {
   if (d->stream)
     cudaStreamSynchronize(d->stream);
   poissonFree(d->mg);
-  void *ps[] = {d->dModel, d->dTables, d->dRegion, d->dNodeContact, d->dNodeRes, d->dNodeOhmic,
+  void *ps[] = {d->dModel, d->dTables, d->dLogTab, d->dRegion, d->dNodeContact, d->dNodeRes, d->dNodeOhmic,
                 d->dPot, d->dNr, d->dConc, d->dExp, d->dEx, d->dEy, d->dN, d->dDrop, d->dBlock,
                 d->dList, d->dListNode, d->dListCount, d->dGList, d->dGNode, d->dKept,
                 d->dChunkCount, d->dResNodes,
@@ -1057,6 +1189,9 @@ template <class T> static int32_t createModel(DeviceImpl *d, const emcg_model_de
     d->surfaces = d->surfaces || m.surface_kind[b] != EMCG_SURFACE_SPECULAR;
   EMCG_TRY(up((T **)&d->dTables, tab.data(), tab.size(), d->stream));
   K.tables = (const T *)d->dTables;
+  if (sizeof(T) == 8)
+    EMCG_TRY(uploadLogTable(&d->dLogTab));
+  K.logT = d->dLogTab;
   EMCG_TRY(up((ModelK<T> **)&d->dModel, &K, 1, d->stream));
   const size_t n = (size_t)d->nx * d->ny;
   EMCG_CUDA(cudaMalloc(&d->dEx, n * sizeof(T)));
@@ -1342,6 +1477,16 @@ static int32_t compact(DeviceImpl *d) {
   return EMCG_OK;
 }
 
+// the move kernel of a scheme (the double engine's plain Philox moves have their
+// own, devMoveQueuedKernel)
+template <class T, int SCHEME, bool REPLAY> static auto moveKernel(bool surfaces) {
+  if constexpr (sizeof(T) == 8 && !REPLAY)
+    return devMoveKernel<T, SCHEME, REPLAY, true>;
+  else
+    return surfaces ? devMoveKernel<T, SCHEME, REPLAY, true>
+                    : devMoveKernel<T, SCHEME, REPLAY, false>;
+}
+
 // compactAfter = false: the removed particles stay marked in dDrop for the
 // contact handling's single compaction (device step)
 template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compactAfter = true) {
@@ -1357,8 +1502,12 @@ template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compa
     setError("replay needs the FP64 engine");
     return EMCG_ERR_ARG;
   }
+#define EMCG_MOVEQ(SCH)                                                                          \
+  devMoveQueuedKernel<SCH><<<nb, 256, 0, d->stream>>>(                                    \
+      st, M, G, Ex, Ey, c.charge, c.dt, d->dN, step, k0, k1, c.stream, d->dDrop, d->dNetto,      \
+      d->dErr)
 #define EMCG_MOVE(SCH, REP)                                                                      \
-  (d->surfaces ? devMoveKernel<T, SCH, REP, true> : devMoveKernel<T, SCH, REP, false>)           \
+  moveKernel<T, SCH, REP>(d->surfaces)                                                           \
       <<<nb, 256, 0, d->stream>>>(st, M, G, Ex, Ey, (T)c.charge, (T)c.dt, d->dN, step, k0, k1,    \
                                   c.stream, d->dDrop, d->dNetto, d->dWords[0], d->dOff[0],        \
                                   d->dErr)
@@ -1373,6 +1522,19 @@ template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compa
       else
         EMCG_MOVE(EMCG_PM_NEC_VWD, true);
     }
+  } else if (sizeof(T) == 8 && !d->surfaces) {
+    // (a surface mechanism draws inside the first flight, so that its electrons'
+    // random numbers would have to travel with them)
+    if constexpr (sizeof(T) == 8) {
+      if (c.pm_scheme == EMCG_PM_NGP)
+        EMCG_MOVEQ(EMCG_PM_NGP);
+      else if (c.pm_scheme == EMCG_PM_CIC)
+        EMCG_MOVEQ(EMCG_PM_CIC);
+      else if (c.pm_scheme == EMCG_PM_NEC)
+        EMCG_MOVEQ(EMCG_PM_NEC);
+      else
+        EMCG_MOVEQ(EMCG_PM_NEC_VWD);
+    }
   } else if (c.pm_scheme == EMCG_PM_NGP) {
     EMCG_MOVE(EMCG_PM_NGP, false);
   } else if (c.pm_scheme == EMCG_PM_CIC) {
@@ -1383,6 +1545,7 @@ template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compa
     EMCG_MOVE(EMCG_PM_NEC_VWD, false);
   }
 #undef EMCG_MOVE
+#undef EMCG_MOVEQ
   EMCG_CUDA(cudaGetLastError());
   d->replay[0] = false;
   return compactAfter ? compact(d) : EMCG_OK;

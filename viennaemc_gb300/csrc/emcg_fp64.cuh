@@ -1,0 +1,74 @@
+// Double-precision building blocks for a GPU whose schedulers issue one double
+// instruction of a warp in 64 clocks: square root, reciprocal and quotient from
+// the hardware's approximations with one correction each, and comparisons and
+// frame rotations without double instructions.  All give the correctly rounded
+// result or its neighbour; arguments outside their range go to the library.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace emcg {
+
+// 1 / sqrt(t) for normal t > 0: the hardware's approximation (about 20 bits)
+// and one step of Householder's method of third order (Householder 1970):
+// with e = 1 - t y^2, y (1 + e / 2 + 3 e^2 / 8)
+__device__ __forceinline__ double rsqrtD(double t) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
+  const double e = fma(-t * y, y, 1.0);
+  return fma(fma(0.375, e, 0.5), y * e, y);
+}
+
+// 1 / d for normal d whose reciprocal is normal: the hardware's approximation
+// (about 20 bits) and y (1 + r + r^2), r = 1 - d y (the geometric series to
+// third order)
+__device__ __forceinline__ double rcpD(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double r = fma(-d, y, 1.0);
+  return fma(y, fma(r, r, r), y);
+}
+
+// sqrt(x): x / sqrt(x) corrected once; 0, subnormals, infinities, negative
+// values and NaN go to the library's
+__device__ __forceinline__ double sqrtD(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  if (h - 0x00100000u >= 0x7fe00000u)
+    return sqrt(x);
+  const double y = rsqrtD(x), s = x * y;
+  return fma(fma(-s, s, x), 0.5 * y, s);
+}
+
+// a / b: a times 1 / b corrected once; where an exponent is near the range's
+// ends the library's division
+__device__ __forceinline__ double divD(double a, double b) {
+  const uint32_t ha = (uint32_t)__double2hiint(a) & 0x7fffffffu,
+                 hb = (uint32_t)__double2hiint(b) & 0x7fffffffu;
+  // both in [2^-500, 2^500]
+  if (ha - 0x20b00000u >= 0x3e800000u || hb - 0x20b00000u >= 0x3e800000u)
+    return a / b;
+  const double inv = rcpD(b), q = a * inv;
+  return fma(fma(-b, q, a), inv, q);
+}
+
+// a < b for a double a and b >= 0 without a double-precision instruction: the
+// bit patterns of non-negative doubles order like the values, those of
+// negative ones are negative integers; a NaN is not below
+__device__ __forceinline__ bool belowD(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  return x < y && (unsigned long long)x <= 0xfff0000000000000ull;
+}
+
+// q as an integer part and 20 fractional bits, for 0 <= q < 2^30; false outside
+__device__ __forceinline__ bool fixedOf(double q, uint64_t &f) {
+  const uint64_t b = (uint64_t)__double_as_longlong(q);
+  const int e = (int)(b >> 52) - 1023;
+  if (e >= 30) // also a negative q, infinities and NaN
+    return false;
+  const uint64_t mant = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+  f = e < -31 ? 0 : mant >> (32 - e);
+  return true;
+}
+
+} // namespace emcg

@@ -111,6 +111,19 @@ inline int32_t validateModel(const emcg_model_desc &m) {
   return EMCG_OK;
 }
 
+// logTab()'s table on the device (ModelK::logT)
+inline int32_t uploadLogTable(double **dst) {
+  static const std::vector<double> tab = [] { // a constant, formed once
+    std::vector<double> t(kLogTab);
+    for (int i = 0; i < kLogTab; i++)
+      t[i] = logTabEntry(i);
+    return t;
+  }();
+  EMCG_CUDA(cudaMalloc(dst, kLogTab * sizeof(double)));
+  EMCG_CUDA(cudaMemcpy(*dst, tab.data(), kLogTab * sizeof(double), cudaMemcpyHostToDevice));
+  return EMCG_OK;
+}
+
 // ValleyK::perm of a subvalley frame
 inline uint32_t permOf(const double R[9]) {
   uint32_t p = 0, cols = 0;
