@@ -340,7 +340,7 @@ template <class T>
 __device__ __forceinline__ void devStore(const StateK<T> &st, const DevK &G, int64_t i,
                                          const T k[3], const T pos[2], T E, T tau, T gtau,
                                          int valley, int sub, int region, bool removed,
-                                         uint8_t *drop, int32_t *netto) {
+                                         uint8_t *drop, int32_t *dropCount, int32_t *netto) {
   st.kx[i] = k[0];
   st.ky[i] = k[1];
   st.kz[i] = k[2];
@@ -352,6 +352,7 @@ __device__ __forceinline__ void devStore(const StateK<T> &st, const DevK &G, int
   st.meta[i] = packMeta(valley, sub, region);
   drop[i] = removed ? 1 : 0;
   if (removed) {
+    atomicAdd(&dropCount[i / kCB], 1);
     int cx = clampi(roundIdx<T>(pos[0], G.hx, G.invhx), 0, G.nx - 1);
     int cy = clampi(roundIdx<T>(pos[1], G.hy, G.invhy), 0, G.ny - 1);
     int c = G.nodeContact[cy * G.nx + cx];
@@ -373,7 +374,8 @@ __global__ void __launch_bounds__(256)
                         const double *__restrict__ Ex, const double *__restrict__ Ey,
                         double charge, double dt, const int64_t *__restrict__ nPtr, uint32_t step,
                         uint32_t key0, uint32_t key1, uint32_t stream, uint8_t *__restrict__ drop,
-                        int32_t *__restrict__ netto, int *__restrict__ err) {
+                        int32_t *__restrict__ dropCount, int32_t *__restrict__ netto,
+                        int *__restrict__ err) {
   __shared__ double q[8][256]; // k, pos, E, tau, gtau of the queued electrons
   __shared__ uint32_t qMeta[256];
   __shared__ uint16_t qIdx[256];
@@ -403,7 +405,8 @@ __global__ void __launch_bounds__(256)
       qIdx[s] = (uint16_t)threadIdx.x;
     } else {
       devStepEnd(M, dt, k, tau, gtau, rng, removed);
-      devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
+      devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, dropCount,
+           netto);
     }
   }
   __syncthreads();
@@ -424,7 +427,8 @@ __global__ void __launch_bounds__(256)
   recordErr(err, devEvents<double, SCHEME, false>(M, G, Ex, Ey, charge, dt, k, pos, E, tau, valley,
                                                   sub, region, rng, removed));
   devStepEnd(M, dt, k, tau, gtau, rng, removed);
-  devStore(st, G, j, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
+  devStore(st, G, j, k, pos, E, tau, gtau, valley, sub, region, removed, drop, dropCount,
+           netto);
 }
 
 // the float instance is capped at 64 registers, 4 blocks of 256 per SM (72
@@ -434,9 +438,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
     devMoveKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
                   const T *__restrict__ Ex, const T *__restrict__ Ey, T charge, T dt,
                   const int64_t *__restrict__ nPtr, uint32_t step, uint32_t key0, uint32_t key1,
-                  uint32_t stream, uint8_t *__restrict__ drop, int32_t *__restrict__ netto,
-                  const uint64_t *__restrict__ rw, const int64_t *__restrict__ roff,
-                  int *__restrict__ err) {
+                  uint32_t stream, uint8_t *__restrict__ drop, int32_t *__restrict__ dropCount,
+                  int32_t *__restrict__ netto, const uint64_t *__restrict__ rw,
+                  const int64_t *__restrict__ roff, int *__restrict__ err) {
   const int64_t n = *nPtr;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
@@ -462,10 +466,20 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
                                           sub, region, src, removed);
   }
   recordErr(err, e);
-  devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, netto);
+  devStore(st, G, i, k, pos, E, tau, gtau, valley, sub, region, removed, drop, dropCount,
+           netto);
 }
 
 // ---- stable compaction ------------------------------------------------------
+// Beside its move and its Poisson solve a device step is a chain of small
+// kernels, each a few us of launch latency and dependent reads: their number is
+// what bounds them.  So the kernels that drop a particle count it for its block
+// themselves, a block adds up the counts before it instead of a scan between two
+// launches, the compaction and the injection assign the charge of the particles
+// that they place, the first kernel clears the step's counters, and the last one
+// writes the outcome into page-locked memory.  10 nodes a step on the stream
+// instead of 24; resistor 201 x 101, 500k electrons FP32: 0.502 -> 0.444 ms a step,
+// 101 x 51, 50k electrons FP64 0.394 -> 0.329, 8 MOSFETs of 401 x 201 at once 7.6 -> 6.8 ms per 5.
 __device__ __forceinline__ int blockExclusiveScan(int v, int *total) {
   __shared__ int warpSums[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -496,16 +510,26 @@ __device__ __forceinline__ int blockExclusiveScan(int v, int *total) {
   return off;
 }
 
-__global__ void compactCountKernel(const uint8_t *__restrict__ drop, const int64_t *__restrict__ nPtr,
-                                   int32_t *__restrict__ blockCount) {
-  const int64_t n = *nPtr;
-  const int64_t i = (int64_t)blockIdx.x * kCB + threadIdx.x;
-  int keep = (i < n && !drop[i]) ? 1 : 0;
-  int tot;
-  blockExclusiveScan(keep, &tot);
-  if (threadIdx.x == 0)
-    blockCount[blockIdx.x] = tot;
+// Sum of counts[0 .. m) in every thread of the block.
+__device__ __forceinline__ int blockSum(const int32_t *__restrict__ counts, int m) {
+  __shared__ int part[32];
+  int v = 0;
+  for (int t = threadIdx.x; t < m; t += blockDim.x)
+    v += counts[t];
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0)
+    part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? part[threadIdx.x & 31] : 0;
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  return v;
 }
+
+// up to this many blocks of kCB particles (4 million) each block of a compaction
+// adds up the counts of those before it, which costs a read of the counts and
+// no launch; beyond, one block scans them first (scanBlocksKernel)
+constexpr int kPrefixBlocks = 4096;
 
 // exclusive scan of nb block counts (one block); total -> *nOut
 __global__ void scanBlocksKernel(int32_t *__restrict__ counts, int nb, int64_t *__restrict__ nOut) {
@@ -521,296 +545,6 @@ __global__ void scanBlocksKernel(int32_t *__restrict__ counts, int nb, int64_t *
   }
   if (threadIdx.x == 0)
     *nOut = carry;
-}
-
-template <class T>
-__global__ void compactScatterKernel(StateK<T> src, StateK<T> dst, const uint8_t *__restrict__ drop,
-                                     const int64_t *__restrict__ nPtr,
-                                     const int32_t *__restrict__ blockOff) {
-  const int64_t n = *nPtr;
-  const int64_t i = (int64_t)blockIdx.x * kCB + threadIdx.x;
-  int keep = (i < n && !drop[i]) ? 1 : 0;
-  int tot;
-  int r = blockExclusiveScan(keep, &tot);
-  if (!keep)
-    return;
-  int64_t j = blockOff[blockIdx.x] + r;
-  dst.kx[j] = src.kx[i];
-  dst.ky[j] = src.ky[i];
-  dst.kz[j] = src.kz[i];
-  dst.px[j] = src.px[i];
-  dst.py[j] = src.py[i];
-  dst.pz[j] = src.pz[i];
-  dst.E[j] = src.E[i];
-  dst.tau[j] = src.tau[i];
-  dst.gtau[j] = src.gtau[i];
-  dst.meta[j] = src.meta[i];
-}
-
-// ---- contacts (include/ParticleHandler/emcBasicParticleHandler.hpp:158-192) --
-// list of the particles sitting at reservoir nodes, in index order
-template <class T>
-__global__ void reservoirListKernel(StateK<T> st, DevK G, const int64_t *__restrict__ nPtr,
-                                    const uint8_t *__restrict__ skip,
-                                    int32_t *__restrict__ list, int32_t *__restrict__ listNode,
-                                    int32_t *__restrict__ listCount) {
-  const int64_t n = *nPtr;
-  const int64_t i = (int64_t)blockIdx.x * kCB + threadIdx.x;
-  int node = -1;
-  if (i < n && !(skip && skip[i])) { // skip: removed by the move, not yet compacted
-    int cx = clampi(roundIdx<T>(st.px[i], G.hx, G.invhx), 0, G.nx - 1);
-    int cy = clampi(roundIdx<T>(st.py[i], G.hy, G.invhy), 0, G.ny - 1);
-    int g = cy * G.nx + cx;
-    if (G.nodeRes[g] >= 0)
-      node = g;
-  }
-  int tot;
-  int r = blockExclusiveScan(node >= 0 ? 1 : 0, &tot);
-  if (node >= 0) {
-    list[(int64_t)blockIdx.x * kCB + r] = (int32_t)i;
-    listNode[(int64_t)blockIdx.x * kCB + r] = node;
-  }
-  if (threadIdx.x == 0)
-    listCount[blockIdx.x] = tot;
-}
-
-// the per-block reservoir lists, concatenated in block order: all reservoir
-// particles in index order (off = exclusive scan of the block counts)
-__global__ void gatherListKernel(const int32_t *__restrict__ list,
-                                 const int32_t *__restrict__ listNode,
-                                 const int32_t *__restrict__ off, int nb,
-                                 const int64_t *__restrict__ total, int32_t *__restrict__ gList,
-                                 int32_t *__restrict__ gNode) {
-  const int b = blockIdx.x;
-  const int o = off[b];
-  const int cnt = (b + 1 < nb ? off[b + 1] : (int)*total) - o;
-  for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-    gList[o + j] = list[(int64_t)b * kCB + j];
-    gNode[o + j] = listNode[(int64_t)b * kCB + j];
-  }
-}
-
-// Ranking of the particles on reservoir nodes (emcBasicParticleHandler::
-// handleOhmicContacts, :158-192): the r-th particle at a node (r from 0, in
-// particle order) stays while r * carriers is below the expected number there,
-// the rest are marked for removal.  The gathered list (particle order) is cut
-// into kRankChunks chunks; a warp per (node, chunk) counts the node's entries
-// in its chunk (contactCountKernel), then ranks them from the counts of the
-// earlier chunks (contactRankKernel), so no warp walks the whole list.
-constexpr int kRankChunks = 16;
-
-__device__ __forceinline__ void rankChunk(int R, int c, int &j0, int &j1) {
-  const int len = (R + kRankChunks - 1) / kRankChunks;
-  j0 = min(R, c * len);
-  j1 = min(R, j0 + len);
-}
-
-__global__ void contactCountKernel(const int32_t *__restrict__ gNode,
-                                   const int64_t *__restrict__ total,
-                                   const int32_t *__restrict__ resNodes, int nRes,
-                                   int32_t *__restrict__ chunkCount) {
-  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= nRes * kRankChunks)
-    return;
-  const int r = w / kRankChunks, c = w - r * kRankChunks;
-  const int g = resNodes[r];
-  int j0, j1;
-  rankChunk((int)*total, c, j0, j1);
-  int cnt = 0;
-  for (int base = j0; base < j1; base += 32) {
-    const int j = base + lane;
-    cnt += __popc(__ballot_sync(0xffffffffu, j < j1 && gNode[j] == g));
-  }
-  if (lane == 0)
-    chunkCount[w] = cnt;
-}
-
-__global__ void contactRankKernel(const int32_t *__restrict__ gList,
-                                  const int32_t *__restrict__ gNode,
-                                  const int64_t *__restrict__ total,
-                                  const int32_t *__restrict__ resNodes, int nRes,
-                                  const double *__restrict__ expNr, double nrC,
-                                  const int32_t *__restrict__ nodeContact,
-                                  const int32_t *__restrict__ chunkCount,
-                                  uint8_t *__restrict__ drop, int32_t *__restrict__ kept,
-                                  int32_t *__restrict__ remInj) {
-  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= nRes * kRankChunks)
-    return;
-  const int r = w / kRankChunks, c = w - r * kRankChunks;
-  const int g = resNodes[r];
-  const double e = expNr[g];
-  int j0, j1;
-  rankChunk((int)*total, c, j0, j1);
-  int seen = 0; // the node's entries in the earlier chunks
-  for (int q = 0; q < c; q++)
-    seen += chunkCount[r * kRankChunks + q];
-  int nKept = 0, nDrop = 0;
-  for (int base = j0; base < j1; base += 32) {
-    const int j = base + lane;
-    const bool mine = j < j1 && gNode[j] == g;
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (mine) {
-      const int rk = seen + __popc(m & ((1u << lane) - 1u));
-      if ((double)rk * nrC < e)
-        nKept++;
-      else {
-        drop[gList[j]] = 1;
-        nDrop++;
-      }
-    }
-    seen += __popc(m);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    nKept += __shfl_xor_sync(0xffffffffu, nKept, o);
-    nDrop += __shfl_xor_sync(0xffffffffu, nDrop, o);
-  }
-  if (lane == 0) {
-    if (nKept)
-      atomicAdd(&kept[g], nKept);
-    if (nDrop)
-      atomicAdd(&remInj[nodeContact[g]], -nDrop);
-  }
-}
-
-// particles to inject per reservoir node (emcAbstractParticleHandler.hpp:200-216)
-__global__ void injectCountKernel(const int32_t *__restrict__ resNodes, int nRes,
-                                  const double *__restrict__ expNr, const int32_t *__restrict__ kept,
-                                  double nrC, int32_t *__restrict__ injCount) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nRes)
-    return;
-  int g = resNodes[r];
-  double diff = expNr[g] - (double)kept[g] * nrC;
-  int c = 0;
-  while (diff > 0 && c < (1 << 20)) {
-    c++;
-    diff -= nrC;
-  }
-  injCount[r] = c;
-}
-
-// emcElectron::generateInjectedParticle + initParticlePos (2-D)
-template <class T, class Src>
-__device__ __forceinline__ void initParticle2D(const ModelK<T> &M, const DevK &G, int cx, int cy,
-                                               int region, bool tauRegionIsValley, Src &rng,
-                                               T k[3], T pos[2], T &E, T &tau, T &gtau,
-                                               int &valley, int &sub) {
-  const int c[2] = {cx, cy};
-  const int ext[2] = {G.nx, G.ny};
-  const double h[2] = {G.hx, G.hy};
-#pragma unroll
-  for (int d = 0; d < 2; d++) {
-    if (c[d] == ext[d] - 1)
-      pos[d] = ((T)c[d] - rng.u01() * T(0.5)) * (T)h[d];
-    else if (c[d] == 0)
-      pos[d] = rng.u01() * T(0.5) * (T)h[d];
-    else
-      pos[d] = ((T)c[d] + rng.u01() - T(0.5)) * (T)h[d];
-  }
-  valley = (int)m_floor((T)M.nV * rng.ulog());
-  const ValleyK<T> &V = M.v[valley];
-  sub = (int)m_floor((T)V.deg * rng.ulog());
-  E = T(-1.5) * (T)G.Vt * drawLog(M, rng.ulog());
-  randomDirection(V.cK * m_sqrt(gammaOf(V, E)), rng, k);
-#pragma unroll
-  for (int d = 0; d < 2; d++)
-    if ((c[d] == 0 && k[d] < T(0)) || (c[d] == ext[d] - 1 && k[d] > T(0)))
-      k[d] *= T(-1);
-  tau = -drawLog(M, rng.ulog()) * tauOf(M, valley, tauRegionIsValley ? valley : region);
-  gtau = -drawLog(M, rng.ulog()) * M.grainTau;
-}
-
-template <class T, bool REPLAY>
-__global__ void injectKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
-                             const int32_t *__restrict__ resNodes, int nRes,
-                             const int32_t *__restrict__ injBase, const int64_t *__restrict__ injTotal,
-                             int64_t *__restrict__ nPtr, int64_t capacity, uint32_t step,
-                             uint32_t key0, uint32_t key1, uint32_t stream, bool tauRegionIsValley,
-                             int32_t *__restrict__ remInj, const uint64_t *__restrict__ rw,
-                             const int64_t *__restrict__ roff, int *__restrict__ err) {
-  const int64_t total = *injTotal;
-  const int64_t n = *nPtr;
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= total)
-    return;
-  if (n + total > capacity) {
-    if (j == 0)
-      recordErr(err, EMCG_ERR_CAPACITY);
-    return;
-  }
-  int lo = 0, hi = nRes - 1; // last r with injBase[r] <= j
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (injBase[mid] <= j)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  const int g = resNodes[lo];
-  const int cx = g % G.nx, cy = g / G.nx;
-  const int region = G.region[g];
-  T k[3], pos[2], E, tau, gtau;
-  int valley, sub;
-  const ModelK<T> &M = models[0];
-  if constexpr (REPLAY) {
-    ReplaySrc src{rw, roff[j], roff[j + 1], 0};
-    initParticle2D(M, G, cx, cy, region, tauRegionIsValley, src, k, pos, E, tau, gtau, valley, sub);
-    if (src.bad || src.pos != src.end)
-      recordErr(err, EMCG_ERR_REPLAY);
-  } else {
-    PhiloxSrc<T> src;
-    src.init((uint32_t)j, step, stream | 0x80000000u, key0, key1);
-    initParticle2D(M, G, cx, cy, region, tauRegionIsValley, src, k, pos, E, tau, gtau, valley, sub);
-  }
-  const int64_t d = n + j;
-  st.kx[d] = k[0];
-  st.ky[d] = k[1];
-  st.kz[d] = k[2];
-  st.px[d] = pos[0];
-  st.py[d] = pos[1];
-  st.pz[d] = T(0);
-  st.E[d] = E;
-  st.tau[d] = tau;
-  st.gtau[d] = gtau;
-  st.meta[d] = packMeta(valley, sub, region);
-  atomicAdd(&remInj[G.nodeContact[g]], 1);
-}
-
-__global__ void addCountKernel(int64_t *nPtr, const int64_t *add, int64_t capacity) {
-  if (*nPtr + *add <= capacity)
-    *nPtr += *add;
-}
-
-// initial particles at given nodes (counts decided on the host)
-template <class T>
-__global__ void devInitKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
-                              const int32_t *__restrict__ nodeOf, int64_t n, uint32_t key0,
-                              uint32_t key1, uint32_t stream, bool tauRegionIsValley) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  const int g = nodeOf[i];
-  const int region = G.region[g];
-  T k[3], pos[2], E, tau, gtau;
-  int valley, sub;
-  PhiloxSrc<T> src;
-  src.init((uint32_t)i, 0xFFFFFFFFu, stream, key0, key1);
-  initParticle2D(models[0], G, g % G.nx, g / G.nx, region, tauRegionIsValley, src, k, pos, E,
-                 tau, gtau, valley, sub);
-  st.kx[i] = k[0];
-  st.ky[i] = k[1];
-  st.kz[i] = k[2];
-  st.px[i] = pos[0];
-  st.py[i] = pos[1];
-  st.pz[i] = T(0);
-  st.E[i] = E;
-  st.tau[i] = tau;
-  st.gtau[i] = gtau;
-  st.meta[i] = packMeta(valley, sub, region);
 }
 
 // ---- particle -> mesh ------------------------------------------------------
@@ -867,33 +601,29 @@ __device__ __forceinline__ void fixAdd(const DevK &G, unsigned long long *fix, i
   if (hi)
     atomicAdd(p + 1, hi);
 }
-
+// one particle at (px, py) to the nodes around it
 template <class T, int SCHEME>
-__global__ void assignKernel(StateK<T> st, DevK G, const int64_t *__restrict__ nPtr, double nrC,
-                             int fixBits, unsigned long long *__restrict__ fix) {
-  const int64_t n = *nPtr;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
+__device__ __forceinline__ void assignParticle(const DevK &G, T px, T py, double nrC, int fixBits,
+                                               unsigned long long *__restrict__ fix) {
   int mx, my;
   if constexpr (sizeof(T) == 4) {
     const float s = ldexpf((float)nrC, fixBits);
     unsigned long long v[4];
     if (SCHEME == EMCG_PM_NGP) {
-      mx = roundIdx<float>(st.px[i], G.hx, G.invhx);
-      my = roundIdx<float>(st.py[i], G.hy, G.invhy);
+      mx = roundIdx<float>(px, G.hx, G.invhx);
+      my = roundIdx<float>(py, G.hy, G.invhy);
       fixAdd(G, fix, mx, my, __float2ull_rn(s), 0ull);
       return;
     } else if (SCHEME == EMCG_PM_CIC) {
-      const float wX = floorDiv<float>(st.px[i], G.hx, G.invhx, mx);
-      const float wY = floorDiv<float>(st.py[i], G.hy, G.invhy, my);
+      const float wX = floorDiv<float>(px, G.hx, G.invhx, mx);
+      const float wY = floorDiv<float>(py, G.hy, G.invhy, my);
       v[0] = __float2ull_rn(wX * wY * s);
       v[1] = __float2ull_rn((1.f - wX) * wY * s);
       v[2] = __float2ull_rn(wX * (1.f - wY) * s);
       v[3] = __float2ull_rn((1.f - wX) * (1.f - wY) * s);
     } else {
-      floorDiv<float>(st.px[i], G.hx, G.invhx, mx);
-      floorDiv<float>(st.py[i], G.hy, G.invhy, my);
+      floorDiv<float>(px, G.hx, G.invhx, mx);
+      floorDiv<float>(py, G.hy, G.invhy, my);
       v[0] = v[1] = v[2] = v[3] = __float2ull_rn(0.25f * s);
     }
     fixAdd(G, fix, mx, my, v[0], 0ull);
@@ -903,22 +633,22 @@ __global__ void assignKernel(StateK<T> st, DevK G, const int64_t *__restrict__ n
   } else {
     double w[4];
     if (SCHEME == EMCG_PM_NGP) {
-      mx = roundIdx<T>(st.px[i], G.hx, G.invhx);
-      my = roundIdx<T>(st.py[i], G.hy, G.invhy);
+      mx = roundIdx<T>(px, G.hx, G.invhx);
+      my = roundIdx<T>(py, G.hy, G.invhy);
       unsigned long long lo, hi;
       toFix128(nrC, fixBits, lo, hi);
       fixAdd(G, fix, mx, my, lo, hi);
       return;
     } else if (SCHEME == EMCG_PM_CIC) {
-      const double wX = (double)floorDiv<T>(st.px[i], G.hx, G.invhx, mx);
-      const double wY = (double)floorDiv<T>(st.py[i], G.hy, G.invhy, my);
+      const double wX = (double)floorDiv<T>(px, G.hx, G.invhx, mx);
+      const double wY = (double)floorDiv<T>(py, G.hy, G.invhy, my);
       w[0] = wX * wY * nrC;
       w[1] = (1 - wX) * wY * nrC;
       w[2] = wX * (1 - wY) * nrC;
       w[3] = (1 - wX) * (1 - wY) * nrC;
     } else {
-      floorDiv<T>(st.px[i], G.hx, G.invhx, mx);
-      floorDiv<T>(st.py[i], G.hy, G.invhy, my);
+      floorDiv<T>(px, G.hx, G.invhx, mx);
+      floorDiv<T>(py, G.hy, G.invhy, my);
       w[0] = w[1] = w[2] = w[3] = 0.25 * nrC;
     }
     const int cx[4] = {mx, mx + 1, mx, mx + 1}, cy[4] = {my, my, my + 1, my + 1};
@@ -931,11 +661,367 @@ __global__ void assignKernel(StateK<T> st, DevK G, const int64_t *__restrict__ n
   }
 }
 
+template <class T, int SCHEME>
+__global__ void assignKernel(StateK<T> st, DevK G, const int64_t *__restrict__ nPtr, double nrC,
+                             int fixBits, unsigned long long *__restrict__ fix) {
+  const int64_t n = *nPtr;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n)
+    assignParticle<T, SCHEME>(G, st.px[i], st.py[i], nrC, fixBits, fix);
+}
+
+// The particles that stay, in their order, to dst; *nOut their number.  dropCount:
+// the dropped ones of each block of kCB (scanned: the sum of those before it, and
+// *nOut that of all).  SCHEME >= 0: their charge is assigned too.
+template <class T, int SCHEME>
+__global__ void __launch_bounds__(kCB)
+    compactScatterKernel(StateK<T> src, StateK<T> dst, DevK G, const uint8_t *__restrict__ drop,
+                         const int64_t *__restrict__ nPtr, const int32_t *__restrict__ dropCount,
+                         int64_t *__restrict__ nOut, bool scanned, double nrC, int fixBits,
+                         unsigned long long *__restrict__ fix) {
+  const int64_t n = *nPtr;
+  const int b = blockIdx.x;
+  if (b == 0) { // (the only block that reads or writes *nOut)
+    const int64_t all = scanned ? *nOut : blockSum(dropCount, gridDim.x);
+    if (threadIdx.x == 0)
+      *nOut = n - all;
+  }
+  if ((int64_t)b * kCB >= n)
+    return;
+  const int before = scanned ? dropCount[b] : blockSum(dropCount, b);
+  const int64_t i = (int64_t)b * kCB + threadIdx.x;
+  int keep = (i < n && !drop[i]) ? 1 : 0;
+  int tot;
+  int r = blockExclusiveScan(keep, &tot);
+  if (!keep)
+    return;
+  const int64_t j = (int64_t)b * kCB - before + r;
+  const T px = src.px[i], py = src.py[i];
+  dst.kx[j] = src.kx[i];
+  dst.ky[j] = src.ky[i];
+  dst.kz[j] = src.kz[i];
+  dst.px[j] = px;
+  dst.py[j] = py;
+  dst.pz[j] = src.pz[i];
+  dst.E[j] = src.E[i];
+  dst.tau[j] = src.tau[i];
+  dst.gtau[j] = src.gtau[i];
+  dst.meta[j] = src.meta[i];
+  if constexpr (SCHEME >= 0)
+    assignParticle<T, SCHEME>(G, px, py, nrC, fixBits, fix);
+}
+
+// ---- contacts (include/ParticleHandler/emcBasicParticleHandler.hpp:158-192) --
+// list of the particles sitting at reservoir nodes, in index order
+template <class T>
+__global__ void reservoirListKernel(StateK<T> st, DevK G, const int64_t *__restrict__ nPtr,
+                                    const uint8_t *__restrict__ skip,
+                                    int32_t *__restrict__ list, int32_t *__restrict__ listNode,
+                                    int32_t *__restrict__ listCount) {
+  const int64_t n = *nPtr;
+  const int64_t i = (int64_t)blockIdx.x * kCB + threadIdx.x;
+  int node = -1;
+  if (i < n && !(skip && skip[i])) { // skip: removed by the move, not yet compacted
+    int cx = clampi(roundIdx<T>(st.px[i], G.hx, G.invhx), 0, G.nx - 1);
+    int cy = clampi(roundIdx<T>(st.py[i], G.hy, G.invhy), 0, G.ny - 1);
+    int g = cy * G.nx + cx;
+    if (G.nodeRes[g] >= 0)
+      node = g;
+  }
+  int tot;
+  int r = blockExclusiveScan(node >= 0 ? 1 : 0, &tot);
+  if (node >= 0) {
+    list[(int64_t)blockIdx.x * kCB + r] = (int32_t)i;
+    listNode[(int64_t)blockIdx.x * kCB + r] = node;
+  }
+  if (threadIdx.x == 0)
+    listCount[blockIdx.x] = tot;
+}
+
+// the per-block reservoir lists, concatenated in block order: all reservoir
+// particles in index order, *total of them (counts: per block; scanned: the sum of
+// those before it, and *total that of all)
+__global__ void gatherListKernel(const int32_t *__restrict__ list,
+                                 const int32_t *__restrict__ listNode,
+                                 const int32_t *__restrict__ counts, int nb, bool scanned,
+                                 int64_t *__restrict__ total, int32_t *__restrict__ gList,
+                                 int32_t *__restrict__ gNode) {
+  const int b = blockIdx.x;
+  if (!scanned && b == nb - 1) {
+    const int all = blockSum(counts, nb);
+    if (threadIdx.x == 0)
+      *total = all;
+  }
+  int o, cnt;
+  if (scanned) {
+    o = counts[b];
+    cnt = (b + 1 < nb ? counts[b + 1] : (int)*total) - o;
+  } else {
+    cnt = counts[b];
+    if (cnt == 0)
+      return;
+    o = blockSum(counts, b);
+  }
+  for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
+    gList[o + j] = list[(int64_t)b * kCB + j];
+    gNode[o + j] = listNode[(int64_t)b * kCB + j];
+  }
+}
+
+// Ranking of the particles on reservoir nodes (emcBasicParticleHandler::
+// handleOhmicContacts, :158-192): the r-th particle at a node (r from 0, in
+// particle order) stays while r * carriers is below the expected number there,
+// the rest are marked for removal.  The gathered list (particle order) is cut
+// into kRankChunks chunks; a warp per (node, chunk) counts the node's entries
+// in its chunk (contactCountKernel), then ranks them from the counts of the
+// earlier chunks (contactRankKernel), so no warp walks the whole list.
+constexpr int kRankChunks = 16;
+
+__device__ __forceinline__ void rankChunk(int R, int c, int &j0, int &j1) {
+  const int len = (R + kRankChunks - 1) / kRankChunks;
+  j0 = min(R, c * len);
+  j1 = min(R, j0 + len);
+}
+
+__global__ void contactCountKernel(const int32_t *__restrict__ gNode,
+                                   const int64_t *__restrict__ total,
+                                   const int32_t *__restrict__ resNodes, int nRes,
+                                   int32_t *__restrict__ chunkCount) {
+  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (w >= nRes * kRankChunks)
+    return;
+  const int r = w / kRankChunks, c = w - r * kRankChunks;
+  const int g = resNodes[r];
+  int j0, j1;
+  rankChunk((int)*total, c, j0, j1);
+  int cnt = 0;
+  for (int base = j0; base < j1; base += 32) {
+    const int j = base + lane;
+    cnt += __popc(__ballot_sync(0xffffffffu, j < j1 && gNode[j] == g));
+  }
+  if (lane == 0)
+    chunkCount[w] = cnt;
+}
+
+__global__ void contactRankKernel(const int32_t *__restrict__ gList,
+                                  const int32_t *__restrict__ gNode,
+                                  const int64_t *__restrict__ total,
+                                  const int32_t *__restrict__ resNodes, int nRes,
+                                  const double *__restrict__ expNr, double nrC,
+                                  const int32_t *__restrict__ nodeContact,
+                                  const int32_t *__restrict__ chunkCount,
+                                  uint8_t *__restrict__ drop, int32_t *__restrict__ dropCount,
+                                  int32_t *__restrict__ kept, int32_t *__restrict__ remInj) {
+  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (w >= nRes * kRankChunks)
+    return;
+  const int r = w / kRankChunks, c = w - r * kRankChunks;
+  const int g = resNodes[r];
+  const double e = expNr[g];
+  int j0, j1;
+  rankChunk((int)*total, c, j0, j1);
+  int seen = 0; // the node's entries in the earlier chunks
+  for (int q = 0; q < c; q++)
+    seen += chunkCount[r * kRankChunks + q];
+  int nKept = 0, nDrop = 0;
+  for (int base = j0; base < j1; base += 32) {
+    const int j = base + lane;
+    const bool mine = j < j1 && gNode[j] == g;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (mine) {
+      const int rk = seen + __popc(m & ((1u << lane) - 1u));
+      if ((double)rk * nrC < e)
+        nKept++;
+      else {
+        drop[gList[j]] = 1;
+        atomicAdd(&dropCount[gList[j] / kCB], 1);
+        nDrop++;
+      }
+    }
+    seen += __popc(m);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nKept += __shfl_xor_sync(0xffffffffu, nKept, o);
+    nDrop += __shfl_xor_sync(0xffffffffu, nDrop, o);
+  }
+  if (lane == 0) {
+    if (nKept)
+      atomicAdd(&kept[g], nKept);
+    if (nDrop)
+      atomicAdd(&remInj[nodeContact[g]], -nDrop);
+  }
+}
+
+// particles to inject per reservoir node (emcAbstractParticleHandler.hpp:200-216),
+// as the sum of those at the nodes before it; *total: all (one block)
+__global__ void __launch_bounds__(1024)
+    injectCountKernel(const int32_t *__restrict__ resNodes, int nRes,
+                      const double *__restrict__ expNr, const int32_t *__restrict__ kept,
+                      double nrC, int32_t *__restrict__ injBase, int64_t *__restrict__ total) {
+  int64_t carry = 0;
+  for (int base = 0; base < nRes; base += blockDim.x) {
+    const int r = base + threadIdx.x;
+    int c = 0;
+    if (r < nRes) {
+      const int g = resNodes[r];
+      double diff = expNr[g] - (double)kept[g] * nrC;
+      while (diff > 0 && c < (1 << 20)) {
+        c++;
+        diff -= nrC;
+      }
+    }
+    int tot;
+    const int ex = blockExclusiveScan(c, &tot);
+    if (r < nRes)
+      injBase[r] = (int32_t)(carry + ex);
+    carry += tot;
+  }
+  if (threadIdx.x == 0)
+    *total = carry;
+}
+
+// emcElectron::generateInjectedParticle + initParticlePos (2-D)
+template <class T, class Src>
+__device__ __forceinline__ void initParticle2D(const ModelK<T> &M, const DevK &G, int cx, int cy,
+                                               int region, bool tauRegionIsValley, Src &rng,
+                                               T k[3], T pos[2], T &E, T &tau, T &gtau,
+                                               int &valley, int &sub) {
+  const int c[2] = {cx, cy};
+  const int ext[2] = {G.nx, G.ny};
+  const double h[2] = {G.hx, G.hy};
+#pragma unroll
+  for (int d = 0; d < 2; d++) {
+    if (c[d] == ext[d] - 1)
+      pos[d] = ((T)c[d] - rng.u01() * T(0.5)) * (T)h[d];
+    else if (c[d] == 0)
+      pos[d] = rng.u01() * T(0.5) * (T)h[d];
+    else
+      pos[d] = ((T)c[d] + rng.u01() - T(0.5)) * (T)h[d];
+  }
+  valley = (int)m_floor((T)M.nV * rng.ulog());
+  const ValleyK<T> &V = M.v[valley];
+  sub = (int)m_floor((T)V.deg * rng.ulog());
+  E = T(-1.5) * (T)G.Vt * drawLog(M, rng.ulog());
+  randomDirection(V.cK * m_sqrt(gammaOf(V, E)), rng, k);
+#pragma unroll
+  for (int d = 0; d < 2; d++)
+    if ((c[d] == 0 && k[d] < T(0)) || (c[d] == ext[d] - 1 && k[d] > T(0)))
+      k[d] *= T(-1);
+  tau = -drawLog(M, rng.ulog()) * tauOf(M, valley, tauRegionIsValley ? valley : region);
+  gtau = -drawLog(M, rng.ulog()) * M.grainTau;
+}
+
+// (behind the *nBase particles that stay; the new number to *nPtr.  SCHEME >= 0:
+// the injected ones' charge is assigned too)
+template <class T, bool REPLAY, int SCHEME>
+__global__ void injectKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
+                             const int32_t *__restrict__ resNodes, int nRes,
+                             const int32_t *__restrict__ injBase, const int64_t *__restrict__ injTotal,
+                             const int64_t *__restrict__ nBase, int64_t *__restrict__ nPtr,
+                             int64_t capacity, uint32_t step,
+                             uint32_t key0, uint32_t key1, uint32_t stream, bool tauRegionIsValley,
+                             int32_t *__restrict__ remInj, const uint64_t *__restrict__ rw,
+                             const int64_t *__restrict__ roff, int *__restrict__ err, double nrC,
+                             int fixBits, unsigned long long *__restrict__ fix) {
+  const int64_t total = *injTotal;
+  const int64_t n = *nBase;
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j == 0)
+    *nPtr = n + total <= capacity ? n + total : n;
+  if (j >= total)
+    return;
+  if (n + total > capacity) {
+    if (j == 0)
+      recordErr(err, EMCG_ERR_CAPACITY);
+    return;
+  }
+  int lo = 0, hi = nRes - 1; // last r with injBase[r] <= j
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (injBase[mid] <= j)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  const int g = resNodes[lo];
+  const int cx = g % G.nx, cy = g / G.nx;
+  const int region = G.region[g];
+  T k[3], pos[2], E, tau, gtau;
+  int valley, sub;
+  const ModelK<T> &M = models[0];
+  if constexpr (REPLAY) {
+    ReplaySrc src{rw, roff[j], roff[j + 1], 0};
+    initParticle2D(M, G, cx, cy, region, tauRegionIsValley, src, k, pos, E, tau, gtau, valley, sub);
+    if (src.bad || src.pos != src.end)
+      recordErr(err, EMCG_ERR_REPLAY);
+  } else {
+    PhiloxSrc<T> src;
+    src.init((uint32_t)j, step, stream | 0x80000000u, key0, key1);
+    initParticle2D(M, G, cx, cy, region, tauRegionIsValley, src, k, pos, E, tau, gtau, valley, sub);
+  }
+  const int64_t d = n + j;
+  st.kx[d] = k[0];
+  st.ky[d] = k[1];
+  st.kz[d] = k[2];
+  st.px[d] = pos[0];
+  st.py[d] = pos[1];
+  st.pz[d] = T(0);
+  st.E[d] = E;
+  st.tau[d] = tau;
+  st.gtau[d] = gtau;
+  st.meta[d] = packMeta(valley, sub, region);
+  atomicAdd(&remInj[G.nodeContact[g]], 1);
+  if constexpr (SCHEME >= 0)
+    assignParticle<T, SCHEME>(G, pos[0], pos[1], nrC, fixBits, fix);
+}
+
+// initial particles at given nodes (counts decided on the host)
+template <class T>
+__global__ void devInitKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
+                              const int32_t *__restrict__ nodeOf, int64_t n, uint32_t key0,
+                              uint32_t key1, uint32_t stream, bool tauRegionIsValley) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n)
+    return;
+  const int g = nodeOf[i];
+  const int region = G.region[g];
+  T k[3], pos[2], E, tau, gtau;
+  int valley, sub;
+  PhiloxSrc<T> src;
+  src.init((uint32_t)i, 0xFFFFFFFFu, stream, key0, key1);
+  initParticle2D(models[0], G, g % G.nx, g / G.nx, region, tauRegionIsValley, src, k, pos, E,
+                 tau, gtau, valley, sub);
+  st.kx[i] = k[0];
+  st.ky[i] = k[1];
+  st.kz[i] = k[2];
+  st.px[i] = pos[0];
+  st.py[i] = pos[1];
+  st.pz[i] = T(0);
+  st.E[i] = E;
+  st.tau[i] = tau;
+  st.gtau[i] = gtau;
+  st.meta[i] = packMeta(valley, sub, region);
+}
+
+// The outcome of a step, written by its last kernel into a page-locked block that
+// the host reads after the step's event: no copy follows on the stream.
+struct StepOut {
+  int32_t *host; // NULL: none; [nc] netto counts, then the error word
+  const int32_t *netto, *remInj;
+  const int *err;
+  int nc;
+};
 // the fixed-point sums as particle counts, and the concentration
 // (include/emcSimulationResults.hpp:98-116)
 __global__ void concKernel(DevK G, const unsigned long long *__restrict__ fix, int fixBits,
-                           double *__restrict__ nr, double *__restrict__ conc) {
+                           double *__restrict__ nr, double *__restrict__ conc, StepOut out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (out.host)
+    for (int j = i; j <= out.nc; j += gridDim.x * blockDim.x)
+      out.host[j] = j < out.nc ? out.netto[j] - out.remInj[j] : *out.err;
   if (i >= G.nx * G.ny)
     return;
   nr[i] = ldexp((double)fix[2 * i + 1], 64 - fixBits) + ldexp((double)fix[2 * i], -fixBits);
@@ -948,6 +1034,14 @@ __global__ void concKernel(DevK G, const unsigned long long *__restrict__ fix, i
   conc[i] = c;
 }
 
+// The counters and sums that a step's kernels start from at zero (kept == NULL:
+// none), cleared by the step's first kernel rather than by a memset each.
+struct StepZero {
+  int32_t *kept;           // per node
+  unsigned long long *fix; // two words per node
+  int32_t *dropCount, *netto, *remInj;
+  int nDrop, nc; // entries of dropCount; of netto and remInj
+};
 // The E field of the PM scheme.  NGP, CIC: at the grid points
 // (include/PMSchemes/emcEFieldCalculation.hpp:13-30).  NEC: forward differences
 // on the edges (calcEFieldAtEdgeMidPts, :35-52).  Both then take the boundary
@@ -956,10 +1050,21 @@ __global__ void concKernel(DevK G, const unsigned long long *__restrict__ fix, i
 // differences, 0 on the last edge, no boundary pass.
 template <class T>
 __global__ void efieldKernel(DevK G, const double *__restrict__ pot, T *__restrict__ Ex,
-                             T *__restrict__ Ey, int scheme) {
+                             T *__restrict__ Ey, int scheme, StepZero z) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (z.kept)
+    for (int j = i; j < max(z.nDrop, z.nc); j += gridDim.x * blockDim.x) {
+      if (j < z.nDrop)
+        z.dropCount[j] = 0;
+      if (j < z.nc)
+        z.netto[j] = z.remInj[j] = 0;
+    }
   if (i >= G.nx * G.ny)
     return;
+  if (z.kept) {
+    z.kept[i] = 0;
+    z.fix[2 * i] = z.fix[2 * i + 1] = 0;
+  }
   const int nx = G.nx, ny = G.ny, x = i % nx, y = i / nx;
   const bool edges = scheme == EMCG_PM_NEC || scheme == EMCG_PM_NEC_VWD;
   auto ex = [&](int xi) {
@@ -1034,6 +1139,7 @@ struct DeviceImpl {
   int32_t *dGList = nullptr, *dGNode = nullptr; // reservoir particles in index order
   int32_t *dResNodes = nullptr, *dInjCount = nullptr;
   int32_t *dNetto = nullptr, *dRemInj = nullptr;
+  int32_t *hOut = nullptr, *hOutDev = nullptr; // a step's outcome (StepOut): host, device address
   // deposition: 128-bit fixed-point node sums (low, high word) at 2^fixBits
   // (double engine) or 2^fixBitsF (float engine, low word only)
   unsigned long long *dNodeFix = nullptr;
@@ -1137,6 +1243,7 @@ int32_t destroyDevice(emcg_handle *h) {
   freeRateScratch(d->rateScratch);
   for (void *p : ps)
     cudaFree(p);
+  cudaFreeHost(d->hOut);
   for (int b = 0; b < 4; b++)
     cudaFree(d->dBnd[b]);
   for (int w = 0; w < 2; w++) {
@@ -1357,6 +1464,9 @@ extern "C" int32_t emcg_device_create(const emcg_model_desc *model, const emcg_d
        cudaMalloc(&d->dInjCount, (d->resNodesH.size() + 1) * sizeof(int32_t)) == cudaSuccess &&
        cudaMalloc(&d->dNetto, (d->nContacts + 1) * sizeof(int32_t)) == cudaSuccess &&
        cudaMalloc(&d->dRemInj, (d->nContacts + 1) * sizeof(int32_t)) == cudaSuccess &&
+       cudaHostAlloc(&d->hOut, (d->nContacts + 1) * sizeof(int32_t), cudaHostAllocMapped) ==
+           cudaSuccess &&
+       cudaHostGetDevicePointer(&d->hOutDev, d->hOut, 0) == cudaSuccess &&
        cudaMalloc(&d->dNodeFix, 2 * n * sizeof(unsigned long long)) == cudaSuccess &&
        cudaMalloc(&d->dErr, sizeof(int)) == cudaSuccess;
   if (!ok) {
@@ -1453,27 +1563,47 @@ extern "C" int32_t emcg_device_create(const emcg_model_desc *model, const emcg_d
 
 namespace emcg {
 
-template <class T> static int32_t efieldT(DeviceImpl *d) {
+template <class T> static int32_t efieldT(DeviceImpl *d, const StepZero &zero = StepZero{}) {
   const int n = d->nx * d->ny;
   efieldKernel<T><<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dPot, (T *)d->dEx,
-                                                          (T *)d->dEy, d->cfg.pm_scheme);
+                                                          (T *)d->dEy, d->cfg.pm_scheme, zero);
   EMCG_CUDA(cudaGetLastError());
   return EMCG_OK;
 }
 
-static int32_t compact(DeviceImpl *d) {
+// fixed-point exponent of the engine's charge sums
+static int fixBitsOf(const DeviceImpl *d) { return d->precision == EMCG_FP64 ? d->fixBits : d->fixBitsF; }
+
+// The particles not marked in dDrop, of which dBlock holds the number per block,
+// to the other state; their number to dN[1].  assign: their charge is assigned
+// in the same pass.
+template <class T> static int32_t compactT(DeviceImpl *d, bool assign) {
   const int nb = d->nBlocks();
-  compactCountKernel<<<nb, kCB, 0, d->stream>>>(d->dDrop, d->dN, d->dBlock);
-  scanBlocksKernel<<<1, 1024, 0, d->stream>>>(d->dBlock, nb, d->dN + 1);
-  if (d->precision == EMCG_FP64)
-    compactScatterKernel<double><<<nb, kCB, 0, d->stream>>>(
-        devState<double>(d, d->cur), devState<double>(d, 1 - d->cur), d->dDrop, d->dN, d->dBlock);
-  else
-    compactScatterKernel<float><<<nb, kCB, 0, d->stream>>>(
-        devState<float>(d, d->cur), devState<float>(d, 1 - d->cur), d->dDrop, d->dN, d->dBlock);
+  const bool scanned = nb > kPrefixBlocks;
+  if (scanned)
+    scanBlocksKernel<<<1, 1024, 0, d->stream>>>(d->dBlock, nb, d->dN + 1);
+  auto k = compactScatterKernel<T, -1>;
+  if (assign)
+    k = d->cfg.pm_scheme == EMCG_PM_NGP   ? compactScatterKernel<T, EMCG_PM_NGP>
+        : d->cfg.pm_scheme == EMCG_PM_CIC ? compactScatterKernel<T, EMCG_PM_CIC>
+                                          : compactScatterKernel<T, EMCG_PM_NEC>;
+  k<<<nb, kCB, 0, d->stream>>>(devState<T>(d, d->cur), devState<T>(d, 1 - d->cur), devK(d), d->dDrop,
+                               d->dN, d->dBlock, d->dN + 1, scanned, d->cfg.carriers_per_particle,
+                               fixBitsOf(d), d->dNodeFix);
   EMCG_CUDA(cudaGetLastError());
-  EMCG_CUDA(cudaMemcpyAsync(d->dN, d->dN + 1, sizeof(int64_t), cudaMemcpyDeviceToDevice, d->stream));
   d->cur = 1 - d->cur;
+  return EMCG_OK;
+}
+// the injection kernel that assigns the charge by the engine's scheme, or assigns none
+template <class T, bool REPLAY> static auto injectOf(const DeviceImpl *d, bool assign) {
+  return !assign                              ? injectKernel<T, REPLAY, -1>
+         : d->cfg.pm_scheme == EMCG_PM_NGP ? injectKernel<T, REPLAY, EMCG_PM_NGP>
+         : d->cfg.pm_scheme == EMCG_PM_CIC ? injectKernel<T, REPLAY, EMCG_PM_CIC>
+                                           : injectKernel<T, REPLAY, EMCG_PM_NEC>;
+}
+// the new number of particles, where no injection writes it
+static int32_t keepCount(DeviceImpl *d) {
+  EMCG_CUDA(cudaMemcpyAsync(d->dN, d->dN + 1, sizeof(int64_t), cudaMemcpyDeviceToDevice, d->stream));
   return EMCG_OK;
 }
 
@@ -1497,20 +1627,22 @@ template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compa
   const ModelK<T> *M = (const ModelK<T> *)d->dModel;
   const T *Ex = (const T *)d->dEx, *Ey = (const T *)d->dEy;
   DevK G = devK(d);
+  if (compactAfter) // a step's first kernel has cleared them
+    EMCG_CUDA(cudaMemsetAsync(d->dBlock, 0, d->nBlocks() * sizeof(int32_t), d->stream));
   bool rep = d->replay[0];
   if (rep && sizeof(T) != 8) {
     setError("replay needs the FP64 engine");
     return EMCG_ERR_ARG;
   }
 #define EMCG_MOVEQ(SCH)                                                                          \
-  devMoveQueuedKernel<SCH><<<nb, 256, 0, d->stream>>>(                                    \
-      st, M, G, Ex, Ey, c.charge, c.dt, d->dN, step, k0, k1, c.stream, d->dDrop, d->dNetto,      \
-      d->dErr)
+  devMoveQueuedKernel<SCH><<<nb, 256, 0, d->stream>>>(                                           \
+      st, M, G, Ex, Ey, c.charge, c.dt, d->dN, step, k0, k1, c.stream, d->dDrop, d->dBlock,      \
+      d->dNetto, d->dErr)
 #define EMCG_MOVE(SCH, REP)                                                                      \
   moveKernel<T, SCH, REP>(d->surfaces)                                                           \
       <<<nb, 256, 0, d->stream>>>(st, M, G, Ex, Ey, (T)c.charge, (T)c.dt, d->dN, step, k0, k1,    \
-                                  c.stream, d->dDrop, d->dNetto, d->dWords[0], d->dOff[0],        \
-                                  d->dErr)
+                                  c.stream, d->dDrop, d->dBlock, d->dNetto, d->dWords[0],         \
+                                  d->dOff[0], d->dErr)
   if (rep) {
     if constexpr (sizeof(T) == 8) {
       if (c.pm_scheme == EMCG_PM_NGP)
@@ -1548,84 +1680,89 @@ template <class T> static int32_t moveT(DeviceImpl *d, uint32_t step, bool compa
 #undef EMCG_MOVEQ
   EMCG_CUDA(cudaGetLastError());
   d->replay[0] = false;
-  return compactAfter ? compact(d) : EMCG_OK;
+  if (compactAfter) {
+    EMCG_TRY(compactT<T>(d, false));
+    EMCG_TRY(keepCount(d));
+  }
+  return EMCG_OK;
 }
 
 // movedDrops: the move's removals are still marked in dDrop (moveT without its
 // compaction); the reservoir list skips them and one compaction removes both.
 // The ranks are those of the compacted order, since compaction is stable.
+// They are part of a step then, whose first kernel cleared the counters, and the
+// charge is assigned on the way.
 template <class T> static int32_t contactsT(DeviceImpl *d, uint32_t step, bool movedDrops = false) {
   const int nb = d->nBlocks();
   const int n = d->nx * d->ny;
   cudaStream_t st = d->stream;
   DevK G = devK(d);
   const int nRes = (int)d->resNodesH.size();
-  if (!movedDrops)
+  if (!movedDrops) {
     EMCG_CUDA(cudaMemsetAsync(d->dDrop, 0, d->capacity, st));
-  EMCG_CUDA(cudaMemsetAsync(d->dKept, 0, n * sizeof(int32_t), st));
+    EMCG_CUDA(cudaMemsetAsync(d->dBlock, 0, nb * sizeof(int32_t), st));
+    EMCG_CUDA(cudaMemsetAsync(d->dKept, 0, n * sizeof(int32_t), st));
+  }
   reservoirListKernel<T><<<nb, kCB, 0, st>>>(devState<T>(d, d->cur), G, d->dN,
                                              movedDrops ? d->dDrop : nullptr, d->dList,
                                              d->dListNode, d->dListCount);
-  scanBlocksKernel<<<1, 1024, 0, st>>>(d->dListCount, nb, d->dN + 3);
-  gatherListKernel<<<nb, 256, 0, st>>>(d->dList, d->dListNode, d->dListCount, nb, d->dN + 3,
-                                       d->dGList, d->dGNode);
+  const bool scanned = nb > kPrefixBlocks;
+  if (scanned)
+    scanBlocksKernel<<<1, 1024, 0, st>>>(d->dListCount, nb, d->dN + 3);
+  gatherListKernel<<<nb, 256, 0, st>>>(d->dList, d->dListNode, d->dListCount, nb, scanned,
+                                       d->dN + 3, d->dGList, d->dGNode);
   if (nRes > 0) {
     const unsigned rb = (unsigned)(((int64_t)nRes * kRankChunks * 32 + 255) / 256);
     contactCountKernel<<<rb, 256, 0, st>>>(d->dGNode, d->dN + 3, d->dResNodes, nRes,
                                            d->dChunkCount);
     contactRankKernel<<<rb, 256, 0, st>>>(d->dGList, d->dGNode, d->dN + 3, d->dResNodes, nRes,
                                           d->dExp, d->cfg.carriers_per_particle,
-                                          d->dNodeContact, d->dChunkCount, d->dDrop, d->dKept,
-                                          d->dRemInj);
+                                          d->dNodeContact, d->dChunkCount, d->dDrop, d->dBlock,
+                                          d->dKept, d->dRemInj);
   }
   EMCG_CUDA(cudaGetLastError());
-  EMCG_TRY(compact(d));
+  EMCG_TRY(compactT<T>(d, movedDrops));
   if (nRes == 0)
-    return EMCG_OK;
-  injectCountKernel<<<(nRes + 255) / 256, 256, 0, st>>>(d->dResNodes, nRes, d->dExp, d->dKept,
-                                                        d->cfg.carriers_per_particle, d->dInjCount);
-  scanBlocksKernel<<<1, 1024, 0, st>>>(d->dInjCount, nRes, d->dN + 2);
+    return keepCount(d);
+  injectCountKernel<<<1, 1024, 0, st>>>(d->dResNodes, nRes, d->dExp, d->dKept,
+                                        d->cfg.carriers_per_particle, d->dInjCount, d->dN + 2);
   const emcg_device_config &c = d->cfg;
   uint32_t k0 = (uint32_t)c.seed, k1 = (uint32_t)(c.seed >> 32);
   const int ib = (int)((d->injBound + 255) / 256);
-  bool rep = d->replay[1];
-  if (rep) {
-    if constexpr (sizeof(T) == 8)
-      injectKernel<T, true><<<ib, 256, 0, st>>>(
-          devState<T>(d, d->cur), (const ModelK<T> *)d->dModel, G, d->dResNodes, nRes,
-          d->dInjCount, d->dN + 2, d->dN, d->capacity, step, k0, k1, c.stream,
-          c.tau_region_is_valley != 0, d->dRemInj, d->dWords[1], d->dOff[1], d->dErr);
-  } else {
-    injectKernel<T, false><<<ib, 256, 0, st>>>(
-        devState<T>(d, d->cur), (const ModelK<T> *)d->dModel, G, d->dResNodes, nRes,
-        d->dInjCount, d->dN + 2, d->dN, d->capacity, step, k0, k1, c.stream,
-        c.tau_region_is_valley != 0, d->dRemInj, nullptr, nullptr, d->dErr);
-  }
-  addCountKernel<<<1, 1, 0, st>>>(d->dN, d->dN + 2, d->capacity);
+  const bool rep = d->replay[1];
+  auto k = injectOf<T, false>(d, movedDrops);
+  if constexpr (sizeof(T) == 8)
+    if (rep)
+      k = injectOf<T, true>(d, movedDrops);
+  k<<<ib, 256, 0, st>>>(devState<T>(d, d->cur), (const ModelK<T> *)d->dModel, G, d->dResNodes, nRes,
+                        d->dInjCount, d->dN + 2, d->dN + 1, d->dN, d->capacity, step, k0, k1,
+                        c.stream, c.tau_region_is_valley != 0, d->dRemInj,
+                        rep ? d->dWords[1] : nullptr, rep ? d->dOff[1] : nullptr, d->dErr,
+                        c.carriers_per_particle, fixBitsOf(d), d->dNodeFix);
   EMCG_CUDA(cudaGetLastError());
   d->replay[1] = false;
+  return EMCG_OK;
+}
+
+// the concentration from the charge sums; out: a step's outcome to the host
+static int32_t concentration(DeviceImpl *d, const StepOut &out = StepOut{}) {
+  const int n = d->nx * d->ny;
+  concKernel<<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dNodeFix, fixBitsOf(d), d->dNr,
+                                                     d->dConc, out);
+  EMCG_CUDA(cudaGetLastError());
   return EMCG_OK;
 }
 
 template <class T> static int32_t assignT(DeviceImpl *d) {
   const int n = d->nx * d->ny;
   const int nb = (int)((d->capacity + 255) / 256);
-  const int fb = sizeof(T) == 4 ? d->fixBitsF : d->fixBits;
-  const double nrC = d->cfg.carriers_per_particle;
-  const StateK<T> st = devState<T>(d, d->cur);
   EMCG_CUDA(cudaMemsetAsync(d->dNodeFix, 0, 2 * n * sizeof(unsigned long long), d->stream));
-  if (d->cfg.pm_scheme == EMCG_PM_NGP)
-    assignKernel<T, EMCG_PM_NGP><<<nb, 256, 0, d->stream>>>(st, devK(d), d->dN, nrC, fb,
-                                                           d->dNodeFix);
-  else if (d->cfg.pm_scheme == EMCG_PM_CIC)
-    assignKernel<T, EMCG_PM_CIC><<<nb, 256, 0, d->stream>>>(st, devK(d), d->dN, nrC, fb,
-                                                           d->dNodeFix);
-  else
-    assignKernel<T, EMCG_PM_NEC><<<nb, 256, 0, d->stream>>>(st, devK(d), d->dN, nrC, fb,
-                                                           d->dNodeFix);
-  concKernel<<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dNodeFix, fb, d->dNr, d->dConc);
-  EMCG_CUDA(cudaGetLastError());
-  return EMCG_OK;
+  auto k = d->cfg.pm_scheme == EMCG_PM_NGP   ? assignKernel<T, EMCG_PM_NGP>
+           : d->cfg.pm_scheme == EMCG_PM_CIC ? assignKernel<T, EMCG_PM_CIC>
+                                             : assignKernel<T, EMCG_PM_NEC>;
+  k<<<nb, 256, 0, d->stream>>>(devState<T>(d, d->cur), devK(d), d->dN, d->cfg.carriers_per_particle,
+                               fixBitsOf(d), d->dNodeFix);
+  return concentration(d);
 }
 
 static int32_t poissonRun(DeviceImpl *d, bool eq, bool reset, double *rel, int *cycles) {
@@ -1822,7 +1959,6 @@ extern "C" int32_t emcg_device_step(emcg_handle *h, int32_t n_steps, uint32_t st
   EMCG_TRY(devOf(h, &d));
   EMCG_CHECK_ARG(n_steps >= 0, "n_steps must be >= 0");
   const int nc = d->nContacts;
-  std::vector<int32_t> hn(2 * (nc + 1));
   double stepMs = 0, poisMs = 0;
   d->poissonCycles = d->poissonSolves = 0;
   for (int s = 0; s < n_steps; s++) {
@@ -1839,22 +1975,17 @@ extern "C" int32_t emcg_device_step(emcg_handle *h, int32_t n_steps, uint32_t st
     d->bcReset = false;
     if (ps)
       return ps;
-    EMCG_TRY(d->precision == EMCG_FP64 ? efieldT<double>(d) : efieldT<float>(d));
-    EMCG_CUDA(cudaMemsetAsync(d->dNetto, 0, (nc + 1) * sizeof(int32_t), d->stream));
-    EMCG_CUDA(cudaMemsetAsync(d->dRemInj, 0, (nc + 1) * sizeof(int32_t), d->stream));
-    // one compaction per step, after the contacts (the move's removals wait marked)
+    const StepZero zero = {d->dKept, d->dNodeFix, d->dBlock, d->dNetto, d->dRemInj, d->nBlocks(),
+                           nc + 1};
+    EMCG_TRY(d->precision == EMCG_FP64 ? efieldT<double>(d, zero) : efieldT<float>(d, zero));
+    // one compaction per step, after the contacts (the move's removals wait
+    // marked), which assigns the charge too
     EMCG_TRY(d->precision == EMCG_FP64 ? moveT<double>(d, step0 + s, false)
                                        : moveT<float>(d, step0 + s, false));
     EMCG_TRY(d->precision == EMCG_FP64 ? contactsT<double>(d, step0 + s, true)
                                        : contactsT<float>(d, step0 + s, true));
-    EMCG_TRY(d->precision == EMCG_FP64 ? assignT<double>(d) : assignT<float>(d));
+    EMCG_TRY(concentration(d, {d->hOutDev, d->dNetto, d->dRemInj, d->dErr, nc}));
     EMCG_CUDA(cudaEventRecord(d->ev[1], d->stream));
-    if (netto) {
-      EMCG_CUDA(cudaMemcpyAsync(hn.data(), d->dNetto, nc * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                d->stream));
-      EMCG_CUDA(cudaMemcpyAsync(hn.data() + nc + 1, d->dRemInj, nc * sizeof(int32_t),
-                                cudaMemcpyDeviceToHost, d->stream));
-    }
     EMCG_CUDA(cudaEventSynchronize(d->ev[1]));
     float ms = 0;
     cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]);
@@ -1868,10 +1999,11 @@ extern "C" int32_t emcg_device_step(emcg_handle *h, int32_t n_steps, uint32_t st
     d->poissonSolves++;
     if (ps)
       return ps;
-    EMCG_TRY(readErr(d));
+    if (d->hOut[nc])
+      EMCG_TRY(readErr(d));
     if (netto)
       for (int c = 0; c < nc; c++)
-        netto[(int64_t)s * nc + c] = hn[c] - hn[nc + 1 + c];
+        netto[(int64_t)s * nc + c] = d->hOut[c];
   }
   d->stepMs = stepMs;
   d->poissonMs = poisMs;
