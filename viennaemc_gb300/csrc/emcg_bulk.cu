@@ -1168,13 +1168,13 @@ template <class T>
 static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nModels,
                            const emcg_ensemble_desc *ens, int nEns) {
   std::vector<ModelK<T>> mk(nModels);
-  if (sizeof(T) == 8)
-    EMCG_TRY(uploadLogTable(&b->dLogTab));
   b->dTables.assign(nModels, nullptr);
   b->rates.resize(nModels);
   for (int i = 0; i < nModels; i++) {
     std::vector<T> tab;
     EMCG_TRY(buildModelK<T>(models[i], mk[i], tab));
+    if (sizeof(T) == 8 && !b->dLogTab) // (after a model's own checks)
+      EMCG_TRY(uploadLogTable(&b->dLogTab));
     b->rates[i] = rateLayoutOf(models[i]);
     EMCG_CUDA(cudaMalloc(&b->dTables[i], tab.size() * sizeof(T)));
     EMCG_CUDA(cudaMemcpy(b->dTables[i], tab.data(), tab.size() * sizeof(T),
