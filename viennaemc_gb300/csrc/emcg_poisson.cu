@@ -81,6 +81,12 @@ __device__ __forceinline__ double dmaxPos(double a, double b) {
                          (unsigned long long)__double_as_longlong(b)));
 }
 
+// a > 0, and a < b, for non-negative a and b, without a double-precision instruction
+__device__ __forceinline__ bool bitsPositive(double a) { return __double_as_longlong(a) > 0; }
+__device__ __forceinline__ bool bitsBelow(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
 // F(phi) at node i = (x, y) of the reference equation (the SOR fixed point
 // of emcSORSolver.hpp:131-197 times the FV area), with p = exp(-phi) and n
 // (the concentration, or exp(phi) at equilibrium).  Both solve paths call this
@@ -91,31 +97,50 @@ __device__ __forceinline__ double dmaxPos(double a, double b) {
 struct NodeF {
   double F, p, n;
 };
-__device__ __forceinline__ NodeF nodeResidual(const double *__restrict__ pot,
-                                              const double *__restrict__ conc,
-                                              const double *__restrict__ C,
-                                              const double *__restrict__ gSum,
-                                              const double *__restrict__ gV, int i, int x, int y,
-                                              int nx, int ny, double hF0, double hF1, double c2,
-                                              double hP, const double *tab) {
-  const double phi = pot[i];
-  const double w = x > 0 ? pot[i - 1] : pot[i + 1];
-  const double e = x < nx - 1 ? pot[i + 1] : pot[i - 1];
-  const double s = y > 0 ? pot[i - nx] : pot[i + nx];
-  const double nn = y < ny - 1 ? pot[i + nx] : pot[i - nx];
-  const double gs = gSum[i], gv = gV[i];
+struct NodeIn { // what it reads: the potential at the node and beside it, the rest there
+  double phi, w, e, s, nn, gs, gv, conc, C;
+};
+__device__ __forceinline__ NodeIn nodeLoad(const double *__restrict__ pot,
+                                           const double *__restrict__ conc,
+                                           const double *__restrict__ C,
+                                           const double *__restrict__ gSum,
+                                           const double *__restrict__ gV, int i, int x, int y,
+                                           int nx, int ny) {
+  NodeIn q;
+  q.phi = pot[i];
+  q.w = x > 0 ? pot[i - 1] : pot[i + 1];
+  q.e = x < nx - 1 ? pot[i + 1] : pot[i - 1];
+  q.s = y > 0 ? pot[i - nx] : pot[i + nx];
+  q.nn = y < ny - 1 ? pot[i + nx] : pot[i - nx];
+  q.gs = gSum[i];
+  q.gv = gV[i];
+  q.conc = conc ? conc[i] : 0.;
+  q.C = C[i];
+  return q;
+}
+__device__ __forceinline__ NodeF nodeResidual(const NodeIn &q, bool conc, double hF0, double hF1,
+                                              double c2, double hP, const double *tab) {
   NodeF r;
-  r.p = expTab(-phi, tab);
-  r.n = conc ? conc[i] : expTab(phi, tab);
-  double F = hF0 * (w + e);
-  F = fma(hF1, s + nn, F);
-  F = fma(c2, phi, F); // c2 = -2 (hF0 + hF1)
-  F = fma(hP, (r.p - r.n) + C[i], F);
-  if (((__double_as_longlong(gs) | __double_as_longlong(gv)) << 1) != 0)
-    F += gv - gs * phi;
+  r.p = expTab(bitsd(dbits(q.phi) ^ 0x8000000000000000ull), tab);
+  r.n = conc ? q.conc : expTab(q.phi, tab);
+  double F = hF0 * (q.w + q.e);
+  F = fma(hF1, q.s + q.nn, F);
+  F = fma(c2, q.phi, F); // c2 = -2 (hF0 + hF1)
+  F = fma(hP, (r.p - r.n) + q.C, F);
+  if (((__double_as_longlong(q.gs) | __double_as_longlong(q.gv)) << 1) != 0)
+    F += q.gv - q.gs * q.phi;
   r.F = F;
   return r;
 }
+// in the multigrid's type, and back
+template <class MT> __device__ __forceinline__ MT mgOf(double x) {
+  if constexpr (sizeof(MT) == 4)
+    return toFloat(x);
+  else
+    return x;
+}
+__device__ __forceinline__ double doubleOf(float v) { return toDouble(v); }
+__device__ __forceinline__ double doubleOf(double v) { return v; }
 
 // F(phi) of the reference equation, the Jacobian's reaction density and the
 // FV-scaled right-hand side of the correction equation on level 0.
@@ -140,15 +165,15 @@ __global__ void nonlinResidualKernel(const double *__restrict__ pot, const doubl
       rho[i] = MT(0);
     } else {
       int x = i % nx, y = i / nx;
-      const NodeF q = nodeResidual(pot, conc, C, gSum, gV, i, x, y, nx, ny, hF0, hF1,
-                                   -2.0 * (hF0 + hF1), hP, tab);
+      const NodeF q = nodeResidual(nodeLoad(pot, conc, C, gSum, gV, i, x, y, nx, ny),
+                                   conc != nullptr, hF0, hF1, -2.0 * (hF0 + hF1), hP, tab);
       const double F = q.F, p = q.p, n = q.n;
       int bd = (x == 0 || x == nx - 1) + (y == 0 || y == ny - 1);
       // the FV scale (1, 1/2, 1/4) and the maxima in the multigrid's type:
       // exact scalings, and the maximum needs no more than float accuracy
-      const MT fF = (MT)F;
+      const MT fF = mgOf<MT>(F);
       rhs[i] = fF * (bd == 0 ? MT(1) : (bd == 1 ? MT(0.5) : MT(0.25)));
-      rho[i] = (MT)(conc ? p : p + n);
+      rho[i] = mgOf<MT>(conc ? p : p + n);
       aF = fabs(fF);
       if (withScale)
         sc = hP * (fabs(C[i]) + n + p);
@@ -190,7 +215,7 @@ __global__ void updatePotKernel(double *__restrict__ pot, const MT *__restrict__
     // reports it
     if (isfinite(v))
       v = fmin(MT(kMaxNewtonStep), fmax(MT(-kMaxNewtonStep), v));
-    pot[i] += (double)v;
+    pot[i] += doubleOf(v);
     a = isfinite(v) ? fabs(v) : MT(INFINITY);
   }
   double m = blockMax((double)a);
@@ -1175,11 +1200,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       out[2] = -1.;
     return;
   }
-  // Staging.  Every table goes by asynchronous copies, all in flight at once
-  // (a plain copy loop per table waited for each table's loads in turn: 20 us
-  // per launch), in two groups: the exp table and level 0's coefficient
-  // classes, which the first residual needs, and then the rest, which lands
-  // while the first residual runs (it is first needed by the V-cycle).
+  // Staging.  The exp table and level 0's coefficient classes, which the first
+  // residual needs, come first; the rest (first needed by the V-cycle) is fetched
+  // beside it (stageRest).
   const unsigned sBaseAddr = (unsigned)__cvta_generic_to_shared(smem);
   if (!kTail) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(sExp);
@@ -1196,9 +1219,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
   if (threadIdx.x < ranks)
     sBase[threadIdx.x] = static_cast<char *>(cluster.map_shared_rank((void *)smem, threadIdx.x));
-  auto stage = [&](unsigned off, const void *src, int n) {
+  // n words from src to byte off, by the threads t0, t0 + stride, ...
+  auto stage = [&](unsigned off, const void *src, int n, int t0, int stride) {
     const int *sp = static_cast<const int *>(src);
-    for (int k = threadIdx.x; k < n; k += blockDim.x)
+    for (int k = t0; k < n; k += stride)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sBaseAddr + off + 4u * k),
                    "l"(sp + k)
                    : "memory");
@@ -1214,26 +1238,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       clsEnd[l] = nCls;
     }
   }
-  stage(M.L[0].offTab, M.L[0].tab, 8 * M.L[0].nCls * (int)(sizeof(MT) / 4));
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int l = 0; l < M.nLev; l++) {
-    const CLevel<MT> &L = M.L[l];
-    if (l > 0)
-      stage(L.offTab, L.tab, 8 * L.nCls * (int)(sizeof(MT) / 4));
-    if (L.ncx > 0) {
-      stage(L.offPxI, L.pxIdx, L.nx);
-      stage(L.offPxW, L.pxW, L.nx);
-      stage(L.offPyI, L.pyIdx, L.ny);
-      stage(L.offPyW, L.pyW, L.ny);
-      stage(L.offRxI, L.rxIdx, 3 * L.ncx);
-      stage(L.offRxW, L.rxW, 3 * L.ncx);
-      stage(L.offRyI, L.ryIdx, 3 * L.ncy);
-      stage(L.offRyW, L.ryW, 3 * L.ncy);
-      stage(L.offMapX, L.mapX, L.ncx);
-      stage(L.offMapY, L.mapY, L.ncy);
-    }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+  stage(M.L[0].offTab, M.L[0].tab, 8 * M.L[0].nCls * (int)(sizeof(MT) / 4), threadIdx.x,
+        blockDim.x);
   // this CTA's class bytes of the levels [clsEnd[l0 - 1], clsEnd[l1 - 1]), four
   // bytes per thread and pass: the loads first, then the stores
   auto copyCls = [&](int l0, int l1) {
@@ -1263,7 +1269,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     }
   };
   copyCls(0, 1);
-  asm volatile("cp.async.wait_group 1;" ::: "memory"); // the exp table and level 0's classes
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // (no cluster barrier yet: the first access to another CTA's shared memory
   // comes after the cluster barrier of the first residual's maxima)
@@ -1273,10 +1279,33 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   int p0, p1;
   cOwnRows(c, L0, p0, p1);
   const int nOwn = nx * (p1 - p0);
-  // the rest of the staging: the class bytes of the other levels, zero
-  // residuals (Dirichlet nodes keep them), the asynchronous copies; the next
+  // the rest of the staging: the class and transfer tables by asynchronous copies, a
+  // warp per table (the whole block on each in turn took 6 us to issue), the class
+  // bytes of the other levels, zero residuals (Dirichlet nodes keep them); the next
   // cluster barrier makes them visible
   auto stageRest = [&]() {
+    for (int a = threadIdx.x >> 5; a < 11 * M.nLev; a += (int)(blockDim.x >> 5)) {
+      const int l = a / 11, which = a - 11 * l;
+      const CLevel<MT> &L = M.L[l];
+      const void *src = L.tab;
+      unsigned off = L.offTab;
+      int n = l > 0 ? 8 * L.nCls * (int)(sizeof(MT) / 4) : 0;
+      if (which > 0 && L.ncx == 0)
+        continue;
+      switch (which) {
+      case 1: src = L.pxIdx, off = L.offPxI, n = L.nx; break;
+      case 2: src = L.pxW, off = L.offPxW, n = L.nx; break;
+      case 3: src = L.pyIdx, off = L.offPyI, n = L.ny; break;
+      case 4: src = L.pyW, off = L.offPyW, n = L.ny; break;
+      case 5: src = L.rxIdx, off = L.offRxI, n = 3 * L.ncx; break;
+      case 6: src = L.rxW, off = L.offRxW, n = 3 * L.ncx; break;
+      case 7: src = L.ryIdx, off = L.offRyI, n = 3 * L.ncy; break;
+      case 8: src = L.ryW, off = L.offRyW, n = 3 * L.ncy; break;
+      case 9: src = L.mapX, off = L.offMapX, n = L.ncx; break;
+      case 10: src = L.mapY, off = L.offMapY, n = L.ncy; break;
+      }
+      stage(off, src, n, threadIdx.x & 31, 32);
+    }
     copyCls(1, M.nLev);
     for (int l = 0; l < M.nLev; l++) { // the padding around d, and rows past the grid's
       const CLevel<MT> &L = M.L[l];
@@ -1297,7 +1326,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       for (int k = threadIdx.x; k < L.nx * (r1 - r0); k += blockDim.x)
         res[k] = MT(0);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
   };
   if constexpr (kTail) {
     MT *d0 = cRowNearT<true, MT>(c, L0, L0.offD, 0);
@@ -1316,71 +1345,101 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     cluster.sync(); // no CTA leaves while another may still read its shared memory
     return;
   }
-  double rel = INFINITY, scale = 0.;
+  double rel = INFINITY, perScale = 1.;
+  const bool updRule = updTol > 0.;
   int it = 0;
   bool stopped = false;
   const double c2 = -2.0 * (hF0 + hF1);
   for (;; it++) {
     // F(phi), Jacobian reaction and FV-scaled right-hand side (nonlinResidualKernel);
     // the scale of the relative residual from the first iteration's state
+    // Bound by its double-precision instructions on the cluster's few SMs (13 a
+    // node): each node's values are loaded while the one before is worked on, and
+    // the conversions and comparisons go by bits.  With the staging beside it the
+    // 201 x 101 resistor's solve went 0.300 -> 0.283 ms, 401 x 201 0.613 -> 0.568.
     MT aFm = 0;
     double sc = 0.;
-    for (int t = threadIdx.x; t < nOwn; t += blockDim.x) {
-      const int ly = L0.byNx.div(t), y = p0 + ly, x = t - ly * nx, i = y * nx + x;
-      MT *d0 = cRowNearT<true, MT>(c, L0, L0.offD, ly);
-      MT *r0 = cRowNearT<true, MT>(c, L0, L0.offR, ly);
-      MT *rho0 = cRowNearT<true, MT>(c, L0, L0.offRho, ly);
-      d0[x] = MT(0);
-      if (cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, ly)[x]).fixed != MT(0)) {
-        r0[x] = MT(0);
-        rho0[x] = MT(0);
+    auto load = [&](int t) {
+      const int ly = L0.byNx.div(t), y = p0 + ly, x = t - ly * nx;
+      return nodeLoad(pot, conc, C, gSum, gV, y * nx + x, x, y, nx, ny);
+    };
+    // of each scheduler's warps half do their part of the staging first: the
+    // double-precision pipe has the other half's nodes meanwhile
+    const int residualPart = it == 0 ? (int)(threadIdx.x >> 7) & 1 : 0;
+    for (int part = 0; part < 2; part++) {
+      if (part != residualPart) {
+        if (it == 0)
+          stageRest();
         continue;
       }
-      const NodeF q =
-          nodeResidual(pot, conc, C, gSum, gV, i, x, y, nx, ny, hF0, hF1, c2, hP, sExp);
-      const double F = q.F, p = q.p, n = q.n;
-      const int bd = (x == 0 || x == nx - 1) + (y == 0 || y == ny - 1);
-      const MT fF = (MT)F;
-      r0[x] = fF * (bd == 0 ? MT(1) : (bd == 1 ? MT(0.5) : MT(0.25)));
-      rho0[x] = (MT)(conc ? p : p + n);
-      aFm = fmax(aFm, fabs(fF));
-      if (it == 0)
-        sc = dmaxPos(sc, hP * (fabs(C[i]) + n + p));
-      // a NaN would vanish in the maxima: non-finite values count as an
-      // infinite residual, which ends the solve as not converged
-      if (!finiteBits(F) || !finiteBits(p) || !finiteBits(n) || !isfinite(fF))
-        aFm = MT(INFINITY);
+      NodeIn next;
+      if ((int)threadIdx.x < nOwn)
+        next = load(threadIdx.x);
+      for (int t = threadIdx.x; t < nOwn; t += blockDim.x) {
+        const NodeIn in = next;
+        next = load(min(t + (int)blockDim.x, nOwn - 1));
+        const int ly = L0.byNx.div(t), y = p0 + ly, x = t - ly * nx;
+        MT *d0 = cRowNearT<true, MT>(c, L0, L0.offD, ly);
+        MT *r0 = cRowNearT<true, MT>(c, L0, L0.offR, ly);
+        MT *rho0 = cRowNearT<true, MT>(c, L0, L0.offRho, ly);
+        d0[x] = MT(0);
+        if (cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, ly)[x]).fixed != MT(0)) {
+          r0[x] = MT(0);
+          rho0[x] = MT(0);
+          continue;
+        }
+        const NodeF q = nodeResidual(in, conc != nullptr, hF0, hF1, c2, hP, sExp);
+        const double F = q.F, p = q.p, n = q.n;
+        const int bd = (x == 0 || x == nx - 1) + (y == 0 || y == ny - 1);
+        const MT fF = mgOf<MT>(F);
+        r0[x] = fF * (bd == 0 ? MT(1) : (bd == 1 ? MT(0.5) : MT(0.25)));
+        rho0[x] = mgOf<MT>(conc ? p : p + n);
+        aFm = fmax(aFm, fabs(fF));
+        if (it == 0)
+          sc = dmaxPos(sc, hP * (fabs(in.C) + n + p));
+        // a NaN would vanish in the maxima: non-finite values count as an
+        // infinite residual, which ends the solve as not converged
+        if (!finiteBits(F) || !finiteBits(p) || !finiteBits(n) || !isfinite(fF))
+          aFm = MT(INFINITY);
+      }
     }
-    if (it == 0)
-      stageRest();
     double aF = (double)aFm;
     // its cluster barrier also orders the writes above; the maxima are next
     // written after the V-cycle's barriers, when every CTA has read them
     cClusterMax2(c, M.offRed, aF, sc, sh);
     if (it == 0)
-      scale = sc;
-    rel = scale > 0 ? aF / scale : aF;
-    if (rel <= rtol || it == maxCycles || !isfinite(rel))
+      perScale = bitsPositive(sc) ? 1. / sc : 1.;
+    // (every warp takes this decision: comparisons by the bit patterns)
+    rel = aF * perScale;
+    if (!bitsBelow(rtol, rel) || it == maxCycles || !finiteBits(rel))
       break;
     // under the update-size rule a Newton step needs only a rough correction
-    const int nv = updTol <= 0. && rel < M.twoCycleRel ? M.vcycles : 1;
+    const int nv = !updRule && bitsBelow(rel, M.twoCycleRel) ? M.vcycles : 1;
     for (int vc = 0; vc < nv; vc++)
       cVcycle(c, M, cluster);
     // clamped Newton update of this CTA's rows (updatePotKernel); the cluster
     // barrier makes the new values visible to the neighbours' next residual
     MT updM = 0;
-    for (int t = threadIdx.x; t < nOwn; t += blockDim.x) {
-      const int ly = L0.byNx.div(t), x = t - ly * nx;
-      if (cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, ly)[x]).fixed != MT(0))
-        continue;
-      MT v = cRowNearT<true, MT>(c, L0, L0.offD, ly)[x];
-      if (isfinite(v)) // a non-finite correction is passed on to the next residual
-        v = fmin(MT(kMaxNewtonStep), fmax(MT(-kMaxNewtonStep), v));
-      pot[(size_t)(p0 + ly) * nx + x] += (double)v;
-      updM = isfinite(v) ? fmax(updM, fabs(v)) : MT(INFINITY);
+    constexpr int U = 4; // nodes of a thread side by side
+    for (int t0 = threadIdx.x; t0 < nOwn; t0 += U * blockDim.x) {
+      double phi[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        phi[u] = pot[(size_t)p0 * nx + min(t0 + u * (int)blockDim.x, nOwn - 1)];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int t = t0 + u * (int)blockDim.x;
+        if (t >= nOwn || cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, 0)[t]).fixed != MT(0))
+          continue;
+        MT v = cRowNearT<true, MT>(c, L0, L0.offD, 0)[t];
+        if (isfinite(v)) // a non-finite correction is passed on to the next residual
+          v = fmin(MT(kMaxNewtonStep), fmax(MT(-kMaxNewtonStep), v));
+        pot[(size_t)p0 * nx + t] = phi[u] + doubleOf(v);
+        updM = isfinite(v) ? fmax(updM, fabs(v)) : MT(INFINITY);
+      }
     }
     double upd = (double)updM;
-    if (updTol > 0.) {
+    if (updRule) {
       // the maxima of this rule use their own slot (offRed + 16)
       double none = 0.;
       cClusterMax2(c, M.offRed + 16, upd, none, sh);
