@@ -82,3 +82,19 @@ def test_no_allocation_forms(engine, nx, ny, gates):
         200, None, C.byref(rel), C.byref(cyc)))
     assert abs(cyc.value - info[1]) <= 1 and rel.value <= 1e-10
     assert np.max(np.abs(d_pot.cpu().numpy() - want)) <= 1e-8
+
+
+# (columns, rows): two row groups whose last rows are missing in some CTAs; the widest
+# grid of two groups; four groups and an odd width; a column of two rows too many
+@pytest.mark.parametrize("nx,ny", [(401, 197), (511, 120), (303, 229), (255, 301), (305, 263)])
+def test_column_sweeps_equal_one_launch_per_phase(engine, nx, ny):
+    dev = _bar(nx, ny, gates=3)
+    pot, conc = _start(dev, nx + ny)
+    sim = _sim(engine, dev, True)
+    assert sim.poisson_mode(-1) > 1
+    a, ia = _solve(sim, pot, conc)
+    sim.poisson_mode(0)
+    b, ib = _solve(sim, pot, conc)
+    sim.close()
+    assert ia[1] == ib[1]
+    assert np.max(np.abs(a - b)) <= 1e-13 * max(1.0, np.abs(b).max())

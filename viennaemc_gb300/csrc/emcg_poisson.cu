@@ -818,10 +818,146 @@ __device__ __forceinline__ void cSweepsBatch(const CCtx &c, const CLevel<MT> &L,
   }
 }
 
+// Sweeps over a band of more rows than cSweepsHeld takes, held all the same: a
+// thread keeps one column's nodes of either colour in every G-th row, so that their
+// addresses are the first's plus multiples of a constant and a node costs two
+// registers and a byte (right-hand side, reciprocal diagonal, class).  An even G
+// keeps the colour's column.  kColNodes: rows of a thread at most.
+// Measured on 401 x 201 in 16 CTAs (13 rows each), where every half sweep formed those
+// nodes' constants anew before (cSweepsBatch): solve 0.566 -> 0.536 ms, two rows side by
+// side (four: 0.541, by the registers); the 801 x 401 solve, whose tail it is, 1.815 ->
+// 1.748.  Nine or ten rows a thread spill: 0.566; 17 rows (12 CTAs) stay with the other.
+constexpr int kColNodes = 8;
+// G of a level of nx columns in bands of rows: the threads' columns, an even number;
+// 0: the column does not fit
+__host__ __device__ constexpr int columnGroups(int nx, int rows) {
+  const int G = kClusterThreads / ((nx + 1) / 2) & ~1;
+  return rows <= kColNodes * G ? G : 0;
+}
+template <class MT> struct ColumnNodes {
+  unsigned a0;                     // shared address of the first row's correction
+  MT r[kColNodes], inv[kColNodes]; // inv 0: no node or a Dirichlet one
+  unsigned cls[kColNodes / 4];     // four classes in each
+};
+struct Column {
+  int g, G, R;            // first row, rows apart, the band's rows
+  unsigned row;           // bytes of a row
+  unsigned tab;           // the class table
+  unsigned toS, toN;      // from the first and the last row to their outer neighbours, where
+  bool below, above;      // another CTA has them
+};
+// d's address in row j of the column; rows past the band are its last
+__device__ __forceinline__ unsigned columnAt(const Column &q, unsigned a0, int j, int &ly) {
+  ly = min(q.g + j * q.G, q.R - 1);
+  return a0 + (unsigned)(ly - q.g) * q.row;
+}
+template <bool kRes, class MT>
+__device__ __forceinline__ void cColumnRows(const CLevel<MT> &L, const Column &q,
+                                            const ColumnNodes<MT> &h) {
+  constexpr int U = 2; // rows side by side (kColNodes is a multiple)
+#pragma unroll
+  for (int j0 = 0; j0 < kColNodes; j0 += U) {
+    if (j0 * q.G >= q.R)
+      break;
+    MT f[U][4], d[U][4], e[U][4], rho[U], o[U];
+    unsigned a[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      int ly;
+      a[u] = columnAt(q, h.a0, j0 + u, ly);
+      const unsigned k = q.tab + (h.cls[(j0 + u) / 4] >> 8 * ((j0 + u) & 3) & 0xffu) *
+                                     (unsigned)(8 * sizeof(MT));
+      coefAt(k, f[u]);
+      if (kRes) {
+        coefAt(k + 4u * (unsigned)sizeof(MT), e[u]); // area, diagonal, fixed
+        rho[u] = ldsAt(a[u] + (L.offRho - L.offD), MT());
+        o[u] = ldsAt(a[u], MT());
+      }
+      d[u][0] = ldsAt(a[u] - (unsigned)sizeof(MT), MT());
+      d[u][1] = ldsAt(a[u] + (unsigned)sizeof(MT), MT());
+      // beyond the domain's edge the node's own, with a zero coefficient
+      const bool s = ly == 0, n = ly == q.R - 1;
+      d[u][2] = ldsFar(a[u] + (s ? q.toS : 0u - q.row), true, s && q.below, MT());
+      d[u][3] = ldsFar(a[u] + (n ? q.toN : q.row), true, n && q.above, MT());
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      MT s = kRes ? fma(e[u][0], rho[u], e[u][1]) * o[u] : h.r[j0 + u];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        s = fma(kRes ? -f[u][i] : f[u][i], d[u][i], s);
+      stsIf(a[u] + (kRes ? L.offRes - L.offD : 0u), h.inv[j0 + u] != MT(0),
+            kRes ? h.r[j0 + u] - s : s * h.inv[j0 + u]);
+    }
+  }
+}
+template <class MT>
+__device__ __forceinline__ void columnLoad(const CCtx &c, const CLevel<MT> &L, const NearRows &nd,
+                                           int r0, const Column &q, bool mine, int kx, int colour,
+                                           ColumnNodes<MT> &h) {
+  const int x = 2 * kx + ((r0 + q.g + colour) & 1);
+  const bool on = mine && x < L.nx;
+  h.a0 = nd.base + (unsigned)((q.g * L.nx + (on ? x : 0)) * (int)sizeof(MT));
+#pragma unroll
+  for (int j = 0; j < kColNodes; j++) {
+    if (j % 4 == 0)
+      h.cls[j / 4] = 0;
+    h.r[j] = h.inv[j] = MT(0);
+  }
+#pragma unroll
+  for (int j = 0; j < kColNodes; j++) {
+    if (j * q.G >= q.R)
+      break;
+    int ly;
+    const unsigned a = columnAt(q, h.a0, j, ly);
+    const unsigned cls =
+        *reinterpret_cast<const uint8_t *>(c.smem + (int)L.offCls + ly * L.nx + (on ? x : 0));
+    MT e[4];
+    coefAt(q.tab + (8 * cls + 4) * (unsigned)sizeof(MT), e);
+    h.cls[j / 4] |= cls << 8 * (j & 3);
+    h.r[j] = ldsAt(a + (L.offR - L.offD), MT());
+    if (on && q.g + j * q.G < q.R && e[2] == MT(0))
+      h.inv[j] = mgRcp(fma(e[0], ldsAt(a + (L.offRho - L.offD), MT()), e[1]));
+  }
+}
+template <class MT>
+__device__ __forceinline__ void cSweepsColumn(const CCtx &c, const CLevel<MT> &L, int r0, int R,
+                                              int G, int sweeps, int first, bool residual) {
+  const NearRows nd = nearRows<false>(c, L, L.offD);
+  const int half = (L.nx + 1) / 2, g = L.byHalf.div(threadIdx.x);
+  const bool mine = g < min(G, R);
+  const int kx = mine ? (int)threadIdx.x - g * half : 0;
+  Column q;
+  q.g = mine ? g : 0;
+  q.G = G;
+  q.R = R;
+  q.row = (unsigned)(L.nx * (int)sizeof(MT));
+  q.tab = nd.base - L.offD + L.offTab;
+  q.below = r0 > 0;
+  q.above = r0 + R < L.ny;
+  q.toS = q.below ? nd.below - nd.base : 0u;
+  q.toN = q.above ? nd.above - (nd.base + (unsigned)(R - 1) * q.row) : 0u;
+  ColumnNodes<MT> h[2];
+  columnLoad(c, L, nd, r0, q, mine, kx, first, h[0]);
+  columnLoad(c, L, nd, r0, q, mine, kx, first ^ 1, h[1]);
+#pragma unroll 1
+  for (int s = 0; s < sweeps; s++) {
+    cColumnRows<false>(L, q, h[0]);
+    cSync(L);
+    cColumnRows<false>(L, q, h[1]);
+    cSync(L);
+  }
+  if (residual) {
+    cColumnRows<true>(L, q, h[0]);
+    cColumnRows<true>(L, q, h[1]);
+    cSync(L);
+  }
+}
+
 // `sweeps` red-black sweeps over level L, colour `first` first, then (residual)
 // the residual of the correction equation; every CTA passes the same
 // 2 * sweeps (+ 1) barriers whichever form its rows take
-template <class MT>
+template <bool kCol, class MT>
 __device__ void cSmoothSweeps(const CCtx &c, const CLevel<MT> &Lr, int sweeps, int first,
                               bool residual = false) {
   const CLevel<MT> L = Lr;
@@ -853,6 +989,12 @@ __device__ void cSmoothSweeps(const CCtx &c, const CLevel<MT> &Lr, int sweeps, i
   } else if (L.small) {
     cSweepsBatch<true>(c, L, r0, cnt, sweeps, first, residual);
   } else {
+    if constexpr (kCol) {
+      if (const int G = columnGroups(L.nx, L.rowsPer); G > 0) {
+        cSweepsColumn(c, L, r0, r1 - r0, G, sweeps, first, residual);
+        return;
+      }
+    }
     cSweepsBatch<false>(c, L, r0, cnt, sweeps, first, residual);
   }
 }
@@ -1140,19 +1282,19 @@ __device__ __forceinline__ void cClusterMax2(const CCtx &c, unsigned offRed, dou
 
 // One V-cycle over the descriptor's levels: the distributed levels, then those
 // held by CTA 0, and back up.
-template <class MT>
+template <bool kCol, class MT>
 __device__ __forceinline__ void cVcycle(const CCtx &c, const CMG<MT> &M,
                                         cg::cluster_group &cluster) {
   // the distributed levels down ...
   const int Ls = M.firstSmall;
   for (int l = 0; l < Ls; l++) {
-    cSmoothSweeps(c, M.L[l], M.pre, 0, true);
+    cSmoothSweeps<kCol>(c, M.L[l], M.pre, 0, true);
     cRestrict(c, M.L[l], M.L[l + 1]);
   }
   // ... the levels held by CTA 0 ...
   if (c.rank == 0) {
     for (int l = Ls; l + 1 < M.nLev; l++) {
-      cSmoothSweeps(c, M.L[l], M.pre, 0, true);
+      cSmoothSweeps<kCol>(c, M.L[l], M.pre, 0, true);
       cRestrict(c, M.L[l], M.L[l + 1]);
     }
     cCoarse(c, M.L[M.nLev - 1], M.coarseSweeps);
@@ -1161,14 +1303,14 @@ __device__ __forceinline__ void cVcycle(const CCtx &c, const CMG<MT> &M,
       if (M.L[l + 1].warp && !M.L[l].warp)
         __syncthreads();
       cProlong(c, M.L[l], M.L[l + 1]);
-      cSmoothSweeps(c, M.L[l], M.post, 1);
+      cSmoothSweeps<kCol>(c, M.L[l], M.post, 1);
     }
   }
   cluster.sync();
   // ... and the distributed levels up
   for (int l = Ls - 1; l >= 0; l--) {
     cProlong(c, M.L[l], M.L[l + 1]);
-    cSmoothSweeps(c, M.L[l], M.post, 1);
+    cSmoothSweeps<kCol>(c, M.L[l], M.post, 1);
   }
 }
 
@@ -1179,7 +1321,7 @@ __device__ __forceinline__ void cVcycle(const CCtx &c, const CMG<MT> &M,
 // reaction tailR, tailRho of the descriptor's first level, its correction, from
 // zero, to tailD.  bad (may be NULL): not zero, the level tables are incomplete
 // and nothing is done (out[2] = -1).
-template <class MT, bool kTail>
+template <class MT, bool kTail, bool kCol>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     poissonClusterKernel(CMG<MT> Mp, double *__restrict__ pot, const double *__restrict__ conc,
                          const double *__restrict__ C, const double *__restrict__ gSum,
@@ -1339,7 +1481,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     }
     stageRest();
     cluster.sync();
-    cVcycle(c, M, cluster);
+    cVcycle<kCol>(c, M, cluster);
     for (int t = threadIdx.x; t < nOwn; t += blockDim.x)
       tailD[(size_t)p0 * nx + t] = d0[t];
     cluster.sync(); // no CTA leaves while another may still read its shared memory
@@ -1416,7 +1558,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     // under the update-size rule a Newton step needs only a rough correction
     const int nv = !updRule && bitsBelow(rel, M.twoCycleRel) ? M.vcycles : 1;
     for (int vc = 0; vc < nv; vc++)
-      cVcycle(c, M, cluster);
+      cVcycle<kCol>(c, M, cluster);
     // clamped Newton update of this CTA's rows (updatePotKernel); the cluster
     // barrier makes the new values visible to the neighbours' next residual
     MT updM = 0;
@@ -1589,6 +1731,42 @@ template <class MT> cudaLaunchConfig_t clusterConfig(int CL, size_t bytes, cudaS
   return cfg;
 }
 
+// The kernel of a layout: the one with the column sweeps where a distributed level is
+// too large for the others to hold (float); they would slow every other layout's
+// kernel by their registers (201 x 101: 0.282 -> 0.289 ms).
+template <class MT, bool kTail> auto clusterKernel(const CMG<MT> &M) {
+  if constexpr (sizeof(MT) == 4)
+    for (int l = 0; l < M.firstSmall; l++)
+      if ((M.L[l].nx + 1) / 2 * M.L[l].rowsPer > kSweepNodes * kClusterThreads &&
+          columnGroups(M.L[l].nx, M.L[l].rowsPer) > 0)
+        return poissonClusterKernel<MT, kTail, sizeof(MT) == 4>;
+  return poissonClusterKernel<MT, kTail, false>;
+}
+
+// the device's limits taken by a kernel: *maxDyn the dynamic shared memory it may
+// have, *bigOk clusters above 8 CTAs.  The memory attribute is one per kernel, shared
+// by every hierarchy (engines of other grid sizes), so it is set to the device's
+// limit, not to one layout's size.
+template <class K> bool clusterOptIn(K k, size_t *maxDyn, bool *bigOk) {
+  cudaFuncAttributes fa;
+  int dev = 0, optin = 0;
+  if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+          cudaSuccess ||
+      optin <= (int)fa.sharedSizeBytes ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  *maxDyn = std::min(*maxDyn, (size_t)(optin - (int)fa.sharedSizeBytes));
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    *bigOk = false;
+  }
+  return true;
+}
+
 // Largest cluster (16, 14, 12, 10, 8, 4, 2 or 1 CTAs, at most P.clusterCap
 // when that is set) whose layout fits in shared memory and of which the
 // device can hold `concurrent` at once (solves of engines stepped side by
@@ -1604,26 +1782,13 @@ template <class MT, bool kTail>
 ClusterFit clusterFit(const MGSet &P, int cap, int concurrent) {
   ClusterFit fit;
   const int n = P.L[0].nx * P.L[0].ny;
-  auto k = poissonClusterKernel<MT, kTail>;
-  // the kernel may take all the dynamic shared memory a block can have: the
-  // attribute is one per kernel, shared by every hierarchy (engines of other
-  // grid sizes), so it is set to the device's limit, not to one layout's size
-  cudaFuncAttributes fa;
-  int dev = 0, optin = 0;
-  if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-          cudaSuccess ||
-      optin <= (int)fa.sharedSizeBytes ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           optin - (int)fa.sharedSizeBytes) != cudaSuccess) {
-    cudaGetLastError();
+  size_t maxDyn = kClusterSmemMax;
+  bool bigOk = true;
+  if (!clusterOptIn(poissonClusterKernel<MT, kTail, false>, &maxDyn, &bigOk))
     return fit;
-  }
-  const size_t maxDyn = (size_t)(optin - (int)fa.sharedSizeBytes);
-  const bool bigOk =
-      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  if (!bigOk)
-    cudaGetLastError();
+  if constexpr (sizeof(MT) == 4)
+    if (!clusterOptIn(poissonClusterKernel<MT, kTail, true>, &maxDyn, &bigOk))
+      return fit;
   const int cands[] = {16, 14, 12, 10, 8, 4, 2, 1};
   for (int CL : cands) {
     if (cap > 0 && CL > cap)
@@ -1639,17 +1804,17 @@ ClusterFit clusterFit(const MGSet &P, int cap, int concurrent) {
     };
     size_t bytes = 0;
     bool even = true;
-    clusterDesc<MT>(P, CL, &bytes, true);
+    CMG<MT> M = clusterDesc<MT>(P, CL, &bytes, true);
     if (!fits(bytes)) {
       even = false;
-      clusterDesc<MT>(P, CL, &bytes, false);
+      M = clusterDesc<MT>(P, CL, &bytes, false);
       if (!fits(bytes))
         continue;
     }
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = clusterConfig<MT>(CL, bytes, nullptr, &at);
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, k, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&nc, clusterKernel<MT, kTail>(M), &cfg) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -1736,7 +1901,7 @@ void vcycle(const MGSet &P, int l, const MGTail &tail, cudaStream_t st) {
     const CMG<MT> M = clusterDesc<MT>(T, tail.size, &bytes, tail.even);
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = clusterConfig<MT>(tail.size, bytes, st, &at);
-    cudaLaunchKernelEx(&cfg, poissonClusterKernel<MT, true>, M, (double *)nullptr,
+    cudaLaunchKernelEx(&cfg, clusterKernel<MT, true>(M), M, (double *)nullptr,
                        (const double *)nullptr, (const double *)nullptr, (const double *)nullptr,
                        (const double *)nullptr, 0., 0., 0., 0., 0, 0., (const double *)nullptr,
                        (double *)nullptr, (const MT *)K.r, (const MT *)K.rho, K.d,
@@ -2021,7 +2186,7 @@ static int32_t clusterLaunch(PoissonMG &P, double *pot, const double *conc, doub
   const CMG<MT> M = clusterDesc<MT>(mgSet(P), P.clusterSize, &bytes, P.clusterEven);
   cudaLaunchAttribute at;
   cudaLaunchConfig_t cfg = clusterConfig<MT>(P.clusterSize, bytes, st, &at);
-  EMCG_CUDA(cudaLaunchKernelEx(&cfg, poissonClusterKernel<MT, false>, M, pot, conc,
+  EMCG_CUDA(cudaLaunchKernelEx(&cfg, clusterKernel<MT, false>(M), M, pot, conc,
                                (const double *)P.C, (const double *)P.gSum,
                                (const double *)(conc ? P.gVne : P.gVeq), P.hF[0], P.hF[1], P.hP,
                                rtol, maxCycles, P.updTol, (const double *)P.expTab, out,
@@ -2657,7 +2822,7 @@ extern "C" int32_t emcg_poisson_solve_noalloc(const emcg_device_desc *dv, double
     const CMG<float> M = clusterDesc<float>(mg, fit.size, &bytes, fit.even);
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = clusterConfig<float>(fit.size, bytes, st, &at);
-    EMCG_CUDA(cudaLaunchKernelEx(&cfg, poissonClusterKernel<float, false>, M, d_pot, d_conc,
+    EMCG_CUDA(cudaLaunchKernelEx(&cfg, clusterKernel<float, false>(M), M, d_pot, d_conc,
                                  (const double *)C, (const double *)gSum,
                                  (const double *)(d_conc ? gVne : gVeq), hF0, hF1, hP, rtol,
                                  (int)max_cycles, 0., (const double *)expT, stats,
