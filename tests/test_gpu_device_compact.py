@@ -51,3 +51,29 @@ def test_fused_step_equals_its_stages(engine, scheme, capacity, precision):
         assert np.array_equal(getattr(sa, f), getattr(sb, f)), f
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx", [5, 512, 513])
+def test_injection_fills_every_reservoir_node(engine, nx, precision):
+    """Up to 1024 reservoir nodes every block of the injection forms the nodes' numbers
+    itself, beyond one block does so first: after a step each contact node holds its
+    expected number of carriers, rounded up (nearest-node charge)."""
+    from viennaemc_gb300 import _lib as L
+    from viennaemc_gb300 import device as D
+    from viennaemc_gb300.physics import silicon_material
+    h, ny = 1e-9, 6
+    dev = D.Device(silicon_material(), ((nx - 1) * h, (ny - 1) * h), (h, h))
+    dev.setDeviceWidth(6.7e-7)  # 6.7 electrons a cell, 3.35 at a contact node
+    dev.addConstantDopingRegion((0, 0), ((nx - 1) * h, (ny - 1) * h), 1e25)
+    dev.addOhmicContact(D.YMIN, 0.0, (0,), ((nx - 1) * h,))
+    dev.addOhmicContact(D.YMAX, 0.05, (0,), ((nx - 1) * h,))
+    pt = engine.physics.silicon_electron("refbulk", n_levels=500, max_energy=4.0)
+    sim = D.DeviceSimulation(dev, pt, scheme=D.NGP, dt=1e-16, seed=9, precision=precision)
+    sim.calcEquilibriumCharacteristics()
+    n0 = sim.num_particles()
+    netto = sim.performEMCStep(3)
+    assert sim.num_particles() == n0 - int(netto.sum())
+    held = sim.get_grid(L.GRID_NRPART).reshape(ny, nx)
+    assert np.all(held[[0, -1], 1:-1] == 4.0)
+    sim.close()

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "emcg_common.cuh"
+#include "emcg_exp.h"
 #include "emcg_host.h"
 #include "emcg_model.h"
 #include "emcg_poisson.cuh"
@@ -28,7 +29,7 @@ constexpr int kCB = 1024; // compaction block
 struct DevK {
   int nx, ny;
   double hx, hy, invhx, invhy, maxX, maxY;
-  double Vt, Ni, cellVol;
+  double Vt;
   const int32_t *region;      // doping region per node
   const int32_t *nodeContact; // getContactIdx (first boundary), -1 if none
   const uint8_t *nodeOhmic;   // isOhmicContact (first boundary)
@@ -855,12 +856,12 @@ __global__ void contactRankKernel(const int32_t *__restrict__ gList,
   }
 }
 
-// particles to inject per reservoir node (emcAbstractParticleHandler.hpp:200-216),
-// as the sum of those at the nodes before it; *total: all (one block)
-__global__ void __launch_bounds__(1024)
-    injectCountKernel(const int32_t *__restrict__ resNodes, int nRes,
-                      const double *__restrict__ expNr, const int32_t *__restrict__ kept,
-                      double nrC, int32_t *__restrict__ injBase, int64_t *__restrict__ total) {
+// Particles to inject per reservoir node (emcAbstractParticleHandler.hpp:200-216), as
+// the sum of those at the nodes before it; the number of all of them (one block).
+__device__ __forceinline__ int64_t injectCounts(const int32_t *__restrict__ resNodes, int nRes,
+                                                const double *__restrict__ expNr,
+                                                const int32_t *__restrict__ kept, double nrC,
+                                                int32_t *injBase) {
   int64_t carry = 0;
   for (int base = 0; base < nRes; base += blockDim.x) {
     const int r = base + threadIdx.x;
@@ -879,8 +880,15 @@ __global__ void __launch_bounds__(1024)
       injBase[r] = (int32_t)(carry + ex);
     carry += tot;
   }
+  return carry;
+}
+__global__ void __launch_bounds__(1024)
+    injectCountKernel(const int32_t *__restrict__ resNodes, int nRes,
+                      const double *__restrict__ expNr, const int32_t *__restrict__ kept,
+                      double nrC, int32_t *__restrict__ injBase, int64_t *__restrict__ total) {
+  const int64_t all = injectCounts(resNodes, nRes, expNr, kept, nrC, injBase);
   if (threadIdx.x == 0)
-    *total = carry;
+    *total = all;
 }
 
 // emcElectron::generateInjectedParticle + initParticlePos (2-D)
@@ -914,19 +922,35 @@ __device__ __forceinline__ void initParticle2D(const ModelK<T> &M, const DevK &G
   gtau = -drawLog(M, rng.ulog()) * M.grainTau;
 }
 
-// (behind the *nBase particles that stay; the new number to *nPtr.  SCHEME >= 0:
+// reservoir nodes up to which every block of the injection forms the nodes' numbers
+// itself, in shared memory; beyond, one block forms them first (injectCountKernel).
+// With 202 nodes 4.4 us of that kernel and its launch against 1 to 2 us in this one.
+constexpr int kInjNodes = 1024;
+
+// (expNr: as injectCountKernel, in the kernel itself, else NULL;
+// behind the *nBase particles that stay; the new number to *nPtr.  SCHEME >= 0:
 // the injected ones' charge is assigned too)
 template <class T, bool REPLAY, int SCHEME>
 __global__ void injectKernel(StateK<T> st, const ModelK<T> *__restrict__ models, DevK G,
                              const int32_t *__restrict__ resNodes, int nRes,
-                             const int32_t *__restrict__ injBase, const int64_t *__restrict__ injTotal,
+                             const int32_t *__restrict__ injBaseIn,
+                             const int64_t *__restrict__ injTotal,
+                             const double *__restrict__ expNr, const int32_t *__restrict__ kept,
                              const int64_t *__restrict__ nBase, int64_t *__restrict__ nPtr,
                              int64_t capacity, uint32_t step,
                              uint32_t key0, uint32_t key1, uint32_t stream, bool tauRegionIsValley,
                              int32_t *__restrict__ remInj, const uint64_t *__restrict__ rw,
                              const int64_t *__restrict__ roff, int *__restrict__ err, double nrC,
                              int fixBits, unsigned long long *__restrict__ fix) {
-  const int64_t total = *injTotal;
+  __shared__ int32_t sBase[kInjNodes];
+  int64_t total;
+  if (expNr) {
+    total = injectCounts(resNodes, nRes, expNr, kept, nrC, sBase);
+    __syncthreads();
+  } else {
+    total = *injTotal;
+  }
+  const int32_t *injBase = expNr ? sBase : injBaseIn;
   const int64_t n = *nBase;
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j == 0)
@@ -1016,17 +1040,25 @@ struct StepOut {
 };
 // the fixed-point sums as particle counts, and the concentration
 // (include/emcSimulationResults.hpp:98-116)
-__global__ void concKernel(DevK G, const unsigned long long *__restrict__ fix, int fixBits,
-                           double *__restrict__ nr, double *__restrict__ conc, StepOut out) {
+// (lo, hi: the value of the two words' lowest bits; scale = 1 / (Ni cell volume).  Bound
+// by its double-precision instructions: 2 or 3 a node instead of two divisions and two
+// scalings, 401 x 201 10.2 -> 4.3 us)
+__global__ void concKernel(DevK G, const unsigned long long *__restrict__ fix, double lo, double hi,
+                           double scale, double *__restrict__ nr, double *__restrict__ conc,
+                           StepOut out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (out.host)
     for (int j = i; j <= out.nc; j += gridDim.x * blockDim.x)
       out.host[j] = j < out.nc ? out.netto[j] - out.remInj[j] : *out.err;
   if (i >= G.nx * G.ny)
     return;
-  nr[i] = ldexp((double)fix[2 * i + 1], 64 - fixBits) + ldexp((double)fix[2 * i], -fixBits);
+  const ulonglong2 w = reinterpret_cast<const ulonglong2 *>(fix)[i];
+  double n = (double)w.x * lo;
+  if (w.y) // (never in the float engine, whose sums have 64 bits)
+    n = fma((double)w.y, hi, n);
+  nr[i] = n;
   int x = i % G.nx, y = i / G.nx;
-  double c = nr[i] / G.Ni * (1. / G.cellVol);
+  double c = n * scale;
   if (x == 0 || x == G.nx - 1)
     c *= 2;
   if (y == 0 || y == G.ny - 1)
@@ -1048,9 +1080,13 @@ struct StepZero {
 // values of :58-81 (0 normal to an artificial boundary, else the neighbour).
 // NEC-VWD (examples/mosfet2D/NECSchemeVWD.hpp, calcEField): forward
 // differences, 0 on the last edge, no boundary pass.
+// perX, perY: thermal voltage over the differences' distance (a division per node and
+// component before: bound by double-precision instructions, 401 x 201 10.7 -> 4.6 us).
+__device__ __forceinline__ float fieldOf(double v, float) { return toFloat(v); }
+__device__ __forceinline__ double fieldOf(double v, double) { return v; }
 template <class T>
 __global__ void efieldKernel(DevK G, const double *__restrict__ pot, T *__restrict__ Ex,
-                             T *__restrict__ Ey, int scheme, StepZero z) {
+                             T *__restrict__ Ey, int scheme, double perX, double perY, StepZero z) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (z.kept)
     for (int j = i; j < max(z.nDrop, z.nc); j += gridDim.x * blockDim.x) {
@@ -1067,36 +1103,22 @@ __global__ void efieldKernel(DevK G, const double *__restrict__ pot, T *__restri
   }
   const int nx = G.nx, ny = G.ny, x = i % nx, y = i / nx;
   const bool edges = scheme == EMCG_PM_NEC || scheme == EMCG_PM_NEC_VWD;
-  auto ex = [&](int xi) {
-    int j = y * nx + xi;
-    return edges ? (pot[j] - pot[j + 1]) * G.Vt / G.hx
-                 : (pot[j - 1] - pot[j + 1]) * G.Vt / (2 * G.hx);
-  };
-  auto ey = [&](int yi) {
-    int j = yi * nx + x;
-    return edges ? (pot[j] - pot[j + nx]) * G.Vt / G.hy
-                 : (pot[j - nx] - pot[j + nx]) * G.Vt / (2 * G.hy);
-  };
-  if (scheme == EMCG_PM_NEC_VWD) {
-    Ex[i] = (T)(x != nx - 1 ? ex(x) : 0.);
-    Ey[i] = (T)(y != ny - 1 ? ey(y) : 0.);
-    return;
-  }
-  double vx, vy;
-  if (x != 0 && x != nx - 1)
-    vx = ex(x);
-  else if (x == 0)
-    vx = G.bnd[0][y] == -1 ? 0. : ex(1);
-  else
-    vx = G.bnd[1][y] == -1 ? 0. : ex(nx - 2);
-  if (y != 0 && y != ny - 1)
-    vy = ey(y);
-  else if (y == 0)
-    vy = G.bnd[2][x] == -1 ? 0. : ey(1);
-  else
-    vy = G.bnd[3][x] == -1 ? 0. : ey(ny - 2);
-  Ex[i] = (T)vx;
-  Ey[i] = (T)vy;
+  const bool vwd = scheme == EMCG_PM_NEC_VWD;
+  // the node whose difference the field here is, and whether it is zero
+  const int xi = vwd ? x : x == 0 ? 1 : x == nx - 1 ? nx - 2 : x;
+  const int yi = vwd ? y : y == 0 ? 1 : y == ny - 1 ? ny - 2 : y;
+  const bool zeroX = vwd ? x == nx - 1
+                         : (x == 0 && G.bnd[0][y] == -1) || (x == nx - 1 && G.bnd[1][y] == -1);
+  const bool zeroY = vwd ? y == ny - 1
+                         : (y == 0 && G.bnd[2][x] == -1) || (y == ny - 1 && G.bnd[3][x] == -1);
+  const int jx = y * nx + xi, jy = yi * nx + x;
+  T vx = T(0), vy = T(0);
+  if (!zeroX)
+    vx = fieldOf((pot[edges ? jx : jx - 1] - pot[jx + 1]) * perX, T());
+  if (!zeroY)
+    vy = fieldOf((pot[edges ? jy : jy - nx] - pot[jy + nx]) * perY, T());
+  Ex[i] = vx;
+  Ey[i] = vy;
 }
 
 // ---------------------------------------------------------------------------
@@ -1171,8 +1193,6 @@ static DevK devK(const DeviceImpl *d) {
   G.maxX = d->maxX;
   G.maxY = d->maxY;
   G.Vt = d->Vt;
-  G.Ni = d->Ni;
-  G.cellVol = d->cellVol;
   G.region = d->dRegion;
   G.nodeContact = d->dNodeContact;
   G.nodeOhmic = d->dNodeOhmic;
@@ -1565,8 +1585,11 @@ namespace emcg {
 
 template <class T> static int32_t efieldT(DeviceImpl *d, const StepZero &zero = StepZero{}) {
   const int n = d->nx * d->ny;
-  efieldKernel<T><<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dPot, (T *)d->dEx,
-                                                          (T *)d->dEy, d->cfg.pm_scheme, zero);
+  const bool edges = d->cfg.pm_scheme == EMCG_PM_NEC || d->cfg.pm_scheme == EMCG_PM_NEC_VWD;
+  const double span = edges ? 1. : 2.;
+  efieldKernel<T><<<(n + 255) / 256, 256, 0, d->stream>>>(
+      devK(d), d->dPot, (T *)d->dEx, (T *)d->dEy, d->cfg.pm_scheme, d->Vt / (span * d->hx),
+      d->Vt / (span * d->hy), zero);
   EMCG_CUDA(cudaGetLastError());
   return EMCG_OK;
 }
@@ -1724,8 +1747,10 @@ template <class T> static int32_t contactsT(DeviceImpl *d, uint32_t step, bool m
   EMCG_TRY(compactT<T>(d, movedDrops));
   if (nRes == 0)
     return keepCount(d);
-  injectCountKernel<<<1, 1024, 0, st>>>(d->dResNodes, nRes, d->dExp, d->dKept,
-                                        d->cfg.carriers_per_particle, d->dInjCount, d->dN + 2);
+  const bool inBlock = nRes <= kInjNodes;
+  if (!inBlock)
+    injectCountKernel<<<1, 1024, 0, st>>>(d->dResNodes, nRes, d->dExp, d->dKept,
+                                          d->cfg.carriers_per_particle, d->dInjCount, d->dN + 2);
   const emcg_device_config &c = d->cfg;
   uint32_t k0 = (uint32_t)c.seed, k1 = (uint32_t)(c.seed >> 32);
   const int ib = (int)((d->injBound + 255) / 256);
@@ -1735,7 +1760,8 @@ template <class T> static int32_t contactsT(DeviceImpl *d, uint32_t step, bool m
     if (rep)
       k = injectOf<T, true>(d, movedDrops);
   k<<<ib, 256, 0, st>>>(devState<T>(d, d->cur), (const ModelK<T> *)d->dModel, G, d->dResNodes, nRes,
-                        d->dInjCount, d->dN + 2, d->dN + 1, d->dN, d->capacity, step, k0, k1,
+                        d->dInjCount, d->dN + 2, inBlock ? d->dExp : nullptr, d->dKept, d->dN + 1,
+                        d->dN, d->capacity, step, k0, k1,
                         c.stream, c.tau_region_is_valley != 0, d->dRemInj,
                         rep ? d->dWords[1] : nullptr, rep ? d->dOff[1] : nullptr, d->dErr,
                         c.carriers_per_particle, fixBitsOf(d), d->dNodeFix);
@@ -1747,8 +1773,10 @@ template <class T> static int32_t contactsT(DeviceImpl *d, uint32_t step, bool m
 // the concentration from the charge sums; out: a step's outcome to the host
 static int32_t concentration(DeviceImpl *d, const StepOut &out = StepOut{}) {
   const int n = d->nx * d->ny;
-  concKernel<<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dNodeFix, fixBitsOf(d), d->dNr,
-                                                     d->dConc, out);
+  const double lo = std::ldexp(1., -fixBitsOf(d)), hi = std::ldexp(1., 64 - fixBitsOf(d));
+  concKernel<<<(n + 255) / 256, 256, 0, d->stream>>>(devK(d), d->dNodeFix, lo, hi,
+                                                     1. / (d->Ni * d->cellVol), d->dNr, d->dConc,
+                                                     out);
   EMCG_CUDA(cudaGetLastError());
   return EMCG_OK;
 }
