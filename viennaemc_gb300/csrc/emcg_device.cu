@@ -602,6 +602,15 @@ __device__ __forceinline__ void fixAdd(const DevK &G, unsigned long long *fix, i
   if (hi)
     atomicAdd(p + 1, hi);
 }
+// The float engine's sums stay below 2^62: the low word alone, and no value comes
+// back from the memory to wait for (the carry's test needs it).  Compaction with
+// assignment, 390k electrons: 25.4 -> 22.4 us, 500k 29.2 -> 25.2.
+__device__ __forceinline__ void fixAdd64(const DevK &G, unsigned long long *fix, int x, int y,
+                                         unsigned long long v) {
+  if (x < 0 || y < 0 || x >= G.nx || y >= G.ny || v == 0)
+    return;
+  atomicAdd(fix + 2 * ((size_t)y * G.nx + x), v);
+}
 // one particle at (px, py) to the nodes around it
 template <class T, int SCHEME>
 __device__ __forceinline__ void assignParticle(const DevK &G, T px, T py, double nrC, int fixBits,
@@ -613,7 +622,7 @@ __device__ __forceinline__ void assignParticle(const DevK &G, T px, T py, double
     if (SCHEME == EMCG_PM_NGP) {
       mx = roundIdx<float>(px, G.hx, G.invhx);
       my = roundIdx<float>(py, G.hy, G.invhy);
-      fixAdd(G, fix, mx, my, __float2ull_rn(s), 0ull);
+      fixAdd64(G, fix, mx, my, __float2ull_rn(s));
       return;
     } else if (SCHEME == EMCG_PM_CIC) {
       const float wX = floorDiv<float>(px, G.hx, G.invhx, mx);
@@ -627,10 +636,10 @@ __device__ __forceinline__ void assignParticle(const DevK &G, T px, T py, double
       floorDiv<float>(py, G.hy, G.invhy, my);
       v[0] = v[1] = v[2] = v[3] = __float2ull_rn(0.25f * s);
     }
-    fixAdd(G, fix, mx, my, v[0], 0ull);
-    fixAdd(G, fix, mx + 1, my, v[1], 0ull);
-    fixAdd(G, fix, mx, my + 1, v[2], 0ull);
-    fixAdd(G, fix, mx + 1, my + 1, v[3], 0ull);
+    fixAdd64(G, fix, mx, my, v[0]);
+    fixAdd64(G, fix, mx + 1, my, v[1]);
+    fixAdd64(G, fix, mx, my + 1, v[2]);
+    fixAdd64(G, fix, mx + 1, my + 1, v[3]);
   } else {
     double w[4];
     if (SCHEME == EMCG_PM_NGP) {
