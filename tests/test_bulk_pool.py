@@ -93,27 +93,3 @@ def test_pooled_kernel_equals_queued_kernel(engine, model, counts):
         if model != "grain" and n:
             assert np.allclose(oa[:, :, 2], oq[:, :, 2], atol=2)
             assert np.allclose(oa.sum(axis=1)[:, 0], oq.sum(axis=1)[:, 0], rtol=1e-4)
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("dt_over_tau,short,long", [(0.05, 5, 6), (0.19, 5, 6), (0.21, 3, 4),
-                                                    (0.34, 3, 4), (0.36, 3, 3), (0.9, 3, 3)])
-def test_default_pass_actions_follow_the_event_rate(engine, dt_over_tau, short, long):
-    """The float kernel's flights per pass by launch length and events a step; the
-    electrons are those of any other choice, bit for bit."""
-    pt = engine.silicon_electron("jacoboni")
-    dt = dt_over_tau * pt.model_desc().tablesets[0].tau_max
-    out = []
-    for actions in (0, 1, 6):
-        b = engine.BulkBatch([pt], [engine.EnsembleSpec(0, 1000, 1e6, (1, 0, 0), (1e-6,) * 3, dt,
-                                                        7)], "fp32")
-        b.set_launch(queued=2, pass_actions=actions)
-        b.init_particles(0)
-        for steps, want in ((20, short), (100, long)):
-            b.step(steps)
-            assert b.pass_actions() == (actions or want)
-        out.append(b.get_state(0))
-        b.close()
-    for f in ("kx", "ky", "kz", "energy", "px", "py", "pz", "tau", "valley", "sub"):
-        assert np.array_equal(getattr(out[0], f), getattr(out[1], f)), f
-        assert np.array_equal(getattr(out[0], f), getattr(out[2], f)), f

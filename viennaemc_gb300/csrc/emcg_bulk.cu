@@ -685,21 +685,6 @@ constexpr int kPassActions = 6;
 // 0.3155 / 0.3159 / 0.3171, 5 0.3116 / 0.3108 / 0.3149, 6 0.3133 / 0.3128 /
 // 0.3170, 8 0.3256 / 0.3236 / 0.3278
 constexpr int kPassActionsShort = 5;
-// Fewer where events are frequent: after n flights with an event at the end of a
-// share p of them only (1 - p)^n of the lanes still fly, the rest wait for the pass
-// to end.  events: events a step (dt over the free-flight constant).  Measured on
-// 2^20 electrons, 20 / 500 steps a launch, ms at 2, 3, 4, 5, 6 flights:
-//   events 0.095  0.342 0.311 0.302 0.301 0.305 / 7.12 6.17 5.81 5.63 5.59
-//          0.158  0.374 0.346 0.343 0.346 0.355 / 7.68 6.77 6.49 6.42 6.49
-//          0.236  0.411 0.387 0.389 0.402 0.414 / 8.34 7.50 7.31 7.37 7.57
-//          0.277  0.415 0.393 0.397 0.410 0.429 / 8.32 7.52 7.40 7.54 7.83
-//          0.433  0.499 0.485 0.502 0.524 0.549 / 9.94 9.30 9.41 9.79 10.26
-//          0.531  0.550 0.543 0.567 0.597 0.621 / 11.06 10.53 10.78 11.29 11.82
-// and the same order on 1e5 electrons.  The kernel's results do not depend on it.
-constexpr int passActionsFor(bool shortLaunch, double events) {
-  const int most = shortLaunch ? kPassActionsShort : kPassActions;
-  return events < 0.2 ? most : events < 0.35 ? most - 2 : 3;
-}
 // fixed-point scales of a warp's step sums: energy 2^-20 eV, velocity
 // 0.25 m/s per unit; below kFixMax per lane, 32 lanes stay within int32
 constexpr float kFixE = 1048576.f;
@@ -1053,7 +1038,6 @@ struct BulkImpl {
   int64_t totalCap = 0;
   void *dModels = nullptr;
   std::vector<void *> dTables;
-  std::vector<double> modelTau;  // shortest free-flight constant per model, as created
   std::vector<RateLayout> rates; // table layout per model (rate-table rebuild)
   RateScratch rateScratch;        // device scratch of rebuilds
   double *dLogTab = nullptr;      // logTab()'s table (double engine)
@@ -1180,31 +1164,18 @@ static void buildEnsK(const emcg_ensemble_desc &d, const ModelK<T> &M,
   (void)M;
 }
 
-static double shortestTau(const emcg_model_desc &m) {
-  double tau = 2e-15;
-  bool any = false;
-  for (int t = 0; t < m.n_tablesets; t++)
-    if (m.tablesets[t].n_tables > 0) {
-      tau = any ? std::min(tau, m.tablesets[t].tau_max) : m.tablesets[t].tau_max;
-      any = true;
-    }
-  return tau;
-}
-
 template <class T>
 static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nModels,
                            const emcg_ensemble_desc *ens, int nEns) {
   std::vector<ModelK<T>> mk(nModels);
   b->dTables.assign(nModels, nullptr);
   b->rates.resize(nModels);
-  b->modelTau.resize(nModels);
   for (int i = 0; i < nModels; i++) {
     std::vector<T> tab;
     EMCG_TRY(buildModelK<T>(models[i], mk[i], tab));
     if (sizeof(T) == 8 && !b->dLogTab) // (after a model's own checks)
       EMCG_TRY(uploadLogTable(&b->dLogTab));
     b->rates[i] = rateLayoutOf(models[i]);
-    b->modelTau[i] = shortestTau(models[i]);
     EMCG_CUDA(cudaMalloc(&b->dTables[i], tab.size() * sizeof(T)));
     EMCG_CUDA(cudaMemcpy(b->dTables[i], tab.data(), tab.size() * sizeof(T),
                          cudaMemcpyHostToDevice));
@@ -1604,18 +1575,6 @@ static int32_t launchStepTiles(BulkImpl *b, const StateK<T> &st, int ns, uint32_
   return EMCG_OK;
 }
 
-// events of an electron and step, over the batch's electrons (each model's shortest
-// free-flight constant; 2e-15 s without tables, as tauOf)
-static double eventsPerStep(const BulkImpl *b) {
-  double sum = 0, n = 0;
-  for (int e = 0; e < b->nEns; e++) {
-    const emcg_ensemble_desc &d = b->ens[e];
-    sum += (double)b->count[e] * d.dt / b->modelTau[d.model];
-    n += (double)b->count[e];
-  }
-  return n > 0 ? sum / n : 0.;
-}
-
 // src/srcEns: the first launch reads ensemble srcEns's start state from src
 // (the warp-asynchronous kernel only; nullptr: the device state)
 template <class T>
@@ -1634,7 +1593,7 @@ static int32_t stepTyped(BulkImpl *b, int nSteps, uint32_t step0, double *obsHos
   }
   if (b->passAuto) {
     const int first = std::min(b->stepsPerLaunch > 0 ? b->stepsPerLaunch : nSteps, nSteps);
-    b->passActions = passActionsFor(first < kShortLaunchSteps, eventsPerStep(b));
+    b->passActions = first < kShortLaunchSteps ? kPassActionsShort : kPassActions;
   }
   // the double engine's mode 0: pools
   const bool pooled = b->queued == 0 && sizeof(T) == 8 && !b->replay;
