@@ -35,11 +35,10 @@ template <class T> struct ValleyK {
   T cX;                   // hbar / mc: velocity and displacement factor
   T cF[3];                // vogt_i / hbar: dk_ecs = F_ecs cF dt
   int32_t deg;
-  int32_t pad_;
-  // rot as a permutation where its entries are 0 and +-1 (kNoPerm: they are
+  // (double) rot as a permutation where its entries are 0 and +-1 (kNoPerm: they are
   // not): for i = 0..2, bits 4 i .. 4 i + 1 the column of row i's entry, bit
   // 4 i + 2 its sign; bits 16 + 4 i .. the same of the transpose
-  uint32_t perm[EMCG_MAX_DEG];
+  uint32_t perm[sizeof(T) == 8 ? EMCG_MAX_DEG : 1];
 };
 constexpr uint32_t kNoPerm = 0xffffffffu;
 

@@ -174,7 +174,8 @@ int32_t buildModelK(const emcg_model_desc &m, ModelK<T> &K, std::vector<T> &tabl
     for (int s = 0; s < V.deg; s++) {
       for (int i = 0; i < 9; i++)
         O.rot[s][i] = (T)V.rot[s][i];
-      O.perm[s] = permOf(V.rot[s]);
+      if (sizeof(T) == 8)
+        O.perm[s] = permOf(V.rot[s]);
     }
     for (int i = 0; i < 3; i++) {
       O.vogt[i] = (T)d.vogt[i];
