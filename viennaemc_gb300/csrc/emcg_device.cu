@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
 // launches, the compaction and the injection assign the charge of the particles
 // that they place, the first kernel clears the step's counters, and the last one
 // writes the outcome into page-locked memory.  10 nodes a step on the stream
-// instead of 24; resistor 201 x 101, 500k electrons FP32: 0.502 -> 0.444 ms a step,
+// instead of 24 (9 since the injection forms its own numbers); resistor 201 x 101, 500k electrons FP32: 0.502 -> 0.444 ms a step,
 // 101 x 51, 50k electrons FP64 0.394 -> 0.329, 8 MOSFETs of 401 x 201 at once 7.6 -> 6.8 ms per 5.
 __device__ __forceinline__ int blockExclusiveScan(int v, int *total) {
   __shared__ int warpSums[32];
