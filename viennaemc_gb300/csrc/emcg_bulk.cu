@@ -1193,6 +1193,17 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
   return EMCG_OK;
 }
 
+static void dropGraph(BulkImpl *b) {
+  if (b->gexec)
+    cudaGraphExecDestroy(b->gexec);
+  if (b->graph)
+    cudaGraphDestroy(b->graph);
+  b->gexec = nullptr;
+  b->graph = nullptr;
+  b->gKernel = nullptr;
+  b->gNs = -1;
+}
+
 // The tiles of the step kernels: thread blocks of b->blockThreads electrons,
 // or (pool > 0) pools of at most pool electrons, those of an ensemble alike in
 // size.
@@ -1212,11 +1223,14 @@ static int32_t ensureTiles(BulkImpl *b, int pool = 0) {
       t.push_back(x);
     }
   }
+  b->tilesDirty = true; // until the list is in place
   if ((int)t.size() > b->tilesCap) {
+    dropGraph(b); // it holds the old buffer
     cudaFree(b->dTiles);
     b->dTiles = nullptr;
-    b->tilesCap = std::max<int>((int)t.size(), 1);
-    EMCG_CUDA(cudaMalloc(&b->dTiles, sizeof(Tile) * b->tilesCap));
+    b->tilesCap = 0;
+    EMCG_CUDA(cudaMalloc(&b->dTiles, sizeof(Tile) * t.size()));
+    b->tilesCap = (int)t.size();
   }
   if (!t.empty())
     EMCG_CUDA(cudaMemcpyAsync(b->dTiles, t.data(), sizeof(Tile) * t.size(),
@@ -1244,17 +1258,6 @@ static int32_t readError(BulkImpl *b) {
   EMCG_CUDA(cudaMemcpyAsync(b->hErr, b->dErr, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   EMCG_CUDA(cudaStreamSynchronize(b->stream));
   return takeError(b);
-}
-
-static void dropGraph(BulkImpl *b) {
-  if (b->gexec)
-    cudaGraphExecDestroy(b->gexec);
-  if (b->graph)
-    cudaGraphDestroy(b->graph);
-  b->gexec = nullptr;
-  b->graph = nullptr;
-  b->gKernel = nullptr;
-  b->gNs = -1;
 }
 
 // The observable buffers (device sums and their page-locked readback) for at
