@@ -1173,23 +1173,23 @@ static int32_t createTyped(BulkImpl *b, const emcg_model_desc *models, int nMode
   for (int i = 0; i < nModels; i++) {
     std::vector<T> tab;
     EMCG_TRY(buildModelK<T>(models[i], mk[i], tab));
-    if (sizeof(T) == 8 && !b->dLogTab) // (after a model's own checks)
-      EMCG_TRY(uploadLogTable(&b->dLogTab));
+    if (!b->stream) // (after a model's own checks)
+      EMCG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+    if (sizeof(T) == 8 && !b->dLogTab)
+      EMCG_TRY(uploadLogTable(&b->dLogTab, b->stream));
     b->rates[i] = rateLayoutOf(models[i]);
     EMCG_CUDA(cudaMalloc(&b->dTables[i], tab.size() * sizeof(T)));
-    EMCG_CUDA(cudaMemcpy(b->dTables[i], tab.data(), tab.size() * sizeof(T),
-                         cudaMemcpyHostToDevice));
+    EMCG_CUDA(copyToDevice(b->dTables[i], tab.data(), tab.size() * sizeof(T), b->stream));
     mk[i].tables = (const T *)b->dTables[i];
     mk[i].logT = b->dLogTab;
   }
   EMCG_CUDA(cudaMalloc(&b->dModels, sizeof(ModelK<T>) * nModels));
-  EMCG_CUDA(cudaMemcpy(b->dModels, mk.data(), sizeof(ModelK<T>) * nModels,
-                       cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(b->dModels, mk.data(), sizeof(ModelK<T>) * nModels, b->stream));
   std::vector<EnsK<T>> ek(nEns);
   for (int e = 0; e < nEns; e++)
     buildEnsK<T>(ens[e], mk[ens[e].model], models[ens[e].model], b->begin[e], 0, ek[e]);
   EMCG_CUDA(cudaMalloc(&b->dEns, sizeof(EnsK<T>) * nEns));
-  EMCG_CUDA(cudaMemcpy(b->dEns, ek.data(), sizeof(EnsK<T>) * nEns, cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(b->dEns, ek.data(), sizeof(EnsK<T>) * nEns, b->stream));
   return EMCG_OK;
 }
 
@@ -1811,9 +1811,8 @@ extern "C" int32_t emcg_bulk_create(const emcg_model_desc *models, int32_t n_mod
     }
   if (cudaMalloc(&b->dMeta, n * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&b->dErr, sizeof(int)) != cudaSuccess ||
-      cudaMemset(b->dErr, 0, sizeof(int)) != cudaSuccess ||
+      cudaMemsetAsync(b->dErr, 0, sizeof(int), b->stream) != cudaSuccess ||
       cudaHostAlloc(&b->hErr, sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
     setError("CUDA allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
     return fail(EMCG_ERR_CUDA);
@@ -2162,7 +2161,7 @@ extern "C" int32_t emcg_bulk_init(emcg_handle *h, int32_t e, int64_t n, const in
       EMCG_CHECK_ARG(coords[i] >= 0 && coords[i] < ext[i % 3], "coordinate out of the grid");
     if (n) {
       EMCG_CUDA(cudaMalloc(&dC, sizeof(int64_t) * 3 * n));
-      EMCG_CUDA(cudaMemcpy(dC, coords, sizeof(int64_t) * 3 * n, cudaMemcpyHostToDevice));
+      EMCG_CUDA(copyToDevice(dC, coords, sizeof(int64_t) * 3 * n, b->stream));
     }
   }
   const emcg_ensemble_desc &d = b->ens[e];
@@ -2233,8 +2232,8 @@ extern "C" int32_t emcg_set_replay(emcg_handle *h, const uint64_t *words, int64_
     b->offCap = n_offsets;
   }
   if (nwords)
-    EMCG_CUDA(cudaMemcpy(b->dWords, words, sizeof(uint64_t) * nwords, cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(b->dOff, offsets, sizeof(int64_t) * n_offsets, cudaMemcpyHostToDevice));
+    EMCG_CUDA(copyToDevice(b->dWords, words, sizeof(uint64_t) * nwords, b->stream));
+  EMCG_CUDA(copyToDevice(b->dOff, offsets, sizeof(int64_t) * n_offsets, b->stream));
   b->replay = true;
   return EMCG_OK;
 }
@@ -2366,8 +2365,7 @@ extern "C" int32_t emcg_bulk_set_fixed_charges(emcg_handle *h, int32_t e, const 
   for (double v : planes)
     EMCG_CHECK_ARG(std::isfinite(v), "fixed charges: non-finite value");
   EMCG_CUDA(cudaMalloc(&b->dFixed[e], planes.size() * sizeof(double)));
-  EMCG_CUDA(cudaMemcpy(b->dFixed[e], planes.data(), planes.size() * sizeof(double),
-                       cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(b->dFixed[e], planes.data(), planes.size() * sizeof(double), b->stream));
   b->nFixed[e] = n;
   return EMCG_OK;
 }
@@ -2489,7 +2487,7 @@ extern "C" int32_t emcg_grain_kat(emcg_handle *h, int64_t n, double *k, uint32_t
   double *dK = nullptr;
   EMCG_CUDA(cudaMalloc(&dK, 3 * n * sizeof(double)));
   int32_t st = EMCG_OK;
-  if (cudaMemcpy(dK, k, 3 * n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (copyToDevice(dK, k, 3 * n * sizeof(double), b->stream) != cudaSuccess) {
     st = EMCG_ERR_CUDA;
   } else {
     const int blocks = (int)((n + 127) / 128);
@@ -2524,12 +2522,12 @@ extern "C" int32_t emcg_drift_kat(emcg_handle *h, int32_t valley, int64_t n, con
   double *dDt = base, *dF = base + n, *dK = base + 4 * n, *dP = base + 7 * n,
          *dE = base + 10 * n;
   int32_t *dSub = (int32_t *)(base + 11 * n);
-  EMCG_CUDA(cudaMemcpy(dSub, sub, n * sizeof(int32_t), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(dDt, dt, n * sizeof(double), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(dF, force, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(dK, k, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(dP, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(dE, energy, n * sizeof(double), cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(dSub, sub, n * sizeof(int32_t), b->stream));
+  EMCG_CUDA(copyToDevice(dDt, dt, n * sizeof(double), b->stream));
+  EMCG_CUDA(copyToDevice(dF, force, 3 * n * sizeof(double), b->stream));
+  EMCG_CUDA(copyToDevice(dK, k, 3 * n * sizeof(double), b->stream));
+  EMCG_CUDA(copyToDevice(dP, pos, 3 * n * sizeof(double), b->stream));
+  EMCG_CUDA(copyToDevice(dE, energy, n * sizeof(double), b->stream));
   int blocks = (int)((n + 127) / 128);
   if (b->precision == EMCG_FP64)
     driftKatKernel<double><<<blocks, 128, 0, b->stream>>>((const ModelK<double> *)b->dModels,

@@ -70,6 +70,11 @@ void touchPages(void *dst, size_t bytes) {
   p[bytes - 1] = 0;
 }
 
+cudaError_t copyToDevice(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 cudaError_t copyToCaller(void *dst, const void *src, size_t bytes) {
   touchPages(dst, bytes);
   return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);

@@ -1326,7 +1326,7 @@ template <class T> static int32_t createModel(DeviceImpl *d, const emcg_model_de
   EMCG_TRY(up((T **)&d->dTables, tab.data(), tab.size(), d->stream));
   K.tables = (const T *)d->dTables;
   if (sizeof(T) == 8)
-    EMCG_TRY(uploadLogTable(&d->dLogTab));
+    EMCG_TRY(uploadLogTable(&d->dLogTab, d->stream));
   K.logT = d->dLogTab;
   EMCG_TRY(up((ModelK<T> **)&d->dModel, &K, 1, d->stream));
   const size_t n = (size_t)d->nx * d->ny;
@@ -1828,15 +1828,15 @@ extern "C" int32_t emcg_device_set_grid(emcg_handle *h, int32_t which, const dou
   if (which == EMCG_GRID_EX || which == EMCG_GRID_EY) {
     void *e = which == EMCG_GRID_EX ? d->dEx : d->dEy;
     if (d->precision == EMCG_FP64) {
-      EMCG_CUDA(cudaMemcpy(e, v, n * sizeof(double), cudaMemcpyHostToDevice));
+      EMCG_CUDA(copyToDevice(e, v, n * sizeof(double), d->stream));
     } else {
       std::vector<float> f(v, v + n);
-      EMCG_CUDA(cudaMemcpy(e, f.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+      EMCG_CUDA(copyToDevice(e, f.data(), n * sizeof(float), d->stream));
     }
     return EMCG_OK;
   }
   EMCG_CHECK_ARG(dst, "unknown grid %d", which);
-  EMCG_CUDA(cudaMemcpy(dst, v, n * sizeof(double), cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(dst, v, n * sizeof(double), d->stream));
   return EMCG_OK;
 }
 
@@ -1926,8 +1926,8 @@ extern "C" int32_t emcg_device_surface_kat(emcg_handle *h, int32_t boundary, int
     return EMCG_OK;
   double *buf = nullptr;
   EMCG_CUDA(cudaMalloc(&buf, 5 * n * sizeof(double)));
-  EMCG_CUDA(cudaMemcpy(buf, k, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(buf + 3 * n, pos, 2 * n * sizeof(double), cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(buf, k, 3 * n * sizeof(double), d->stream));
+  EMCG_CUDA(copyToDevice(buf + 3 * n, pos, 2 * n * sizeof(double), d->stream));
   const uint32_t k0 = (uint32_t)d->cfg.seed, k1 = (uint32_t)(d->cfg.seed >> 32);
   const int blocks = (int)((n + 127) / 128);
   if (d->precision == EMCG_FP64)
@@ -2250,7 +2250,7 @@ extern "C" int32_t emcg_device_init(emcg_handle *h, int32_t potential_based, int
                  (long long)d->capacity);
   int32_t *dNode = nullptr;
   EMCG_CUDA(cudaMalloc(&dNode, sizeof(int32_t) * std::max<int64_t>(np, 1)));
-  EMCG_CUDA(cudaMemcpy(dNode, nodeOf.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(dNode, nodeOf.data(), sizeof(int32_t) * np, d->stream));
   const int nb = (int)((np + 255) / 256);
   if (np) {
     if (d->precision == EMCG_FP64)
@@ -2304,8 +2304,8 @@ extern "C" int32_t emcg_device_set_replay(emcg_handle *h, int32_t phase, const u
     d->offCap[phase] = n_offsets;
   }
   if (nwords)
-    EMCG_CUDA(cudaMemcpy(d->dWords[phase], words, sizeof(uint64_t) * nwords, cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(d->dOff[phase], offsets, sizeof(int64_t) * n_offsets, cudaMemcpyHostToDevice));
+    EMCG_CUDA(copyToDevice(d->dWords[phase], words, sizeof(uint64_t) * nwords, d->stream));
+  EMCG_CUDA(copyToDevice(d->dOff[phase], offsets, sizeof(int64_t) * n_offsets, d->stream));
   d->replay[phase] = true;
   return EMCG_OK;
 }
@@ -2321,7 +2321,7 @@ template <class T> static int32_t devSetStateT(DeviceImpl *d, const emcg_state *
     for (int64_t i = 0; i < n; i++)
       tmp[i] = src[f] ? (T)src[f][i] : T(0);
     if (n)
-      EMCG_CUDA(cudaMemcpy(d->dState[d->cur][f], tmp.data(), n * sizeof(T), cudaMemcpyHostToDevice));
+      EMCG_CUDA(copyToDevice(d->dState[d->cur][f], tmp.data(), n * sizeof(T), d->stream));
   }
   std::vector<uint32_t> meta((size_t)std::max<int64_t>(n, 1));
   for (int64_t i = 0; i < n; i++) {
@@ -2332,8 +2332,8 @@ template <class T> static int32_t devSetStateT(DeviceImpl *d, const emcg_state *
     meta[i] = packMeta(s->valley[i], s->sub[i], s->region[i]);
   }
   if (n)
-    EMCG_CUDA(cudaMemcpy(d->dMeta[d->cur], meta.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  EMCG_CUDA(cudaMemcpy(d->dN, &n, sizeof(int64_t), cudaMemcpyHostToDevice));
+    EMCG_CUDA(copyToDevice(d->dMeta[d->cur], meta.data(), n * sizeof(uint32_t), d->stream));
+  EMCG_CUDA(copyToDevice(d->dN, &n, sizeof(int64_t), d->stream));
   return EMCG_OK;
 }
 

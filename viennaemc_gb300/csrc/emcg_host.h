@@ -46,6 +46,12 @@ const char *statusName(int32_t s);
 // space), else nullptr: only such ranges are read by kernels over the host link.
 const void *mappedHostRange(const void *p, size_t bytes);
 
+// Copy of host memory to the device on the stream whose kernels read it, complete
+// on return.  The engines' streams do not wait for the null stream, and a plain
+// cudaMemcpy from pageable memory returns once the data is staged, so nothing would
+// order its transfer before their next kernel.
+cudaError_t copyToDevice(void *dst, const void *src, size_t bytes, cudaStream_t st);
+
 // Copy from the device to the caller's array, whose pages are touched first: a
 // copy into ordinary memory that no one has written yet (a freshly zeroed
 // array) takes its page faults from the GPU's side, one after another.  Measured

@@ -111,8 +111,8 @@ inline int32_t validateModel(const emcg_model_desc &m) {
   return EMCG_OK;
 }
 
-// logTab()'s table on the device (ModelK::logT)
-inline int32_t uploadLogTable(double **dst) {
+// logTab()'s table on the device (ModelK::logT), for kernels on stream st
+inline int32_t uploadLogTable(double **dst, cudaStream_t st) {
   static const std::vector<double> tab = [] { // a constant, formed once
     std::vector<double> t(kLogTab);
     for (int i = 0; i < kLogTab; i++)
@@ -120,7 +120,7 @@ inline int32_t uploadLogTable(double **dst) {
     return t;
   }();
   EMCG_CUDA(cudaMalloc(dst, kLogTab * sizeof(double)));
-  EMCG_CUDA(cudaMemcpy(*dst, tab.data(), kLogTab * sizeof(double), cudaMemcpyHostToDevice));
+  EMCG_CUDA(copyToDevice(*dst, tab.data(), kLogTab * sizeof(double), st));
   return EMCG_OK;
 }
 
