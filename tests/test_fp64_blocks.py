@@ -1,0 +1,63 @@
+"""The double engines' building blocks against the plain expressions they stand for,
+natively compiled and through the engines."""
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+def _native(tmp_path, name):
+    exe = tmp_path / name
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off",
+                    f"-I{ROOT}/viennaemc_gb300/csrc", f"{ROOT}/tests/native/{name}.cpp", "-o",
+                    str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+
+
+def test_comparisons_and_fixed_point(tmp_path):
+    assert _native(tmp_path, "fp64_check") == ["0", "0"]
+
+
+def _bar(nx=41, ny=31, h=1e-9):
+    from viennaemc_gb300 import device as D
+    from viennaemc_gb300.physics import silicon_material
+    lx, ly = (nx - 1) * h, (ny - 1) * h
+    dev = D.Device(silicon_material(), (lx, ly), (h, h))
+    dev.addConstantDopingRegion((0, 0), (lx, ly), 1e24)
+    dev.addOhmicContact(D.XMIN, 0.0, (0,), (ly,))
+    dev.addOhmicContact(D.XMAX, 0.0, (0,), (ly,))
+    return dev
+
+
+def _resting(engine, pos):
+    """Electrons at rest at pos (n x 2) without an event ahead; k of -0, so that a
+    field-free flight leaves a coordinate of -0 as it is."""
+    n = len(pos)
+    z = np.zeros(n)
+    return engine.ParticleState.from_arrays(
+        kx=-z, ky=-z, kz=-z, px=pos[:, 0], py=pos[:, 1], pz=z, energy=z,
+        tau=np.full(n, 1.0), grain_tau=np.full(n, 1.0), valley=np.zeros(n, np.int32),
+        sub=np.zeros(n, np.int32), region=np.zeros(n, np.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_minus_zero_is_inside_the_device(engine, precision):
+    """Removal at a contact is for positions < 0 or > max (include/emcParticleDrift.hpp:
+    41-66): -0 and max itself stay."""
+    from viennaemc_gb300 import device as D
+    dev = _bar()
+    pt = engine.physics.silicon_electron("refbulk", n_levels=100, max_energy=4.0)
+    sim = D.DeviceSimulation(dev, pt, scheme=D.NGP, capacity=64, dt=1e-16, precision=precision)
+    y = dev.max_pos[1] / 2
+    pos = np.array([[-0.0, y], [0.0, y], [dev.max_pos[0], y], [-1e-12, y], [3e-9, y]])
+    sim.set_state(_resting(engine, pos))
+    netto = sim.move(step=0)
+    st = sim.get_state()
+    sim.close()
+    assert netto.sum() == 1 and st.n == 4  # the one outside
+    assert sorted(st.px) == sorted(np.float32(pos[[0, 1, 2, 4], 0]) if precision == "fp32"
+                                   else pos[[0, 1, 2, 4], 0])

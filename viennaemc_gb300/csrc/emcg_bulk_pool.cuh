@@ -191,7 +191,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
   p.tau -= t;
   p.in = 0.0;
   p.gtau -= EK.dt;
-  if (belowD(p.gtau, 0.0) || __double_as_longlong(p.gtau) == 0)
+  if (belowD(p.gtau, 0.0) || (__double_as_longlong(p.gtau) << 1) == 0)
     poolGrain(M, EK, pid, step0 + (uint32_t)p.step, p);
   const double *gd = EK.g[valley][sub];
   const double gk = fma(gd[2], p.k[2], fma(gd[1], p.k[1], gd[0] * p.k[0]));

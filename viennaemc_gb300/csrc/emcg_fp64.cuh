@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "emcg_fp64.h"
+
 namespace emcg {
 
 // 1 / sqrt(t) for normal t > 0: the hardware's approximation (about 20 bits)
@@ -50,25 +52,6 @@ __device__ __forceinline__ double divD(double a, double b) {
     return a / b;
   const double inv = rcpD(b), q = a * inv;
   return fma(fma(-b, q, a), inv, q);
-}
-
-// a < b for a double a and b >= 0 without a double-precision instruction: the
-// bit patterns of non-negative doubles order like the values, those of
-// negative ones are negative integers; a NaN is not below
-__device__ __forceinline__ bool belowD(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return x < y && (unsigned long long)x <= 0xfff0000000000000ull;
-}
-
-// q as an integer part and 20 fractional bits, for 0 <= q < 2^30; false outside
-__device__ __forceinline__ bool fixedOf(double q, uint64_t &f) {
-  const uint64_t b = (uint64_t)__double_as_longlong(q);
-  const int e = (int)(b >> 52) - 1023;
-  if (e >= 30) // also a negative q, infinities and NaN
-    return false;
-  const uint64_t mant = (b & 0xfffffffffffffull) | 0x10000000000000ull;
-  f = e < -31 ? 0 : mant >> (32 - e);
-  return true;
 }
 
 } // namespace emcg
