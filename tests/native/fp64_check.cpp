@@ -1,5 +1,7 @@
 // emcg_fp64.h against the plain expressions it stands for: prints the number of
-// disagreements of belowD and of fixedOf.
+// disagreements of belowD and of fixedOf, and the largest errors of rsqrtStep and
+// rcpStep in units of the last place, from approximations of 20 fraction bits within
+// 2^-20 of the value (the instructions' form).
 #include <cmath>
 #include <cstdio>
 #include <random>
@@ -30,6 +32,19 @@ int main() {
     const bool in = fixedOf(q, f);
     badFixed += in != (q < 0x1p30) || (in && f != (uint64_t)std::floor(q * 0x1p20));
   }
-  std::printf("%ld %ld\n", badBelow, badFixed);
+  double worst[2] = {0, 0};
+  std::uniform_real_distribution<double> x(-1000, 1000);
+  for (int i = 0; i < 4000000; i++) {
+    const double t = std::exp2(i & 1 ? x(g) : x(g) * 0.002);
+    for (int k = 0; k < 2; k++) {
+      const long double want = k ? 1.0L / (long double)t : 1.0L / std::sqrt((long double)t);
+      // the 20-bit neighbour below or above
+      const double y = bitsd((dbits((double)want) & ~0xffffffffull) + ((g() & 1) << 32));
+      const double got = k ? rcpStep(t, y) : rsqrtStep(t, y);
+      const double ulp = std::ldexp(1.0, std::ilogb((double)want) - 52);
+      worst[k] = std::fmax(worst[k], (double)std::fabs(((long double)got - want) / ulp));
+    }
+  }
+  std::printf("%ld %ld %.4f %.4f\n", badBelow, badFixed, worst[0], worst[1]);
   return 0;
 }

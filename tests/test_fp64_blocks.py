@@ -17,8 +17,30 @@ def _native(tmp_path, name):
     return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
 
 
-def test_comparisons_and_fixed_point(tmp_path):
-    assert _native(tmp_path, "fp64_check") == ["0", "0"]
+def test_comparisons_fixed_point_and_steps(tmp_path):
+    """The steps round once at the result's size (half a unit); what they leave out is
+    5 e^3 / 16 with |e| < 2^-19 (0.02 units) and r^3 with r < 2^-20 (0.01)."""
+    below, fixed, rsqrt, rcp = _native(tmp_path, "fp64_check")
+    assert (below, fixed) == ("0", "0")
+    assert float(rsqrt) <= 0.53 and float(rcp) <= 0.52
+
+
+@pytest.mark.gpu
+def test_roots_and_quotients_on_the_gpu(engine, tmp_path):
+    """The hardware's approximations cut their argument and their result to 20 fraction
+    bits, so they are within 2^-19; from them the steps' bounds, and sqrtD and divD,
+    corrected once at the result's size, half a unit and a hundredth; at the ends of
+    their ranges the library's results or their neighbours, outside its own."""
+    exe = tmp_path / "fp64_gpu_check"
+    lib = engine._lib
+    subprocess.run([lib._nvcc(), lib.ARCH, "-O3", "-std=c++17", f"-I{lib.INCLUDE}",
+                    f"-I{lib.CSRC}", f"{ROOT}/tests/native/fp64_gpu_check.cu", "-o", str(exe)],
+                   check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    low, approx, rsqrt, rcp, root, quotient, edges = map(float, out)
+    assert low == 0 and approx <= 2.0  # approx: in 2^-20
+    assert rsqrt <= 0.53 and rcp <= 0.52 and root <= 0.51 and quotient <= 0.51
+    assert edges == 0
 
 
 def _bar(nx=41, ny=31, h=1e-9):

@@ -1,8 +1,8 @@
 // Double-precision building blocks for a GPU whose schedulers issue one double
 // instruction of a warp in 64 clocks: square root, reciprocal and quotient from
-// the hardware's approximations with one correction each, and comparisons and
-// frame rotations without double instructions.  All give the correctly rounded
-// result or its neighbour; arguments outside their range go to the library.
+// the hardware's approximations with one correction each.  The results are the
+// correctly rounded ones or their neighbours; sqrtD and divD hand arguments outside
+// their range to the library.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -12,24 +12,17 @@
 
 namespace emcg {
 
-// 1 / sqrt(t) for normal t > 0: the hardware's approximation (about 20 bits)
-// and one step of Householder's method of third order (Householder 1970):
-// with e = 1 - t y^2, y (1 + e / 2 + 3 e^2 / 8)
+// 1 / sqrt(t) for normal t > 0, and 1 / d for normal d whose reciprocal is normal
+// (the caller's to see to: neither has another path)
 __device__ __forceinline__ double rsqrtD(double t) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
-  const double e = fma(-t * y, y, 1.0);
-  return fma(fma(0.375, e, 0.5), y * e, y);
+  return rsqrtStep(t, y);
 }
-
-// 1 / d for normal d whose reciprocal is normal: the hardware's approximation
-// (about 20 bits) and y (1 + r + r^2), r = 1 - d y (the geometric series to
-// third order)
 __device__ __forceinline__ double rcpD(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double r = fma(-d, y, 1.0);
-  return fma(y, fma(r, r, r), y);
+  return rcpStep(d, y);
 }
 
 // sqrt(x): x / sqrt(x) corrected once; 0, subnormals, infinities, negative

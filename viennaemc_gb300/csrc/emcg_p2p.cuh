@@ -41,6 +41,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "emcg_fp64.cuh"
 #include "emcg_host.h"
 
 namespace emcg {
@@ -131,22 +132,14 @@ __device__ __forceinline__ void pairTermF2(f32x2 x, f32x2 y, f32x2 z, f32x2 nx, 
   acc[3] = fma2(c, q, acc[3]);
 }
 
-// The double pair term, the same form.  1 / r: the hardware's approximation
-// (about 20 bits) and one step of Householder's third-order method; 0,
-// subnormal, infinite and NaN r^2 by the reference's 1 / r^2 and square root.
+// The double pair term, the same form.  0, subnormal, infinite and NaN r^2 by the
+// reference's 1 / r^2 and square root.
 __device__ __forceinline__ void pairTermD(double xi, double yi, double zi, double nx, double ny,
                                           double nz, double q, double invCut, double acc[4]) {
   const double dx = xi + nx, dy = yi + ny, dz = zi + nz;
   const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-  double inv;
-  if ((uint32_t)__double2hiint(r2) - 0x00100000u < 0x7fe00000u) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-    const double e = fma(-r2 * y, y, 1.0);
-    inv = fma(fma(0.375, e, 0.5), y * e, y);
-  } else {
-    inv = sqrt(1.0 / r2);
-  }
+  const double inv = (uint32_t)__double2hiint(r2) - 0x00100000u < 0x7fe00000u ? rsqrtD(r2)
+                                                                               : sqrt(1.0 / r2);
   // inv > invCut by the bit patterns (both >= 0; a NaN stays)
   const long long bi = __double_as_longlong(inv);
   const double c = bi > __double_as_longlong(invCut) && bi <= 0x7ff0000000000000ll ? invCut : inv;
