@@ -18,7 +18,7 @@ LIB_PATH = os.path.join(PKG, "libemcgpu.so")
 SOURCES = ["emcg_core.cu", "emcg_bulk.cu", "emcg_device.cu", "emcg_poisson.cu", "emcg_p2p.cu"]
 HEADERS = ["emcg_bulk_pool.cuh", "emcg_common.cuh", "emcg_draws.h", "emcg_exp.h",
            "emcg_fp64.cuh", "emcg_fp64.h", "emcg_host.h", "emcg_log.h", "emcg_model.h",
-           "emcg_p2p.cuh", "emcg_poisson.cuh", "emcg_rates.cuh"]
+           "emcg_p2p.cuh", "emcg_pages.h", "emcg_poisson.cuh", "emcg_rates.cuh"]
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 MAX_VALLEYS, MAX_DEG, MAX_MECH, MAX_NF, MAX_REGIONS = 4, 8, 32, 8, 16

@@ -1,5 +1,6 @@
 // Error reporting, version and page-locked host blocks of libemcgpu.
 #include "emcg_host.h"
+#include "emcg_pages.h"
 
 #include <cstdint>
 #include <map>
@@ -64,10 +65,7 @@ void touchPages(void *dst, size_t bytes) {
   }
   if (at.type != cudaMemoryTypeUnregistered)
     return;
-  volatile char *p = static_cast<volatile char *>(dst);
-  for (size_t o = 0; o < bytes; o += 4096)
-    p[o] = 0;
-  p[bytes - 1] = 0;
+  touchRange(dst, bytes);
 }
 
 cudaError_t copyToDevice(void *dst, const void *src, size_t bytes, cudaStream_t st) {

@@ -59,7 +59,7 @@ cudaError_t copyToDevice(void *dst, const void *src, size_t bytes, cudaStream_t 
 // touched, 11 us to touch it.  On the null stream, complete on return.
 cudaError_t copyToCaller(void *dst, const void *src, size_t bytes);
 // The touch alone, for asynchronous copies (a no-op for page-locked and device
-// memory).
+// memory); the array keeps its values.
 void touchPages(void *dst, size_t bytes);
 
 struct BulkImpl;
