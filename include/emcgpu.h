@@ -591,7 +591,8 @@ int32_t emcg_device_poisson_counts(emcg_handle *h, int64_t *cycles, int64_t *sol
    Working memory is one fixed device array of about 21 MB in this library:
    grids of up to 131072 nodes and 8192 nodes per dimension, at most 64
    contacts (ohmic or gate); larger inputs return EMCG_ERR_ARG and touch
-   nothing.  Every call rebuilds the array's contents, including the
+   nothing.  On the calling thread's stack the call itself takes up to 48 KB,
+   to which the CUDA runtime's own calls add.  Every call rebuilds the array's contents, including the
    statistics that must start at zero.
    The array belongs to this library's device code, which CUDA loads onto a
    device lazily by default: at the library's first kernel launch there or

@@ -1931,26 +1931,31 @@ struct MGTail {
   int level = 0, size = 0;
   bool even = true;
 };
+// The tail's launch (its status is the solve's next cudaGetLastError).  A call: its
+// descriptors, 8 KB, are not on the stack of every level of the recursion.
+template <class MT>
+__attribute__((noinline)) void launchTail(const MGSet &P, const LevelK<MT> &K, const MGTail &tail,
+                                          cudaStream_t st) {
+  MGSet T = P;
+  T.L += tail.level;
+  T.nLev -= tail.level;
+  size_t bytes = 0;
+  const CMG<MT> M = clusterDesc<MT>(T, tail.size, &bytes, tail.even);
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = clusterConfig<MT>(tail.size, bytes, st, &at);
+  cudaLaunchKernelEx(&cfg, clusterKernel<MT, true>(M), M, (double *)nullptr,
+                     (const double *)nullptr, (const double *)nullptr, (const double *)nullptr,
+                     (const double *)nullptr, 0., 0., 0., 0., 0, 0., (const double *)nullptr,
+                     (double *)nullptr, (const MT *)K.r, (const MT *)K.rho, K.d,
+                     (const int *)nullptr);
+}
 template <class MT>
 void vcycle(const MGSet &P, int l, const MGTail &tail, cudaStream_t st) {
   const MGLevel &lv = P.L[l];
   LevelK<MT> K = levelK<MT>(lv);
   const int n = lv.nx * lv.ny;
-  if (tail.level && l == tail.level) {
-    MGSet T = P;
-    T.L += l;
-    T.nLev -= l;
-    size_t bytes = 0;
-    const CMG<MT> M = clusterDesc<MT>(T, tail.size, &bytes, tail.even);
-    cudaLaunchAttribute at;
-    cudaLaunchConfig_t cfg = clusterConfig<MT>(tail.size, bytes, st, &at);
-    cudaLaunchKernelEx(&cfg, clusterKernel<MT, true>(M), M, (double *)nullptr,
-                       (const double *)nullptr, (const double *)nullptr, (const double *)nullptr,
-                       (const double *)nullptr, 0., 0., 0., 0., 0, 0., (const double *)nullptr,
-                       (double *)nullptr, (const MT *)K.r, (const MT *)K.rho, K.d,
-                       (const int *)nullptr);
-    return; // its status is the solve's next cudaGetLastError
-  }
+  if (tail.level && l == tail.level)
+    return launchTail<MT>(P, K, tail, st);
   if (l + 1 == P.nLev) {
     coarseSolveKernel<MT><<<1, 256, 0, st>>>(K, P.coarseSweeps);
     return;
@@ -2366,7 +2371,8 @@ int32_t poissonFinish(PoissonMG &P, double rtol, double *relRes, int *cycles) {
 // -- fine-grid inputs, the multigrid hierarchy, transfer tables and residual
 // statistics -- lives in one file-scope device array of fixed size, reserved
 // when this library's device code is loaded.  It is rebuilt from the caller's
-// description by kernels on every call; the host side uses only stack memory.
+// description by kernels on every call; the host side uses only stack memory, of which
+// a frame of 31 KB and below it the tail's 8 KB or the levels' recursion.
 // Host code cannot pass the array's name to a kernel as an address: the first
 // call on each device asks the runtime for the address (cudaGetSymbolAddress,
 // with that device current) and keeps it.  The array is shared by all calls,
@@ -2379,6 +2385,11 @@ constexpr int kNAMaxNodes = 1 << 17;           // fine-grid nodes, e.g. 401 x 20
 constexpr int kNAMaxDim = 8192;                // nodes per dimension
 constexpr int kNAMaxLevels = 16;               // as the allocating hierarchy
 constexpr int kNAMaxContacts = 64;
+// the boundaries' contacts and the contacts' types: a byte each, so that the copy of
+// them that the call keeps on its stack is 16 KB (131 KB as int); the longest
+// boundary is that of kNAMaxDim nodes by what kNAMaxNodes leaves
+constexpr int kNAMaxEdge = 2 * (kNAMaxDim + kNAMaxNodes / kNAMaxDim) + kNAMaxContacts;
+static_assert(kNAMaxContacts <= 127, "contacts in a byte");
 constexpr int kNAMaxDevices = 64;
 constexpr int kNAVcyclesPerNewton = 3; // as PoissonMG's defaults
 constexpr double kNATwoCycleRel = 1e30;
@@ -2402,9 +2413,8 @@ constexpr size_t kOffStats = kOffResNe + 8ull * kNAMaxNodes; // double [4] resid
 constexpr size_t kOffLevelF = kOffStats + 256;               // float [9 x all levels]
 constexpr size_t kOffTransF = kOffLevelF + 4ull * 9 * kNALevelNodes; // float [1-D]
 constexpr size_t kOffTransI = kOffTransF + 4ull * kNA1D;             // int   [1-D]
-constexpr size_t kOffBnd = kOffTransI + 4ull * kNA1D;                // int   [2 (ny + nx)]
-constexpr size_t kOffCtype = kOffBnd + 4ull * 4 * kNAMaxDim;         // int   [contacts]
-constexpr size_t kOffResMask = kOffCtype + 4ull * kNAMaxContacts;    // u8    [N]
+constexpr size_t kOffBnd = kOffTransI + 4ull * kNA1D;                // i8 [2 (ny + nx) + contacts]
+constexpr size_t kOffResMask = kOffBnd + kNAMaxEdge;                 // u8    [N]
 constexpr size_t kOffFixed = kOffResMask + kNAMaxNodes;              // u8    [all levels]
 constexpr size_t kOffCls = (kOffFixed + kNALevelNodes + 255) & ~size_t(255); // u8 [all levels]
 constexpr size_t kOffTab = kOffCls + kNALevelNodes; // float [levels x classes x 8]
@@ -2442,7 +2452,7 @@ __device__ __forceinline__ double naCoord(const NALevels &lv, int l, int I, bool
 // emcg_device_create prepares on the host for the allocating solver.
 __global__ void naFineSetupKernel(int nx, int ny, double Ni, double hF0, double hF1, double h0,
                                   double h1, NAContacts ct, const double *doping,
-                                  const int32_t *bnd, const int32_t *ctype, double *C,
+                                  const int8_t *bnd, const int8_t *ctype, double *C,
                                   double *gSum, double *gVeq, double *gVne, double *gDx,
                                   double *gDy, uint8_t *resMask, double *resEq, double *resNe,
                                   uint8_t *fixed) {
@@ -2762,22 +2772,19 @@ extern "C" int32_t emcg_poisson_solve_noalloc(const emcg_device_desc *dv, double
   double *resNe = (double *)(S + kOffResNe), *stats = (double *)(S + kOffStats);
   float *levF = (float *)(S + kOffLevelF), *trF = (float *)(S + kOffTransF);
   int *trI = (int *)(S + kOffTransI);
-  int32_t *bnd = (int32_t *)(S + kOffBnd), *ctype;
+  int8_t *bnd = (int8_t *)(S + kOffBnd);
   uint8_t *resMask = S + kOffResMask, *fixedAll = S + kOffFixed;
   EMCG_CUDA(cudaMemcpyAsync(doping, dv->doping, sizeof(double) * n, cudaMemcpyHostToDevice, st));
   // the boundaries' contacts and the contact types behind them, in one copy
-  static_assert(kOffCtype == kOffBnd + 4ull * 4 * kNAMaxDim, "room for the types too");
-  const int32_t *bsrc[4] = {dv->boundary_contact[0], dv->boundary_contact[1],
-                            dv->boundary_contact[2], dv->boundary_contact[3]};
-  int32_t hBnd[4 * kNAMaxDim + kNAMaxContacts];
-  const int nBnd = 2 * (nx + ny);
-  for (int b = 0, o = 0; b < 4; o += b < 2 ? ny : nx, b++)
-    std::memcpy(hBnd + o, bsrc[b], sizeof(int32_t) * (b < 2 ? ny : nx));
-  if (dv->n_contacts)
-    std::memcpy(hBnd + nBnd, dv->contact_type, sizeof(int32_t) * dv->n_contacts);
-  ctype = bnd + nBnd;
-  EMCG_CUDA(cudaMemcpyAsync(bnd, hBnd, sizeof(int32_t) * (nBnd + dv->n_contacts),
-                            cudaMemcpyHostToDevice, st));
+  int8_t hBnd[kNAMaxEdge];
+  int8_t *put = hBnd;
+  for (int b = 0; b < 4; b++)
+    for (int k = 0; k < (b < 2 ? ny : nx); k++)
+      *put++ = (int8_t)dv->boundary_contact[b][k];
+  const int8_t *ctype = bnd + (put - hBnd);
+  for (int c = 0; c < dv->n_contacts; c++)
+    *put++ = (int8_t)dv->contact_type[c];
+  EMCG_CUDA(cudaMemcpyAsync(bnd, hBnd, (size_t)(put - hBnd), cudaMemcpyHostToDevice, st));
   const double hF0 = lv.h1 / lv.h0, hF1 = lv.h0 / lv.h1;
   double hP = 1.;
   hP = hP * lv.h0;
