@@ -302,7 +302,9 @@ int32_t emcg_last_kernel_ms(emcg_handle *h, double *ms);
 /* Tuning: threads per block (multiple of 32, <= 1024; -1 = automatic, the
    default: 256, or 128 for launches of the warp-asynchronous kernel shorter
    than 100 steps, whose blocks' warps end far apart) and steps fused per
-   kernel launch (observables flushed every chunk). 0 keeps the current. */
+   kernel launch (observables flushed every chunk). 0 keeps the current.
+   A double engine's pooled kernel (scatter mode 0) runs one warp per block
+   and takes no block size; its Coulomb, replay and block-queued steps do. */
 int32_t emcg_set_launch(emcg_handle *h, int32_t block_threads,
                         int32_t steps_per_launch);
 /* The block size of the last launch (or the set one) and the steps per
@@ -337,7 +339,8 @@ int32_t emcg_get_pass_actions(emcg_handle *h, int32_t *n);
 
 /* Tuning: register cap of the step kernel, as the minimum number of resident
    256-thread blocks per SM (1 = uncapped, 3 or 4); capped variants apply to
-   blocks of at most 256 threads. */
+   blocks of at most 256 threads.  A double engine's pooled kernel (scatter
+   mode 0) has no capped variant. */
 int32_t emcg_set_occupancy(emcg_handle *h, int32_t min_blocks_per_sm);
 /* Graph replay (enable != 0): each launch of steps is an instantiated CUDA
    graph (observable reset -> step kernel) replayed with its step offset
@@ -345,12 +348,14 @@ int32_t emcg_set_occupancy(emcg_handle *h, int32_t min_blocks_per_sm);
 int32_t emcg_bulk_set_graph(emcg_handle *h, int32_t enable);
 /* Autotuner: runs trial_steps steps (from step0, advancing the ensembles --
    use it as warm-up) with each candidate launch shape (block threads 128 /
-   256, register cap 1 / 3 / 4 resident blocks per SM, lockstep,
-   block-queued or, for float, warp-asynchronous scatter with 3 or 6 free
-   flights per pass), twice: in a forward and then a backward pass over the
-   shapes.  It keeps the shape of least total device time (its pass actions:
-   emcg_get_pass_actions).  *steps_used = steps run (2 x shapes x
-   trial_steps: 13 float shapes, 8 double); outputs may be NULL.  No
+   256, register cap 1 / 3 / 4 resident blocks per SM; float: lockstep,
+   block-queued or warp-asynchronous scatter with 3 or 6 free flights per
+   pass; double: block-queued, and the pooled kernel once), twice: in a
+   forward and then a backward pass over the shapes.  It keeps the shape of
+   least total device time (its pass actions: emcg_get_pass_actions); where
+   that is the pooled kernel, which has neither, the block size and the
+   register cap stay as they were set.  *steps_used = steps run (2 x shapes x
+   trial_steps: 13 float shapes, 4 double); outputs may be NULL.  No
    reference counterpart. */
 int32_t emcg_bulk_autotune(emcg_handle *h, int32_t trial_steps, uint32_t step0,
                            int32_t *steps_used, int32_t *block_threads, int32_t *min_blocks,

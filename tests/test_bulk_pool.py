@@ -93,3 +93,23 @@ def test_pooled_kernel_equals_queued_kernel(engine, model, counts):
         if model != "grain" and n:
             assert np.allclose(oa[:, :, 2], oq[:, :, 2], atol=2)
             assert np.allclose(oa.sum(axis=1)[:, 0], oq.sum(axis=1)[:, 0], rtol=1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("block", [0, 64])
+def test_autotune_of_a_double_engine(engine, block):
+    """The pooled kernel has one shape: it is tried once beside the three block-queued
+    ones, and where it wins (it does, threefold) the block size and the register cap
+    of the other steps stay as they were, automatic ones too."""
+    spec = engine.EnsembleSpec(0, 20000, 1e6, (1, 0, 0), (1e-6,) * 3, 1e-15, 3)
+    b = engine.BulkBatch([engine.silicon_electron("jacoboni")], [spec], "fp64")
+    b.set_launch(block_threads=block, steps_per_launch=7, min_blocks=3)
+    b.init_particles(0)
+    b.step(2)
+    before = b.launch()
+    cfg = b.autotune(5)
+    assert cfg["steps_used"] == 2 * 4 * 5 and cfg["queued"] == 0
+    assert cfg["block_threads"] == before["block_threads"] == (block or 256)
+    assert cfg["min_blocks"] == 3 and b.launch() == before
+    assert np.array_equal(b.step(3)[0, :, :, 2].sum(axis=1), np.full(3, 20000))
+    b.close()

@@ -2400,39 +2400,49 @@ extern "C" int32_t emcg_bulk_autotune(emcg_handle *h, int32_t trial_steps, uint3
   // that the ensembles' warming up from the initial distribution (events get
   // more frequent) weighs on every shape alike; the least total device time
   // wins
-  // (the warp-asynchronous kernel with 3 and with 6 free flights per pass)
+  // (the warp-asynchronous kernel, float only, with 3 and with 6 free flights per
+  // pass; the double engine's pooled kernel has one shape, whatever the block size
+  // and the cap: it runs once, and they stay as they were where it wins)
   struct Cand {
     int block, minb, queued, pass;
   };
-  const Cand cands[] = {{256, 4, 0, 0}, {256, 3, 0, 0}, {256, 1, 0, 0}, {128, 4, 0, 0},
-                        {128, 1, 0, 0}, {256, 4, 1, 0}, {256, 3, 1, 0}, {128, 4, 1, 0},
-                        {256, 4, 2, 3}, {256, 3, 2, 3}, {128, 4, 2, 3}, {256, 4, 2, 6},
-                        {128, 4, 2, 6}};
-  constexpr int kCands = sizeof(cands) / sizeof(cands[0]);
-  const int nCands = b->precision == EMCG_FP32 ? kCands : 8; // mode 2 is float only
+  static const Cand cands32[] = {{256, 4, 0, 0}, {256, 3, 0, 0}, {256, 1, 0, 0}, {128, 4, 0, 0},
+                                 {128, 1, 0, 0}, {256, 4, 1, 0}, {256, 3, 1, 0}, {128, 4, 1, 0},
+                                 {256, 4, 2, 3}, {256, 3, 2, 3}, {128, 4, 2, 3}, {256, 4, 2, 6},
+                                 {128, 4, 2, 6}};
+  static const Cand cands64[] = {{0, 0, 0, 0}, {256, 4, 1, 0}, {256, 3, 1, 0}, {128, 4, 1, 0}};
+  constexpr int kCands = sizeof(cands32) / sizeof(cands32[0]);
+  const bool fp32 = b->precision == EMCG_FP32;
+  const Cand *cands = fp32 ? cands32 : cands64;
+  const int nCands = fp32 ? kCands : (int)(sizeof(cands64) / sizeof(cands64[0]));
   const int keepPer = b->stepsPerLaunch, keepPass = b->passActions;
-  const bool keepPassAuto = b->passAuto;
-  b->autoBlock = false; // the tuner sets the block size
-  b->passAuto = false;  // and the free flights per pass of each shape
+  const int keepBlock = b->blockThreads, keepMin = b->minBlocks, keepQueued = b->queued;
+  const bool keepPassAuto = b->passAuto, keepAuto = b->autoBlock;
+  // the engine as cands[ci] sets it (-1: as it was)
+  auto use = [&](int ci) {
+    const Cand c = ci < 0 ? Cand{0, 0, keepQueued, 0} : cands[ci];
+    const int block = c.block ? c.block : keepBlock;
+    b->tilesDirty = b->tilesDirty || block != b->blockThreads;
+    b->blockThreads = block;
+    b->minBlocks = c.minb ? c.minb : keepMin;
+    b->queued = c.queued;
+    b->autoBlock = c.block ? false : keepAuto;
+    b->passActions = c.pass ? c.pass : keepPass;
+    b->passAuto = c.pass ? false : keepPassAuto;
+  };
   b->stepsPerLaunch = trial_steps;
   double ms[kCands] = {};
   uint32_t s = step0;
   for (int pass = 0; pass < 2 * nCands; pass++) {
     const int ci = pass < nCands ? pass : 2 * nCands - 1 - pass;
-    const Cand &c = cands[ci];
-    if (c.block != b->blockThreads)
-      b->tilesDirty = true;
-    b->blockThreads = c.block;
-    b->minBlocks = c.minb;
-    b->queued = c.queued;
-    b->passActions = c.pass ? c.pass : keepPass;
-    int32_t st = b->precision == EMCG_FP64 ? stepTyped<double>(b, trial_steps, s, nullptr)
-                                           : stepTyped<float>(b, trial_steps, s, nullptr);
+    use(ci);
+    b->passAuto = false; // the tuner sets the free flights per pass of each shape
+    int32_t st = fp32 ? stepTyped<float>(b, trial_steps, s, nullptr)
+                      : stepTyped<double>(b, trial_steps, s, nullptr);
     s += trial_steps;
     if (st != EMCG_OK) {
       b->stepsPerLaunch = keepPer;
-      b->passActions = keepPass;
-      b->passAuto = keepPassAuto;
+      use(-1);
       return st;
     }
     ms[ci] += b->lastMs;
@@ -2441,23 +2451,16 @@ extern "C" int32_t emcg_bulk_autotune(emcg_handle *h, int32_t trial_steps, uint3
   for (int ci = 1; ci < nCands; ci++)
     if (ms[ci] < ms[bi])
       bi = ci;
-  const Cand bestC = cands[bi];
-  if (bestC.block != b->blockThreads)
-    b->tilesDirty = true;
-  b->blockThreads = bestC.block;
-  b->minBlocks = bestC.minb;
-  b->queued = bestC.queued;
-  b->passActions = bestC.pass ? bestC.pass : keepPass;
-  b->passAuto = bestC.pass ? false : keepPassAuto;
+  use(bi);
   b->stepsPerLaunch = keepPer;
   if (steps_used)
     *steps_used = (int32_t)(s - step0);
   if (block_threads)
-    *block_threads = bestC.block;
+    *block_threads = b->blockThreads;
   if (min_blocks)
-    *min_blocks = bestC.minb;
+    *min_blocks = b->minBlocks;
   if (queued)
-    *queued = bestC.queued;
+    *queued = b->queued;
   return EMCG_OK;
 }
 
