@@ -113,3 +113,39 @@ def test_autotune_of_a_double_engine(engine, block):
     assert cfg["min_blocks"] == 3 and b.launch() == before
     assert np.array_equal(b.step(3)[0, :, :, 2].sum(axis=1), np.full(3, 20000))
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [20, 20000])
+def test_event_limit_of_a_step(engine, n):
+    """An electron may have 65,536 events in a step, real or self-scattering: a step of
+    62,000 mean free flights (249 is a standard deviation) runs, one of 69,000 does not,
+    in the pooled kernel as in the block-queued one.  Without a field the first gives
+    equal electrons, bar last-ulp branch flips."""
+    pt = engine.silicon_electron("jacoboni")
+    got = {}
+    for flights in (62000, 69000):
+        for mode in (0, 1):
+            spec = engine.EnsembleSpec(0, 20, 0.0, (1, 0, 0), (1e-6,) * 3, 1e-15, 3)
+            more = [engine.EnsembleSpec(0, n - 20, 0.0, (1, 0, 0), (1e-6,) * 3, 1e-18, 4)] * (n > 20)
+            b = engine.BulkBatch([pt], [spec] + more, "fp64")
+            tau = float(np.atleast_1d(b.get_rates(0)[1])[0])
+            b.close()
+            spec = engine.EnsembleSpec(0, 20, 0.0, (1, 0, 0), (1e-6,) * 3, flights * tau, 3)
+            b = engine.BulkBatch([pt], [spec] + more, "fp64")
+            b.set_launch(queued=mode)
+            for e in range(1 + len(more)):
+                b.init_particles(e)
+            if flights == 69000:
+                with pytest.raises(engine._lib.EmcgError, match="gave up"):
+                    b.step(1)
+            else:
+                b.step(1)
+                got[mode] = b.get_state(0)
+            b.close()
+    a, q = got[0], got[1]
+    bad = (a.valley != q.valley) | (a.sub != q.sub)
+    for f in ("kx", "ky", "kz", "energy", "tau"):
+        x, y = getattr(a, f), getattr(q, f)
+        bad |= np.abs(x - y) > 1e-9 * np.max(np.abs(y))
+    assert bad.sum() <= 1

@@ -39,9 +39,13 @@ namespace emcg {
 constexpr int kPoolWindow = 8; // steps an electron may be ahead of the pool's slowest
 constexpr int kPoolFold = 4;   // steps added up at a time, by eight lanes each
 constexpr int kPoolFields = 13; // k, d, E, tau, gtau, in, x in shared memory
-constexpr uint32_t kPoolMaxWords = 2u << 16; // draws of one electron in one step
+constexpr uint32_t kPoolMaxEvents = 1u << 16; // of one electron in one step
 
+// an electron's kind word: PoolKind, its mechanism in bits 8 to 12, its events in the
+// step above
 enum PoolKind : uint32_t { kFlight = 0, kSelect = 1, kScatter = 2, kDone = 3 };
+constexpr uint32_t kKindMask = 0xffu, kPoolEvent = 1u << 13;
+static_assert(EMCG_MAX_MECH <= 32 && kPoolMaxEvents < (1u << 19), "the kind word's fields");
 
 template <int G> struct PoolShape {
   static constexpr int P = 32 * G;
@@ -119,7 +123,7 @@ struct PoolEl {
   double k[3], d[3], x[3]; // ellipse-frame k, its displacement not yet in x, position
   double E, tau, gtau, in; // in: time spent inside the step
   int step;
-  uint32_t words, meta, kind; // draws consumed in the step; PoolKind | mechanism << 8
+  uint32_t words, meta, kind; // draws consumed in the step; the kind word above
 };
 
 // The summed ellipse-frame displacement into the device frame and the periodic
@@ -185,7 +189,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
     p.d[i] = fma(p.k[i] + kO[i], c, p.d[i]);
   if (ev) {
     p.in += t;
-    p.kind = kSelect;
+    p.kind |= kSelect; // (from kFlight)
     return false;
   }
   p.tau -= t;
@@ -198,6 +202,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
   vd = vh * (gk + gk);
   p.step++;
   p.words = 0;
+  p.kind = kFlight;
   return true;
 }
 
@@ -211,12 +216,12 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
   int valley = kOne ? 0 : (int)(p.meta & 0xff);
   const int region = p.meta >> 16;
   const int ts = M.tsIndex[valley][region];
+  if (p.kind / kPoolEvent >= kPoolMaxEvents)
+    return EMCG_ERR_TIMEOUT;
   if (ts < 0)
     return EMCG_ERR_OUT_OF_TABLE;
-  if (rng.i > kPoolMaxWords)
-    return EMCG_ERR_TIMEOUT;
   const int nT = M.tsN[ts];
-  p.kind = kFlight;
+  p.kind = (p.kind / kPoolEvent + 1) * kPoolEvent; // kFlight, an event more
   if (nT > 0) {
     const long long rnd = __double_as_longlong(rng.u01());
     const double *row = M.tables + M.tsOff[ts] + (int64_t)levelFast(p.E, M.dE, M.invdE, M.nLevels) * nT;
@@ -229,7 +234,7 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
       if (t < nT) {
         const int mi = M.tsMech[ts][t];
         const MechK<double> &me = M.m[mi];
-        p.kind = kScatter | (uint32_t)mi << 8;
+        p.kind |= kScatter | (uint32_t)mi << 8;
         p.words = rng.i;
         valley = kOne ? 0 : me.finalValley;
         // a direction takes two draws, an intervalley event its subvalley's too
@@ -238,7 +243,7 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
     }
   }
   p.tau = -poolLog(rng.ulog(), M.logT) * tauOf(M, valley, region);
-  if (p.kind == kFlight)
+  if ((p.kind & kKindMask) == kFlight)
     p.words = rng.i;
   return 0;
 }
@@ -248,7 +253,7 @@ template <bool kOne>
 __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK<double> &M,
                                             uint32_t pid, uint32_t step0, PoolEl &p) {
   PoolDraws rng(EK, pid, step0 + (uint32_t)p.step, p.words);
-  const MechK<double> &me = M.m[p.kind >> 8];
+  const MechK<double> &me = M.m[(p.kind >> 8) & 31u];
   int valley = kOne ? 0 : (int)(p.meta & 0xff), sub = (p.meta >> 8) & 0xff;
   const int region = p.meta >> 16;
   double kd[3];
@@ -280,7 +285,7 @@ __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK
   }
   rotate<false>(M.v[valley], sub, kd, p.k);
   p.words = rng.i + 1; // the free flight's draw is taken
-  p.kind = kFlight;
+  p.kind &= ~(kPoolEvent - 1); // kFlight
 }
 
 // G: pools of up to 32 G electrons, one warp per block and pool; kOne: every
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(32)
 #pragma unroll
     for (int g = 0; g < G; g++) {
       const int s = kReg ? p.step : stp[32 * g + lane];
-      const uint32_t k = (kReg ? p.kind : kind[32 * g + lane]) & 0xffu;
+      const uint32_t k = (kReg ? p.kind : kind[32 * g + lane]) & kKindMask;
       mF[g] = __ballot_sync(0xffffffffu, k == kFlight && s < limit);
       mS[g] = __ballot_sync(0xffffffffu, k == kSelect);
       mR[g] = __ballot_sync(0xffffffffu, k == kScatter);
