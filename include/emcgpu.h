@@ -567,6 +567,13 @@ int32_t emcg_device_step_many(emcg_handle **h, int32_t n, int32_t n_steps, uint3
    -1 = leave as is.  *cluster_size (may be NULL) receives the CTAs per
    cluster of the solve in use, 0 for the multi-launch path. */
 int32_t emcg_device_poisson_mode(emcg_handle *h, int32_t mode, int32_t *cluster_size);
+/* The form of the engine's solve as it is planned now: *ctas of the cluster
+   that runs the whole of it in one launch (0: none); else the first multigrid
+   level *tail_level that one launch of a cluster of *tail_ctas runs with all
+   coarser ones, the finer in one launch per phase (0: all in one launch per
+   phase).  Outputs may be NULL.  No reference counterpart. */
+int32_t emcg_device_poisson_form(emcg_handle *h, int32_t *ctas, int32_t *tail_level,
+                                 int32_t *tail_ctas);
 /* Upper bound on the CTAs of the single-launch Poisson cluster (0: none; the
    largest size whose layout fits is taken, 16, 14, 12, 10, 8, 4, 2 or 1).
    The result does not depend on the size.  *cluster_size (may be NULL)
@@ -619,6 +626,11 @@ int32_t emcg_poisson_solve_noalloc(const emcg_device_desc *dev, double *d_pot,
                                    const double *d_conc, int32_t reset_bc, int32_t smooth,
                                    double rtol, int32_t max_cycles, void *cuda_stream,
                                    double *rel_residual, int32_t *cycles);
+/* The form (as emcg_device_poisson_form) that the calling thread's last
+   emcg_poisson_solve_noalloc took; all 0 before the first.  A grid whose
+   levels have more than 64 different coefficient tuples runs in one launch
+   per phase. */
+int32_t emcg_poisson_noalloc_form(int32_t *ctas, int32_t *tail_level, int32_t *tail_ctas);
 
 #ifdef __cplusplus
 }

@@ -61,5 +61,5 @@ def test_call_without_a_gpu():
 
 @pytest.mark.gpu
 def test_solves_on_a_small_stack(engine):
-    rc, out, err = _run(True, 192 << 10, [(201, 101, 0), (360, 361, 0), (301, 61, 40)])
+    rc, out, err = _run(True, 192 << 10, [(201, 101, 0), (360, 361, 0), (301, 61, 61)])
     assert (rc, out) == (0, ["0"] * 6), err

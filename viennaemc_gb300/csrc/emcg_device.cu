@@ -2144,6 +2144,21 @@ extern "C" int32_t emcg_device_poisson_mode(emcg_handle *h, int32_t mode, int32_
   return EMCG_OK;
 }
 
+extern "C" int32_t emcg_device_poisson_form(emcg_handle *h, int32_t *ctas, int32_t *tail_level,
+                                            int32_t *tail_ctas) {
+  DeviceImpl *d;
+  EMCG_TRY(devOf(h, &d));
+  const PoissonMG &P = d->mg;
+  const bool tail = P.useCluster && !P.clusterSize && P.tailLevel;
+  if (ctas)
+    *ctas = P.useCluster ? P.clusterSize : 0;
+  if (tail_level)
+    *tail_level = tail ? P.tailLevel : 0;
+  if (tail_ctas)
+    *tail_ctas = tail ? P.tailSize : 0;
+  return EMCG_OK;
+}
+
 extern "C" int32_t emcg_device_set_poisson_cluster(emcg_handle *h, int32_t max_ctas,
                                                    int32_t *cluster_size) {
   DeviceImpl *d;

@@ -2692,6 +2692,18 @@ static int32_t poissonScratchAddress(unsigned char **out) {
 
 } // namespace emcg
 
+// the form of the thread's last solve (emcg_poisson_noalloc_form)
+static thread_local int32_t g_noallocForm[3] = {};
+
+extern "C" int32_t emcg_poisson_noalloc_form(int32_t *ctas, int32_t *tail_level,
+                                             int32_t *tail_ctas) {
+  int32_t *const out[3] = {ctas, tail_level, tail_ctas};
+  for (int k = 0; k < 3; k++)
+    if (out[k])
+      *out[k] = g_noallocForm[k];
+  return EMCG_OK;
+}
+
 extern "C" int32_t emcg_poisson_solve_noalloc(const emcg_device_desc *dv, double *d_pot,
                                               const double *d_conc, int32_t reset_bc,
                                               int32_t smooth, double rtol, int32_t max_cycles,
@@ -2898,6 +2910,9 @@ extern "C" int32_t emcg_poisson_solve_noalloc(const emcg_device_desc *dv, double
       tail.even = t.even;
     }
   }
+  g_noallocForm[0] = done ? fit.size : 0;
+  g_noallocForm[1] = tail.level;
+  g_noallocForm[2] = tail.level ? tail.size : 0;
   for (; !done && it <= max_cycles; it++) {
     // the residual maxima accumulate by atomic max and must start at zero
     EMCG_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(double), st));

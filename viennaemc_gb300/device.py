@@ -408,6 +408,13 @@ class DeviceSimulation:
         L.check(self._lib.emcg_device_poisson_mode(self.h, int(mode), C.byref(cs)))
         return cs.value
 
+    def poisson_form(self):
+        """(CTAs of the cluster that runs the whole solve, first multigrid level that a
+        cluster runs below finer levels, that cluster's CTAs); 0: none."""
+        out = [C.c_int32() for _ in range(3)]
+        L.check(self._lib.emcg_device_poisson_form(self.h, *map(C.byref, out)))
+        return tuple(v.value for v in out)
+
     def set_poisson_cluster(self, max_ctas=0):
         """Bound the CTAs of the single-launch Poisson cluster (0: none);
         returns the cluster size in use (0: multi-launch path)."""
