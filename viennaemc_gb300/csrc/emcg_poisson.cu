@@ -466,26 +466,6 @@ __device__ __forceinline__ void cOwnRows(const CCtx &c, const CLevel<MT> &L, int
   }
 }
 
-// row y of an array of level L, wherever it lives
-template <class T, class MT>
-__device__ __forceinline__ T *cRow(const CCtx &c, const CLevel<MT> &L, unsigned off, int y) {
-  if (L.small)
-    return reinterpret_cast<T *>((c.rank == 0 ? c.smem : c.base[0]) + off) + (size_t)y * L.nx;
-  const int owner = L.byRows.div(y);
-  return reinterpret_cast<T *>((owner == c.rank ? c.smem : c.base[owner]) + off) +
-         (size_t)(y - owner * L.rowsPer) * L.nx;
-}
-
-// row r0 + ly of level L, for this CTA's rows and their neighbours
-template <class T, class MT>
-__device__ __forceinline__ T *cRowNear(const CCtx &c, const CLevel<MT> &L, unsigned off, int ly) {
-  if (L.small || (ly >= 0 && ly < L.rowsPer))
-    return reinterpret_cast<T *>(c.smem + off) + (size_t)ly * L.nx;
-  if (ly < 0)
-    return reinterpret_cast<T *>(c.base[c.rank - 1] + off) + (size_t)(L.rowsPer - 1) * L.nx;
-  return reinterpret_cast<T *>(c.base[c.rank + 1] + off);
-}
-
 template <class T> __device__ __forceinline__ const T *cTab(const CCtx &c, unsigned off) {
   return reinterpret_cast<const T *>(c.smem + off);
 }
@@ -515,28 +495,17 @@ template <class MT> __device__ __forceinline__ int cStride(const CLevel<MT> &L) 
   return L.warp ? 32 : (int)blockDim.x;
 }
 
-// row accessors of a phase; kS: the row is in this CTA's shared memory (its
-// own rows, or any row of a level held whole by CTA 0 in a phase that runs
-// there), so the accesses compile to shared-memory loads and stores rather
-// than generic ones
-template <bool kS, class T, class MT>
-__device__ __forceinline__ T *cRowT(const CCtx &c, const CLevel<MT> &L, unsigned off, int y) {
-  if (kS)
-    return reinterpret_cast<T *>(c.smem + off) + (size_t)y * L.nx;
-  return cRow<T>(c, L, off, y);
-}
-template <bool kS, class T, class MT>
-__device__ __forceinline__ T *cRowNearT(const CCtx &c, const CLevel<MT> &L, unsigned off, int ly) {
-  if (kS)
-    return reinterpret_cast<T *>(c.smem + off) + (size_t)ly * L.nx;
-  return cRowNear<T>(c, L, off, ly);
+// row ly of the CTA's own rows of an array of level L
+template <class T, class MT>
+__device__ __forceinline__ T *cOwn(const CCtx &c, const CLevel<MT> &L, unsigned off, int ly) {
+  return reinterpret_cast<T *>(c.smem + off) + (size_t)ly * L.nx;
 }
 
 // Several red-black sweeps over level L with each thread's nodes held in
 // registers: a thread keeps the same nodes of each colour over the three sweeps,
 // so their position, class, right-hand side and the diagonal's reciprocal are
 // formed once, and a half sweep reads only the coefficients and the neighbours'
-// corrections.  The arithmetic is cSmoothT's.
+// corrections.  The arithmetic is sweepValue's.
 //
 // A phase costs its longest chain of dependent instructions and what the four
 // warps of a scheduler issue in it, not its work: so a thread's nodes go through
@@ -1207,10 +1176,10 @@ template <class MT> __device__ void cCoarse(const CCtx &c, const CLevel<MT> &L, 
     if (threadIdx.x < 32) {
       const int i = threadIdx.x, x = i % L.nx, y = i / L.nx;
       const bool live = i < n;
-      const Coef<MT> K = cCoef(c, L, live ? cRowT<true, uint8_t>(c, L, L.offCls, y)[x] : 0);
-      MT *dp = live ? cRowT<true, MT>(c, L, L.offD, y) + x : nullptr;
-      const MT r = live ? cRowT<true, MT>(c, L, L.offR, y)[x] : MT(0);
-      const MT den = live ? fma(K.area, cRowT<true, MT>(c, L, L.offRho, y)[x], K.diag0) : MT(1);
+      const Coef<MT> K = cCoef(c, L, live ? cOwn<uint8_t>(c, L, L.offCls, y)[x] : 0);
+      MT *dp = live ? cOwn<MT>(c, L, L.offD, y) + x : nullptr;
+      const MT r = live ? cOwn<MT>(c, L, L.offR, y)[x] : MT(0);
+      const MT den = live ? fma(K.area, cOwn<MT>(c, L, L.offRho, y)[x], K.diag0) : MT(1);
       const MT inv = mgRcp(den);
       const bool upd = live && K.fixed == MT(0);
       MT d = live ? *dp : MT(0);
@@ -1235,20 +1204,20 @@ template <class MT> __device__ void cCoarse(const CCtx &c, const CLevel<MT> &L, 
     for (int color = 0; color < 2; color++) {
       for (int i = threadIdx.x; i < n; i += stride) {
         const int x = i % L.nx, y = i / L.nx;
-        const Coef<MT> K = cCoef(c, L, cRowT<true, uint8_t>(c, L, L.offCls, y)[x]);
+        const Coef<MT> K = cCoef(c, L, cOwn<uint8_t>(c, L, L.offCls, y)[x]);
         if (((x + y) & 1) != color || K.fixed != MT(0))
           continue;
-        MT *d = cRowT<true, MT>(c, L, L.offD, y);
-        MT s = cRowT<true, MT>(c, L, L.offR, y)[x];
+        MT *d = cOwn<MT>(c, L, L.offD, y);
+        MT s = cOwn<MT>(c, L, L.offR, y)[x];
         if (x > 0)
           s = fma(K.cw, d[x - 1], s);
         if (x < L.nx - 1)
           s = fma(K.ce, d[x + 1], s);
         if (y > 0)
-          s = fma(K.cs, cRowT<true, MT>(c, L, L.offD, y - 1)[x], s);
+          s = fma(K.cs, cOwn<MT>(c, L, L.offD, y - 1)[x], s);
         if (y < L.ny - 1)
-          s = fma(K.cn, cRowT<true, MT>(c, L, L.offD, y + 1)[x], s);
-        d[x] = s * mgRcp(fma(K.area, cRowT<true, MT>(c, L, L.offRho, y)[x], K.diag0));
+          s = fma(K.cn, cOwn<MT>(c, L, L.offD, y + 1)[x], s);
+        d[x] = s * mgRcp(fma(K.area, cOwn<MT>(c, L, L.offRho, y)[x], K.diag0));
       }
       cSync(L);
     }
@@ -1500,9 +1469,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     asm volatile("cp.async.wait_all;" ::: "memory");
   };
   if constexpr (kTail) {
-    MT *d0 = cRowNearT<true, MT>(c, L0, L0.offD, 0);
-    MT *r0 = cRowNearT<true, MT>(c, L0, L0.offR, 0);
-    MT *rho0 = cRowNearT<true, MT>(c, L0, L0.offRho, 0);
+    MT *d0 = cOwn<MT>(c, L0, L0.offD, 0);
+    MT *r0 = cOwn<MT>(c, L0, L0.offR, 0);
+    MT *rho0 = cOwn<MT>(c, L0, L0.offRho, 0);
     for (int t = threadIdx.x; t < nOwn; t += blockDim.x) {
       d0[t] = MT(0);
       r0[t] = tailR[(size_t)p0 * nx + t];
@@ -1550,11 +1519,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         const NodeIn in = next;
         next = load(min(t + (int)blockDim.x, nOwn - 1));
         const int ly = L0.byNx.div(t), y = p0 + ly, x = t - ly * nx;
-        MT *d0 = cRowNearT<true, MT>(c, L0, L0.offD, ly);
-        MT *r0 = cRowNearT<true, MT>(c, L0, L0.offR, ly);
-        MT *rho0 = cRowNearT<true, MT>(c, L0, L0.offRho, ly);
+        MT *d0 = cOwn<MT>(c, L0, L0.offD, ly);
+        MT *r0 = cOwn<MT>(c, L0, L0.offR, ly);
+        MT *rho0 = cOwn<MT>(c, L0, L0.offRho, ly);
         d0[x] = MT(0);
-        if (cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, ly)[x]).fixed != MT(0)) {
+        if (cCoef(c, L0, cOwn<uint8_t>(c, L0, L0.offCls, ly)[x]).fixed != MT(0)) {
           r0[x] = MT(0);
           rho0[x] = MT(0);
           continue;
@@ -1600,9 +1569,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int t = t0 + u * (int)blockDim.x;
-        if (t >= nOwn || cCoef(c, L0, cRowNearT<true, uint8_t>(c, L0, L0.offCls, 0)[t]).fixed != MT(0))
+        if (t >= nOwn ||
+            cCoef(c, L0, cOwn<uint8_t>(c, L0, L0.offCls, 0)[t]).fixed != MT(0))
           continue;
-        MT v = cRowNearT<true, MT>(c, L0, L0.offD, 0)[t];
+        MT v = cOwn<MT>(c, L0, L0.offD, 0)[t];
         if (isfinite(v)) // a non-finite correction is passed on to the next residual
           v = fmin(MT(kMaxNewtonStep), fmax(MT(-kMaxNewtonStep), v));
         pot[(size_t)p0 * nx + t] = phi[u] + doubleOf(v);
