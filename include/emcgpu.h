@@ -612,7 +612,9 @@ int32_t emcg_device_poisson_counts(emcg_handle *h, int64_t *cycles, int64_t *sol
    (CUDA_MODULE_LOADING=EAGER loads it when the context is created).  A
    caller whose memory pool will claim the rest of the GPU should therefore
    make one call at start-up, before the pool takes the device.
-   The first call on each device also looks the array's address up
+   The first call on each device also loads the kernels of every form of the
+   solve, whichever its own grid takes, so that no later call takes device
+   memory for them.  It looks the array's address up
    (cudaGetSymbolAddress, with that device current) and keeps it for the
    life of the process; make it before any stream capture begins on that
    device.  The kept address is not valid after cudaDeviceReset on that

@@ -2641,6 +2641,27 @@ __global__ void naTransferKernel(const __grid_constant__ NALevels lv,
 static __device__ __align__(256) unsigned char g_poissonScratch[kNABytes];
 static std::atomic<void *> g_poissonScratchAddr[kNAMaxDevices];
 
+// The kernels of every form of the solve, loaded: the runtime loads a kernel at its
+// first use, into device memory, and which form a call takes depends on its grid.  So
+// the first call on a device loads them all, and no later one takes memory.
+template <class... K> static int32_t loadKernels(K... k) {
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaSuccess;
+  ((e = e == cudaSuccess ? cudaFuncGetAttributes(&fa, k) : e), ...);
+  EMCG_CUDA(e);
+  return EMCG_OK;
+}
+static int32_t loadSolveKernels() {
+  return loadKernels(naFineSetupKernel, naLevelSetupKernel, naTransferKernel, naClassKernel,
+                     expTableKernel, resetBCKernel, nonlinResidualKernel<float>,
+                     smoothKernel<float>, restrictKernel<float>, prolongKernel<float>,
+                     coarseSolveKernel<float>, updatePotKernel<float>,
+                     poissonClusterKernel<float, false, false>,
+                     poissonClusterKernel<float, false, true>,
+                     poissonClusterKernel<float, true, false>,
+                     poissonClusterKernel<float, true, true>);
+}
+
 static int32_t poissonScratchAddress(unsigned char **out) {
   int dev = -1;
   EMCG_CUDA(cudaGetDevice(&dev));
@@ -2654,6 +2675,7 @@ static int32_t poissonScratchAddress(unsigned char **out) {
                cudaGetErrorString(e));
       return EMCG_ERR_CUDA;
     }
+    EMCG_TRY(loadSolveKernels());
     g_poissonScratchAddr[dev].store(p, std::memory_order_release);
   }
   *out = static_cast<unsigned char *>(p);
