@@ -401,8 +401,8 @@ int32_t emcg_get_rates(emcg_handle *h, int32_t model, double *tables, double *ta
    inv_cutoff: 1 / cutoff radius [1/m] (1e9: the reference's 1 nm; 0: none);
    images: copies of the cubic box of width box on each side in x, y and z
    (0: the box alone; a particle sees its own copies, not itself);
-   precision: EMCG_FP64 (the reference's arithmetic order) or EMCG_FP32
-   (float pair terms, double sums per tile).  force: 3 x n, potential: n;
+   precision: EMCG_FP64 (double terms, the reference's to their rounding) or
+   EMCG_FP32 (float pair terms, double sums per tile).  force: 3 x n, potential: n;
    *kernel_ms (may be NULL): device time of the sums. */
 int32_t emcg_p2p_coulomb(const double *pos, const double *charge, int64_t n,
                          double inv_cutoff, double box, int32_t images,

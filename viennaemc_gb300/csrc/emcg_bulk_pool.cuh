@@ -23,7 +23,7 @@
 // only by real scattering, as in the float engine's warp-asynchronous kernel.
 // Measured, lockstep -> pools: 10,000 electrons x 100 steps 3.65 -> 1.01 ms a call
 // with its read-back, 250,007 x 20 steps 4.00 -> 0.94 ms, 10^6 electrons 1.8e9
-// -> 5.6e9 particle-steps/s, 92 double instructions per 32 particle-steps at 82 %
+// -> 5.6e9 particle-steps/s, 92 double instructions per 32 particle-steps at 83 %
 // of the pipe.  A window of 16 steps costs resident pools (4.6e9), one of 4 with
 // 128 electrons per pool gains 4 % at 10^6 electrons and loses as much at 10^4.
 // Integer instructions replace double ones where the result is the same bit for
@@ -224,7 +224,8 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
   p.kind = (p.kind / kPoolEvent + 1) * kPoolEvent; // kFlight, an event more
   if (nT > 0) {
     const long long rnd = __double_as_longlong(rng.u01());
-    const double *row = M.tables + M.tsOff[ts] + (int64_t)levelFast(p.E, M.dE, M.invdE, M.nLevels) * nT;
+    const double *row =
+        M.tables + M.tsOff[ts] + (int64_t)levelFast(p.E, M.dE, M.invdE, M.nLevels) * nT;
     // non-negative doubles compare like their bit patterns
     if (rnd <= __double_as_longlong(ldg(row + nT - 1))) {
       int t = 0;

@@ -368,7 +368,7 @@ __device__ __forceinline__ void devStore(const StateK<T> &st, const DevK &G, int
 // So the events of a block are queued and one warp -- another one from block to
 // block, as warps of the same number share a scheduler -- works on 32 of them at
 // a time.  Measured with the building blocks of emcg_fp64.cuh, 5e4 electrons
-// (nearest-node scheme, under ncu): 105 -> 37 us.
+// (nearest-node scheme, under ncu): 105 -> 39 us.
 template <int SCHEME>
 __global__ void __launch_bounds__(256)
     devMoveQueuedKernel(StateK<double> st, const ModelK<double> *__restrict__ models, DevK G,
@@ -478,9 +478,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
 // themselves, a block adds up the counts before it instead of a scan between two
 // launches, the compaction and the injection assign the charge of the particles
 // that they place, the first kernel clears the step's counters, and the last one
-// writes the outcome into page-locked memory.  10 nodes a step on the stream
-// instead of 24 (9 since the injection forms its own numbers); resistor 201 x 101, 500k electrons FP32: 0.502 -> 0.444 ms a step,
-// 101 x 51, 50k electrons FP64 0.394 -> 0.329, 8 MOSFETs of 401 x 201 at once 7.6 -> 6.8 ms per 5.
+// writes the outcome into page-locked memory.  9 nodes a step on the stream instead of
+// 24.  Measured with 10 (before the injection formed its own numbers): resistor 201 x
+// 101, 500k electrons FP32 0.502 -> 0.444 ms a step, 101 x 51, 50k electrons FP64 0.394
+// -> 0.329, 8 MOSFETs of 401 x 201 at once 7.6 -> 6.8 ms per 5.
 __device__ __forceinline__ int blockExclusiveScan(int v, int *total) {
   __shared__ int warpSums[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

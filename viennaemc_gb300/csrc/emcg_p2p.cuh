@@ -24,10 +24,10 @@
 //   so that the 13 issue as 6.5 packed instructions with the same results (add,
 //   mul, fma .rn.f32x2), and the hardware's rsqrt is taken without the code
 //   around it for subnormal arguments: a tile whose sums are not finite, as they
-//   are with such an argument, is summed again with rsqrtf.  10.2 instructions
-//   per pair instead of 19.5; the register reads of the packed instructions
-//   bound it now (a loop of packed fma with distinct operands runs at 38 to 44
-//   per clock and SM, 64 with one operand): 1.31e12 -> 2.05e12 pairs/s at
+//   are with such an argument, is summed again with rsqrtf.  10.9 instructions
+//   per pair instead of 19.5; the register reads of the packed instructions bound
+//   it now (a loop of packed fma with distinct operands runs at 38 to 44 per clock
+//   and SM, 64 with one operand): 1.31e12 -> 2.05e12 pairs/s at
 //   32,768 charges, 1.73e12 -> 2.25e12 at 262,144.
 // - double: an SM issues a double instruction of a warp every 16 clocks, so
 //   their number counts: 18 per pair with 1 / r from the hardware's
