@@ -83,3 +83,49 @@ def test_minus_zero_is_inside_the_device(engine, precision):
     assert netto.sum() == 1 and st.n == 4  # the one outside
     assert sorted(st.px) == sorted(np.float32(pos[[0, 1, 2, 4], 0]) if precision == "fp32"
                                    else pos[[0, 1, 2, 4], 0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h", [1e-9, 0.5e-9, 0.7e-9])
+@pytest.mark.parametrize("scheme", ["ngp", "cic"])
+def test_grid_lookups_beside_whole_and_half_numbers(engine, scheme, h):
+    """The node of a position (the nearest, and the lower one with its weight) is that of
+    v / h, also a few units in the last place from k h and (k + 1/2) h, and between."""
+    from viennaemc_gb300 import _lib as L
+    from viennaemc_gb300 import device as D
+    nx, ny = 201, 31
+    dev = _bar(nx, ny, h)
+    pt = engine.physics.silicon_electron("refbulk", n_levels=100, max_energy=4.0)
+    rs = np.random.default_rng(17)
+    k = rs.integers(0, 2 * (nx - 1), 6000)
+    x = np.abs(k * (h / 2) * (1 + rs.integers(-4, 5, k.size) * 2.0 ** -53))
+    x[4000:] = rs.random(2000) * (nx - 1) * h
+    x[5000:] = (k[5000:] * (h / 2)) * (1 + (rs.random(1000) - 0.5) * 2.0 ** -17)
+    x = np.clip(x, 0.0, dev.max_pos[0])
+    y = np.full(x.size, 3 * h)
+    sim = D.DeviceSimulation(dev, pt, scheme=D.NGP if scheme == "ngp" else D.CIC,
+                             capacity=x.size)
+    sim.set_state(_resting(engine, np.stack([x, y], 1)))
+    sim.assign()
+    got = sim.get_grid(L.GRID_NRPART).reshape(ny, nx) / sim.carriers
+    sim.close()
+    want = np.zeros((ny, nx))
+    if scheme == "ngp":
+        q = x / h
+        near = np.floor(q) + (q - np.floor(q) >= 0.5)
+        np.add.at(want, (np.full(x.size, int(np.rint(y[0] / h))), near.astype(int)), 1.0)
+        assert np.array_equal(got, want)
+    else:
+        m, w = [], []
+        for v in (x, y):
+            q = v / h
+            m.append(np.floor(q).astype(int))
+            w.append(q - np.floor(q))
+        for dx in (0, 1):
+            for dy in (0, 1):
+                cx, cy = m[0] + dx, m[1] + dy
+                on = (cx < nx) & (cy < ny)
+                wt = (w[0] if dx == 0 else 1 - w[0]) * (w[1] if dy == 0 else 1 - w[1])
+                np.add.at(want, (cy[on], cx[on]), wt[on])
+        # a weight is off by a unit in the last place of q < 256 at most
+        assert np.max(np.abs(got - want)) <= 2.0 ** -45 * np.max(np.bincount(m[0]) * 2 + 2)
