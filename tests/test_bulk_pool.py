@@ -149,3 +149,38 @@ def test_event_limit_of_a_step(engine, n):
         x, y = getattr(a, f), getattr(q, f)
         bad |= np.abs(x - y) > 1e-9 * np.max(np.abs(y))
     assert bad.sum() <= 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model", ["silicon", "tilted"])
+@pytest.mark.parametrize("n", [7, 600, 60013, 120001])
+@pytest.mark.parametrize("box,dt,spread", [((1e-6, 1e-6, 1e-6), 1e-15, 4.0),
+                                           ((1e-8, 3e-8, 2e-9), 2e-14, 1.0),
+                                           ((2e-9, 2e-9, 5e-9), 3e-15, 2.5)])
+def test_periodic_box_as_the_reference_wraps_it(engine, model, n, box, dt, spread):
+    """One box length is added or taken after a flight (basicBulkParticleHandler.hpp:
+    600-613): electrons that start outside the box come nearer by one a flight, and
+    flights longer than it end outside.  Against the block-queued kernel, which wraps
+    each flight; positions within 1e-9 of a box."""
+    pt = _tilted(engine) if model == "tilted" else engine.physics.silicon_electron("jacoboni")
+    spec = engine.EnsembleSpec(0, n, 2e6, (1, 2, 3), box, dt, 21)
+    rs = np.random.default_rng(n)
+    start = (rs.random((3, n)) - 0.5) * 2 * spread + 0.5
+    got = []
+    for mode in (0, 1):
+        b = engine.BulkBatch([pt], [spec], "fp64")
+        b.set_launch(queued=mode)
+        b.init_particles(0)
+        st = b.get_state(0)
+        for f, x, L in zip(("px", "py", "pz"), start, box):
+            getattr(st, f)[:] = x * L
+        st.tau[::5] *= -1.0  # a timer that ran out before the call
+        b.set_state(0, st)
+        b.step(3)
+        got.append(b.get_state(0))
+        b.close()
+    a, q = got
+    bad = (a.valley != q.valley) | (a.sub != q.sub)
+    for f, L in zip(("px", "py", "pz"), box):
+        bad |= np.abs(getattr(a, f) - getattr(q, f)) > 1e-9 * L
+    assert bad.sum() <= n // 1000

@@ -1150,6 +1150,21 @@ static void buildEnsK(const emcg_ensemble_desc &d, const ModelK<T> &M,
         E.g[v][s][i] = (T)(dv.vogt[i] * de);
       }
     }
+    // a flight's displacement is below |R| max(vogt) (hbar / mc) |k| dt (the
+    // non-parabolicity only shortens it)
+    double frob = 0;
+    for (int s = 0; s < V.deg; s++) {
+      double f = 0;
+      for (int i = 0; i < 9; i++)
+        f += V.rot[s][i] * V.rot[s][i];
+      frob = std::max(frob, std::sqrt(f));
+    }
+    const double per = frob * std::max(dv.vogt[0], std::max(dv.vogt[1], dv.vogt[2])) *
+                       (kHBAR / dv.mc) * d.dt;
+    const double k = V.alpha >= 0 && per > 0
+                         ? 0.5 * std::min(d.box[0], std::min(d.box[1], d.box[2])) / per
+                         : 0.;
+    E.farK2[v] = (uint32_t)(dbits(k * k) >> 32);
   }
   for (int i = 0; i < 3; i++) {
     E.box[i] = (T)d.box[i];

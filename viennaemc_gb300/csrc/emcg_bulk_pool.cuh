@@ -42,10 +42,10 @@ constexpr int kPoolFields = 13; // k, d, E, tau, gtau, in, x in shared memory
 constexpr uint32_t kPoolMaxEvents = 1u << 16; // of one electron in one step
 
 // an electron's kind word: PoolKind, its mechanism in bits 8 to 12, its events in the
-// step above
+// step above, and kPoolFar: its next flight is wrapped by itself (poolFarFlight)
 enum PoolKind : uint32_t { kFlight = 0, kSelect = 1, kScatter = 2, kDone = 3 };
-constexpr uint32_t kKindMask = 0xffu, kPoolEvent = 1u << 13;
-static_assert(EMCG_MAX_MECH <= 32 && kPoolMaxEvents < (1u << 19), "the kind word's fields");
+constexpr uint32_t kKindMask = 0xffu, kPoolEvent = 1u << 13, kPoolFar = 1u << 31;
+static_assert(EMCG_MAX_MECH <= 32 && kPoolMaxEvents < (1u << 18), "the kind word's fields");
 
 template <int G> struct PoolShape {
   static constexpr int P = 32 * G;
@@ -127,9 +127,13 @@ struct PoolEl {
 };
 
 // The summed ellipse-frame displacement into the device frame and the periodic
-// box, as flushPos of the float engine.
+// box, as flushPos of the float engine: flights of less than half a box from a position
+// inside it, for which this is the reference's rule (basicBulkParticleHandler.hpp:
+// 600-613: one box length added or taken after each flight).  kPoolFar: none is summed.
 __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, const double box[3],
                                           PoolEl &p) {
+  if (p.kind & kPoolFar)
+    return;
   double d[3], dd[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
@@ -144,6 +148,48 @@ __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, con
       c -= box[i] * floor(c / box[i]);
     p.x[i] = c;
   }
+}
+
+// outside the box
+__device__ __forceinline__ bool poolOutside(const double *box, double x, double y, double z) {
+  return belowD(x, 0.0) || belowD(box[0], x) || belowD(y, 0.0) || belowD(box[1], y) ||
+         belowD(z, 0.0) || belowD(box[2], z);
+}
+// A flight that may be longer than half a box, or that starts outside it: the earlier
+// flights' displacement d into the position (unless far: there is none), then this
+// one's, i, with the reference's rule.  A call, by values: it is rare, and the flights'
+// sums stay in registers.
+struct PoolFarPos {
+  double x[3];
+  bool out;
+};
+__device__ __noinline__ PoolFarPos poolFarFlight(const ValleyK<double> *V, int sub,
+                                                 const double *box, bool far, double d0,
+                                                 double d1, double d2, double i0, double i1,
+                                                 double i2, double x0, double x1, double x2) {
+  const double d[2][3] = {{d0 * V->vogt[0], d1 * V->vogt[1], d2 * V->vogt[2]},
+                          {i0 * V->vogt[0], i1 * V->vogt[1], i2 * V->vogt[2]}};
+  double s[3], t[3];
+  rotate<true>(*V, sub, d[0], s);
+  rotate<true>(*V, sub, d[1], t);
+  const double x[3] = {x0, x1, x2};
+  PoolFarPos o;
+  for (int i = 0; i < 3; i++) {
+    double c = x[i];
+    if (!far) {
+      c += s[i];
+      if (belowD(c, 0.0) || belowD(box[i], c))
+        c -= box[i] * floor(c / box[i]);
+    }
+    c += t[i];
+    if (belowD(c, 0.0))
+      c += box[i];
+    else if (belowD(box[i], c))
+      c -= box[i];
+    o.x[i] = c;
+  }
+  o.out = poolOutside(box, o.x[0], o.x[1], o.x[2]);
+  return o;
 }
 
 // the grain timer ran out (basicBulkParticleHandler.hpp:215-219)
@@ -162,14 +208,17 @@ __device__ __forceinline__ void poolGrain(const ModelK<double> &M, const EnsK<do
 
 struct PoolValley { // a valley's constants of the free flight
   double cE, alpha2, cX; // hbar^2 / (mc q), 2 alpha, hbar / mc
+  uint32_t farK2;        // EnsK::farK2
 };
 
 // A free flight of p (drift(), include/emcParticleDrift.hpp:11-36, in the ellipse
 // frame) to the end of its step or its next event; true at the end of the step,
-// vd then the velocity along the field.
+// vd then the velocity along the field.  x(i): the position, where it is kept.
+template <class X>
 __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<double> &EK,
                                            const ModelK<double> &M, int valley, int sub,
-                                           uint32_t pid, uint32_t step0, PoolEl &p, double &vd) {
+                                           uint32_t pid, uint32_t step0, PoolEl &p, X x,
+                                           double &vd) {
   const double *fv = EK.fv[valley][sub];
   const double rem = EK.dt - p.in;
   const bool ev = belowD(p.tau, rem);
@@ -181,12 +230,26 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
     p.k[i] = fma(fv[i], t, kO[i]);
   }
   double rs;
-  p.E = energyRoot(V.cE, V.alpha2, fma(p.k[2], p.k[2], fma(p.k[1], p.k[1], p.k[0] * p.k[0])), rs);
+  const double k2 = fma(p.k[2], p.k[2], fma(p.k[1], p.k[1], p.k[0] * p.k[0]));
+  p.E = energyRoot(V.cE, V.alpha2, k2, rs);
   const double vh = V.cX * (0.5 * rs); // hbar / (2 mc (1 + 2 alpha E))
   const double c = vh * t;
+  const bool big = (uint32_t)__double2hiint(k2) >= V.farK2;
+  if (big || (p.kind & kPoolFar)) {
+    const PoolFarPos o = poolFarFlight(
+        &M.v[valley], sub, EK.box, p.kind & kPoolFar, p.d[0], p.d[1], p.d[2],
+        (p.k[0] + kO[0]) * c, (p.k[1] + kO[1]) * c, (p.k[2] + kO[2]) * c, x(0), x(1), x(2));
 #pragma unroll
-  for (int i = 0; i < 3; i++)
-    p.d[i] = fma(p.k[i] + kO[i], c, p.d[i]);
+    for (int i = 0; i < 3; i++) {
+      x(i) = o.x[i];
+      p.d[i] = 0.0;
+    }
+    p.kind = (p.kind & ~kPoolFar) | (big || o.out ? kPoolFar : 0u);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      p.d[i] = fma(p.k[i] + kO[i], c, p.d[i]);
+  }
   if (ev) {
     p.in += t;
     p.kind |= kSelect; // (from kFlight)
@@ -202,7 +265,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
   vd = vh * (gk + gk);
   p.step++;
   p.words = 0;
-  p.kind = kFlight;
+  p.kind &= kPoolFar; // kFlight, no events
   return true;
 }
 
@@ -216,12 +279,13 @@ __device__ __forceinline__ int poolSelect(const EnsK<double> &EK, const ModelK<d
   int valley = kOne ? 0 : (int)(p.meta & 0xff);
   const int region = p.meta >> 16;
   const int ts = M.tsIndex[valley][region];
-  if (p.kind / kPoolEvent >= kPoolMaxEvents)
+  const uint32_t far = p.kind & kPoolFar, events = (p.kind & ~kPoolFar) / kPoolEvent;
+  if (events >= kPoolMaxEvents)
     return EMCG_ERR_TIMEOUT;
   if (ts < 0)
     return EMCG_ERR_OUT_OF_TABLE;
   const int nT = M.tsN[ts];
-  p.kind = (p.kind / kPoolEvent + 1) * kPoolEvent; // kFlight, an event more
+  p.kind = far | (events + 1) * kPoolEvent; // kFlight
   if (nT > 0) {
     const long long rnd = __double_as_longlong(rng.u01());
     const double *row =
@@ -258,6 +322,7 @@ __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK
   int valley = kOne ? 0 : (int)(p.meta & 0xff), sub = (p.meta >> 8) & 0xff;
   const int region = p.meta >> 16;
   double kd[3];
+  bool big = false; // (an elastic mechanism keeps |k|)
   poolFlush(M.v[valley], sub, EK.box, p);
   if (me.kind == EMCG_MECH_COULOMB) {
     toDev(M.v[valley].rot[sub], p.k[0], p.k[1], p.k[2], kd);
@@ -274,6 +339,7 @@ __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK
       p.meta = packMeta(valley, sub, region);
       const double cK = M.v[valley].cK;
       n2 = cK * cK * gammaOf(M.v[valley], p.E);
+      big = (uint32_t)__double2hiint(n2) >= EK.farK2[valley];
     }
     const double nk = sqrtD(n2);
     const double ct = 1.0 - 2.0 * rng.u01(), r1 = rng.u01();
@@ -287,6 +353,8 @@ __device__ __forceinline__ void poolScatter(const EnsK<double> &EK, const ModelK
   rotate<false>(M.v[valley], sub, kd, p.k);
   p.words = rng.i + 1; // the free flight's draw is taken
   p.kind &= ~(kPoolEvent - 1); // kFlight
+  if (big)
+    p.kind |= kPoolFar;
 }
 
 // G: pools of up to 32 G electrons, one warp per block and pool; kOne: every
@@ -317,7 +385,7 @@ __global__ void __launch_bounds__(32)
   const int Q = nVmax * 3;
   const uint32_t pid0 = (uint32_t)(tl.begin - EK.begin);
   // the one valley's constants, in registers
-  const PoolValley one{M.v[0].cE, 2.0 * M.v[0].alpha, M.v[0].cX};
+  const PoolValley one{M.v[0].cE, 2.0 * M.v[0].alpha, M.v[0].cX, EK.farK2[0]};
   int myErr = 0;
 
   PoolEl p;
@@ -351,7 +419,12 @@ __global__ void __launch_bounds__(32)
       p.tau = st.tau[gi];
       p.gtau = st.gtau[gi];
       p.d[0] = p.d[1] = p.d[2] = p.in = 0.0;
-      p.kind = kFlight;
+      // (a negative timer of the caller's may be longer than a step)
+      const double k2 = fma(p.k[2], p.k[2], fma(p.k[1], p.k[1], p.k[0] * p.k[0]));
+      p.kind = (uint32_t)__double2hiint(k2) >= EK.farK2[p.meta & 0xff] ||
+                       __double2hiint(p.tau) < 0 || poolOutside(EK.box, p.x[0], p.x[1], p.x[2])
+                   ? kPoolFar
+                   : 0u; // kFlight
       p.step = 0;
       if (!kReg)
         put(j, 0, kPoolFields);
@@ -467,16 +540,18 @@ __global__ void __launch_bounds__(32)
         get(j, 0, 10);
       const int valley = kOne ? 0 : (int)(p.meta & 0xff), sub = (p.meta >> 8) & 0xff;
       const ValleyK<double> &VK = M.v[valley];
-      const PoolValley V = kOne ? one : PoolValley{VK.cE, 2.0 * VK.alpha, VK.cX};
+      const PoolValley V =
+          kOne ? one : PoolValley{VK.cE, 2.0 * VK.alpha, VK.cX, EK.farK2[valley]};
+      auto x = [&](int i) -> double & { return kReg ? p.x[i] : f[(10 + i) * P + j]; };
       const int slot = p.step & (W - 1);
       double vd;
-      if (poolFlight(V, EK, M, valley, sub, pid, step0, p, vd)) {
+      if (poolFlight(V, EK, M, valley, sub, pid, step0, p, x, vd)) {
         wE[slot * PW + j] = p.E;
         wD[slot * PW + j] = vd;
         if (!kOne)
           wV[slot * P + j] = (uint8_t)valley;
         if (p.step >= nSteps)
-          p.kind = kDone;
+          p.kind |= kDone;
       }
       if (!kReg)
         put(j, 0, 10);
@@ -518,6 +593,7 @@ __global__ void __launch_bounds__(32)
     if (!kReg) {
       get(j, 0, kPoolFields);
       p.meta = meta[j];
+      p.kind = kind[j];
     }
     const ValleyK<double> &V = M.v[p.meta & 0xff];
     const int sub = (p.meta >> 8) & 0xff;

@@ -77,6 +77,9 @@ template <class T> struct EnsK {
   T charge; // [C]
   uint32_t key0, key1, stream;
   uint32_t floatDraws; // EMCG_ENS_FLOAT_DRAWS: the double engine draws as the float one
+  // (double) per valley: the high word of |k|^2 from which a free flight of dt may be
+  // half a box long
+  uint32_t farK2[EMCG_MAX_VALLEYS];
 };
 
 struct Tile {
