@@ -1,5 +1,5 @@
 // emcg_fp64.h against the plain expressions it stands for: prints the number of
-// disagreements of belowD and of fixedOf, and the largest errors of rsqrtStep and
+// disagreements of the comparisons and of fixedOf, and the largest errors of rsqrtStep and
 // rcpStep in units of the last place, from approximations of 20 fraction bits within
 // 2^-20 of the value (the instructions' form).
 #include <cmath>
@@ -21,6 +21,8 @@ int main() {
     for (double b : v)
       if (b >= 0 && !std::signbit(b))
         badBelow += belowD(a, b) != (a < b);
+  for (double a : v)
+    badBelow += (negativeD(a) != (a < 0)) + (notPositiveD(a) != (a <= 0));
   std::uniform_real_distribution<double> e(-40, 33);
   for (double q : v) {
     uint64_t f = 0;

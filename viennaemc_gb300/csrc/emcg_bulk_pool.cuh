@@ -144,7 +144,7 @@ __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, con
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     double c = p.x[i] + dd[i];
-    if (belowD(c, 0.0) || belowD(box[i], c))
+    if (negativeD(c) || belowD(box[i], c))
       c -= box[i] * floor(c / box[i]);
     p.x[i] = c;
   }
@@ -152,8 +152,8 @@ __device__ __forceinline__ void poolFlush(const ValleyK<double> &V, int sub, con
 
 // outside the box
 __device__ __forceinline__ bool poolOutside(const double *box, double x, double y, double z) {
-  return belowD(x, 0.0) || belowD(box[0], x) || belowD(y, 0.0) || belowD(box[1], y) ||
-         belowD(z, 0.0) || belowD(box[2], z);
+  return negativeD(x) || belowD(box[0], x) || negativeD(y) || belowD(box[1], y) ||
+         negativeD(z) || belowD(box[2], z);
 }
 // A flight that may be longer than half a box, or that starts outside it: the earlier
 // flights' displacement d into the position (unless far: there is none), then this
@@ -178,11 +178,11 @@ __device__ __noinline__ PoolFarPos poolFarFlight(const ValleyK<double> *V, int s
     double c = x[i];
     if (!far) {
       c += s[i];
-      if (belowD(c, 0.0) || belowD(box[i], c))
+      if (negativeD(c) || belowD(box[i], c))
         c -= box[i] * floor(c / box[i]);
     }
     c += t[i];
-    if (belowD(c, 0.0))
+    if (negativeD(c))
       c += box[i];
     else if (belowD(box[i], c))
       c -= box[i];
@@ -258,7 +258,7 @@ __device__ __forceinline__ bool poolFlight(const PoolValley &V, const EnsK<doubl
   p.tau -= t;
   p.in = 0.0;
   p.gtau -= EK.dt;
-  if (belowD(p.gtau, 0.0) || (__double_as_longlong(p.gtau) << 1) == 0)
+  if (notPositiveD(p.gtau))
     poolGrain(M, EK, pid, step0 + (uint32_t)p.step, p);
   const double *gd = EK.g[valley][sub];
   const double gk = fma(gd[2], p.k[2], fma(gd[1], p.k[1], gd[0] * p.k[0]));

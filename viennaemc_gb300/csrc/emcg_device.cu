@@ -210,7 +210,7 @@ __device__ __forceinline__ int boundaryOf(const DevK &G, int x, int y) {
 __device__ __forceinline__ bool outside(float v, float mx) { return v < 0.f || v > mx; }
 __device__ __forceinline__ bool outside(double v, double mx) {
   const long long b = __double_as_longlong(v);
-  return belowD(v, 0.0) || (b > __double_as_longlong(mx) && b <= 0x7ff0000000000000ll);
+  return negativeD(v) || (b > __double_as_longlong(mx) && b <= 0x7ff0000000000000ll);
 }
 
 // free flight under force F, then the boundary treatment of

@@ -35,6 +35,14 @@ EMCG_HD bool belowD(double a, double b) {
   return (x == INT64_MIN ? 0 : x) < y && (uint64_t)x <= 0xfff0000000000000ull;
 }
 
+// a < 0 and a <= 0 the same way
+EMCG_HD bool negativeD(double a) {
+  return dbits(a) - 0x8000000000000001ull <= 0x7fefffffffffffffull;
+}
+EMCG_HD bool notPositiveD(double a) {
+  return (int64_t)dbits(a) <= 0 && dbits(a) <= 0xfff0000000000000ull;
+}
+
 // q as an integer part and 20 fractional bits, for 0 <= q < 2^30; false outside
 EMCG_HD bool fixedOf(double q, uint64_t &f) {
   const uint64_t b = dbits(q);
